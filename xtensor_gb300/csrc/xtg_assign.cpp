@@ -356,21 +356,31 @@ static xtg_status assign_rowfused(const Tree& t, const xtg_array& out, int R, co
     };
     while (vec > 1 && !vec_ok(vec)) vec >>= 1;
     const int64_t nvec = (row_len + vec - 1) / vec;
-    int group, nv;
-    auto p2 = [](int64_t x) {
-        int64_t r = 1;
-        while (r < x) r <<= 1;
-        return (int)r;
+    if (nvec > 256 * 16) return fail(XTG_ERR_UNSUPPORTED, "row too long for the fused row kernel");
+    // Lanes per row: the narrowest group of a warp that leaves a lane at most
+    // `most` elements, so that a warp's shuffles, divisions and square roots
+    // serve 32 / group rows.  More elements per lane pay where those cost most
+    // (float64: rows of 321 take 333 / 261 us at 16 / 32 per lane) and with
+    // rows at any element, whose loads and stores are single elements (float32
+    // rows of 131: 81 / 54 / 50 us at 16 / 32 / 48); whole vectors of float32
+    // run best at 16 (rows of 256: 88 us, 95 at 32).  Single elements want
+    // groups of 4 at least: a store of 16 rows x 2 elements touches 16 sectors
+    // (float32 rows of 51: 85 us, 184 with pairs), vectors do not (rows of 16:
+    // 46 us with a lane per row, 77 with 4).
+    const int64_t most = maxsz >= 8 ? 32 : (vec > 1 ? 16 : 48);
+    int group = vec > 1 ? 1 : 4;
+    while (group < 32 && nvec * vec > group * most) group *= 2;
+    if (nvec > 32 * 16) group = 256;
+    // A lane's vectors of the row, rounded up in steps that keep the number
+    // of kernels for all row lengths small; the first `nf` of them lie inside
+    // the row for every lane.
+    auto lane_vecs = [&](int g, int& nf) {
+        const int need = (int)((nvec + g - 1) / g);
+        const int step = need <= 8 ? 1 : (need <= 16 ? 2 : (need <= 32 ? 4 : 8));
+        const int nv = (need + step - 1) / step * step;
+        nf = (int64_t)nv * g == nvec ? nv : nv - step;
+        return nv;
     };
-    if (nvec <= 32 * 16) {
-        group = 32;
-        nv = p2((nvec + 31) / 32);
-    } else if (nvec <= 256 * 16) {
-        group = 256;
-        nv = p2((nvec + 255) / 256);
-    } else {
-        return fail(XTG_ERR_UNSUPPORTED, "row too long for the fused row kernel");
-    }
     xtg::RowParams p;
     memset(&p, 0, sizeof p);
     p.n_rows = n_rows;
@@ -424,54 +434,78 @@ static xtg_status assign_rowfused(const Tree& t, const xtg_array& out, int R, co
     const int recip = (opt("row.recip_div_f64", 1) != 0 ? 1 : 0) | (opt("row.recip_div_f32", 1) != 0 ? 2 : 0);
     int nstat = t.n_rstats;  // real statistics, then the reciprocal nodes' row-invariant slots
     const std::string tree = tree_type(t, t.root, map, recip, &nstat);
-    const int full = (int64_t)nv * group * vec == row_len ? 1 : 0;
 
-    // Bulk-copy variant: every leaf contiguous along the row, 16-byte rows,
-    // warp-sized groups, output contiguous along the row.
-    bool tma = opt("row.tma", 1) != 0 && group == 32 && li[0] == 1 && NL > 0;
-    unsigned buf_bytes = 0;
+    // Bulk-copy variant: every leaf contiguous along the row (with several
+    // rows per warp also from row to row), the output contiguous along the
+    // row.  Rows that do not start and end at 16-byte boundaries go through
+    // the EDGE form.
+    int tgroup = group;
+    bool edge = false;
+    bool tma = opt("row.tma", 1) != 0 && li[0] == 1 && NL > 0;
+    int64_t row_bytes = 0;  // of the widest leaf
     for (int l = 0; tma && l < NL; ++l) {
         const int sz = dt(t.leaves[l].dtype).size;
         const int64_t rb = row_len * sz;
-        if (kinds[l] != 0 || rb % 16 || !aligned(t.leaves[l].data, 16)) tma = false;
+        row_bytes = std::max(row_bytes, rb);
+        if (kinds[l] != 0 || rb < 16 || !aligned(t.leaves[l].data, sz)) tma = false;
+        if (rb % 16 || !aligned(t.leaves[l].data, 16)) edge = true;
         for (int d = 0; tma && d < D.R; ++d)
-            if ((D.st[1 + l][d] * sz) % 16) tma = false;
-        if (tma) {
-            p.loff[l] = buf_bytes;
-            p.lbytes[l] = (unsigned)rb;
-            buf_bytes += (unsigned)rb;
-        }
+            if ((D.st[1 + l][d] * sz) % 16) edge = true;
+        if (n_rows > 1 && (D.R != 1 || D.st[1 + l][0] != row_len)) tgroup = std::max(tgroup, 32);
+    }
+    // A block per row above 8 KiB: a warp's lanes would hold over 64 registers
+    // of the row each, and a buffer per warp leave few warps resident (60000
+    // float64 rows of 2048: 648 us with a warp, 455 with a block).
+    if (tgroup == 256) tgroup = row_bytes > 8192 ? 128 : 32;
+    const int nbuf = opt("row.tma_buffers", 1) == 2 && tgroup == 32 && !edge ? 2 : 1;
+    const int unit_rows = tgroup < 32 ? 32 / tgroup : 1;
+    unsigned buf_bytes = 0;
+    for (int l = 0; tma && l < NL; ++l) {
+        const int sz = dt(t.leaves[l].dtype).size;
+        p.loff[l] = buf_bytes;
+        p.lbytes[l] = (unsigned)(row_len * sz);
+        p.lsize[l] = (unsigned)sz;
+        const int64_t ub = unit_rows * row_len * sz;
+        buf_bytes += (unsigned)((edge ? ub + 31 : ub + 15) / 16 * 16);
     }
     const int tma_block = 128;
+    const int owners = tgroup > 32 ? 1 : tma_block / 32;
     // One buffer per warp by default (refilled once the row is in registers),
     // and a register cap that leaves room for 5 blocks per SM when a lane's
     // share of the row takes at most 64 registers (float64 rows of 1024: 376
     // us per 2^27 elements with 96 registers; 388 at 4 blocks, 422 at 3,
     // 519 uncapped with two buffers — the compiler then spends ~210
     // registers; 6 blocks spill).
-    const int nbuf = opt("row.tma_buffers", 1) == 2 ? 2 : 1;
+    int tnf = 0;
+    const int tnv = lane_vecs(tgroup, tnf);
     int64_t row_regs = 0;
-    for (int l = 0; l < NL; ++l) row_regs += (int64_t)nv * vec * dt(t.leaves[l].dtype).size / 4;
-    const int64_t minb_auto = row_regs <= 64 ? 5 : (row_regs <= 96 ? 3 : 2);
+    for (int l = 0; l < NL; ++l) row_regs += (int64_t)tnv * vec * dt(t.leaves[l].dtype).size / 4;
+    int64_t minb_auto = row_regs <= 64 ? 5 : (row_regs <= 96 ? 3 : 2);
+    // short rows: more units in flight (float64 rows of 64: 233 us at 5, 223 at 8)
+    if (tgroup < 32 && row_regs <= 32) minb_auto = 8;
     const int minb = (int)std::max<int64_t>(1, std::min<int64_t>(opt("row.tma_min_blocks", minb_auto), 16));
-    const size_t dyn = (size_t)buf_bytes * nbuf * (tma_block / 32);
+    const size_t dyn = (size_t)buf_bytes * nbuf * owners;
     if (tma && dyn > 200 * 1024) tma = false;
     if (tma) {
         p.buf_bytes = buf_bytes;
         XTG_TRY(device_error_word(&p.err));
         std::string name = "xtg::k_rowfused_tma<" + tree + ", " + sl + ", " + leafset(t, order, kinds) + ", " +
-                           dt(out.dtype).cname + ", " + std::to_string(vec) + ", " + std::to_string(nv) + ", " +
-                           std::to_string(D.R) + ", " + std::to_string(nstat) + ", " + std::to_string(full) + ", " +
+                           dt(out.dtype).cname + ", " + std::to_string(vec) + ", " + std::to_string(tnv) + ", " +
+                           std::to_string(D.R) + ", " + std::to_string(nstat) + ", " + std::to_string(tnf) + ", " +
+                           std::to_string(tgroup) + ", " + (edge ? "true" : "false") + ", " +
                            std::to_string(nbuf) + ", " + std::to_string(minb) + ">";
         Kernel* kr;
         XTG_TRY(get_kernel(name, tma_block, &kr, dyn));
-        int64_t need = (n_rows + 3) / 4;
-        return launch(kr, grid_for(kr, need), tma_block, &p, stream, dyn);
+        const int64_t units = (n_rows + unit_rows - 1) / unit_rows;
+        return launch(kr, grid_for(kr, (units + owners - 1) / owners), tma_block, &p, stream, dyn);
     }
+    int nf = 0;
+    group = std::max(group, 4);  // a warp's loads from global memory: at least 4 neighbours per row
+    const int nv = lane_vecs(group, nf);
     std::string name = "xtg::k_rowfused<" + tree + ", " + sl + ", " + leafset(t, order, kinds) + ", " +
                        dt(out.dtype).cname + ", " + std::to_string(vec) + ", " + std::to_string(nv) + ", " +
                        std::to_string(group) + ", " + std::to_string(D.R) + ", " + std::to_string(nstat) + ", " +
-                       std::to_string(full) + ">";
+                       std::to_string(nf) + ">";
     const int block = 256;
     Kernel* kr;
     XTG_TRY(get_kernel(name, block, &kr));

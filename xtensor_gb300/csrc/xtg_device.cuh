@@ -554,12 +554,12 @@ __global__ void __launch_bounds__(256) k_assign_chunks(const ChunkParams p) {
 
 // ---------------------------------------------------------------------------
 // Generic warp shuffle of a POD accumulator (word by word).
-template <class A> XTG_DI A shfl_xor_pod(const A& a, int m) {
+template <class A> XTG_DI A shfl_xor_pod(const A& a, int m, unsigned mask = 0xffffffffu) {
     union U { A a; u32 w[(sizeof(A) + 3) / 4]; };
     U in, out;
     in.a = a;
 #pragma unroll
-    for (int i = 0; i < (int)((sizeof(A) + 3) / 4); ++i) out.w[i] = __shfl_xor_sync(0xffffffffu, in.w[i], m);
+    for (int i = 0; i < (int)((sizeof(A) + 3) / 4); ++i) out.w[i] = __shfl_xor_sync(mask, in.w[i], m);
     return out.a;
 }
 
@@ -581,13 +581,22 @@ template <class A> XTG_DI A shfl_idx_pod(const A& a, int src) {
     return out.a;
 }
 
-// Deterministic group reduction: warp butterfly, then warp 0 folds the
-// per-warp results in warp order.  Result valid in thread 0 of the group
-// (GROUP == 32: lane 0 of the warp; GROUP == block: thread 0).
+// Lanes of the caller's group in its warp: the groups of a warp may be at
+// different branches (a row that needs its exact pass), so a group of fewer
+// than 32 lanes names only its own lanes in a shuffle.
+template <int GROUP> XTG_DI unsigned group_mask() {
+    if (GROUP >= 32) return 0xffffffffu;
+    return ((1u << (GROUP & 31)) - 1u) << ((threadIdx.x & 31) & ~(unsigned)(GROUP - 1));
+}
+// Deterministic group reduction: warp butterfly over min(GROUP, 32) lanes,
+// then (GROUP > 32: the whole block) warp 0 folds the per-warp results in
+// warp order.  Result valid in every lane of a group of at most 32, in
+// thread 0 of a block.
 template <int GROUP, class A> XTG_DI A group_reduce(A a, A* smem) {
+    const unsigned mask = group_mask<GROUP>();
 #pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) {
-        A o = shfl_xor_pod(a, m);
+    for (int m = GROUP < 32 ? GROUP / 2 : 16; m >= 1; m >>= 1) {
+        A o = shfl_xor_pod(a, m, mask);
         a.merge(o);
     }
     if (GROUP <= 32) return a;
@@ -3409,19 +3418,21 @@ template <int K, int MODE, class C, class Sub, class... Rest> struct Stats<StatL
     }
 };
 
-// FULL: row_len == NV * group size * VEC, so no element needs a bounds mask.
-template <class Tree, class SL, class LS, class OutT, int VEC, int NV, int GROUP, int RO, int NSTAT, int FULL>
+// NF: the first NF of a lane's NV vectors lie inside the row for every lane
+// (no bounds mask).  GROUP: lanes per row, 4 .. 32 of a warp or a block of 256.
+template <class Tree, class SL, class LS, class OutT, int VEC, int NV, int GROUP, int RO, int NSTAT, int NF>
 __global__ void __launch_bounds__(256) k_rowfused(const RowParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
     __shared__ __align__(16) unsigned char smem_raw[32 * 48];
     Ctx<NSTAT> c;
     c.scal = p.scal;
-    const int gsz = GROUP <= 32 ? 32 : (int)blockDim.x;
+    const int gsz = GROUP <= 32 ? GROUP : (int)blockDim.x;
     const int gpb = (int)blockDim.x / gsz;
     const int gt = (int)threadIdx.x % gsz;
     const i64 gid = (i64)blockIdx.x * gpb + (int)threadIdx.x / gsz;
     const i64 ng = (i64)gridDim.x * gpb;
+    const int len = (int)p.row_len;
     for (i64 row = gid; row < p.n_rows; row += ng) {
         i64 ko[RO];
         decode_dims<RO, true>(p.oshape, (const FastDiv*)0, row, ko);
@@ -3437,10 +3448,10 @@ __global__ void __launch_bounds__(256) k_rowfused(const RowParams p) {
         bool ok[NV][VEC];
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const i64 e0 = ((i64)n * gsz + gt) * VEC;
+            const int e0 = (n * gsz + gt) * VEC;
 #pragma unroll
-            for (int j = 0; j < VEC; ++j) ok[n][j] = FULL || (e0 + j) < p.row_len;
-            if (FULL || e0 < p.row_len) {
+            for (int j = 0; j < VEC; ++j) ok[n][j] = n < NF || (e0 + j) < len;
+            if (n < NF || e0 < len) {
                 i64 off[XTG_KMAX_LEAVES];
 #pragma unroll
                 for (int l = 0; l < LS::N; ++l) off[l] = base[l] + e0 * p.li[l];
@@ -3455,8 +3466,8 @@ __global__ void __launch_bounds__(256) k_rowfused(const RowParams p) {
         for (int d = 0; d < RO; ++d) ob += ko[d] * p.oo[d];
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const i64 e0 = ((i64)n * gsz + gt) * VEC;
-            if (FULL || e0 < p.row_len) {
+            const int e0 = (n * gsz + gt) * VEC;
+            if (n < NF || e0 < len) {
                 OutT v[VEC];
 #pragma unroll
                 for (int j = 0; j < VEC; ++j) v[j] = cvt<OutT>(Tree::ev(rg[n], j, c));
@@ -3467,13 +3478,19 @@ __global__ void __launch_bounds__(256) k_rowfused(const RowParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// K7 with bulk copies.  Each warp owns rows; the rows of every leaf stream
-// into a per-warp buffer in shared memory (one, or a double buffer) with one
-// cp.async.bulk per leaf per row (the TMA engine's 1-D bulk copy, completion
-// counted in bytes on an mbarrier), issued one row ahead, so HBM reads of row
-// i+1 overlap the statistics and the stores of row i.  Requires every leaf to
-// be contiguous along the row, rows 16-byte aligned and a multiple of 16
-// bytes.
+// K7 with bulk copies.  A unit of work is one row (GROUP 32: a warp's,
+// GROUP 128: a block's) or the 32 / GROUP consecutive rows that a warp's
+// groups of 4 .. 16 lanes take; the unit of every leaf streams into a buffer
+// in shared memory (one, or a double buffer) with one cp.async.bulk per leaf
+// (the TMA engine's 1-D bulk copy, completion counted in bytes on an
+// mbarrier), issued one unit ahead, so HBM reads of the next unit overlap
+// the statistics and the stores of this one.  Requires every leaf to be
+// contiguous along the row and, with several rows per unit, from row to row.
+// EDGE: a unit may start and end at any element.  The copy takes its whole
+// 16-byte granules; the elements before and after them (under 16 bytes
+// each) are loaded into registers by the lanes at the time of issue and
+// stored beside the copied bytes before the unit is read, at the offset
+// that keeps shared and global addresses equal modulo 16.
 XTG_DI unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 XTG_DI void mbar_init(u64* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -3726,52 +3743,162 @@ template <class... S> struct LoadRowSmem<LeafSet<S...>> {
     }
 };
 
-// NB = 2: a double buffer per warp, row i + 1 copied while row i is reduced
-// from shared memory.  NB = 1: one buffer per warp, refilled with row i + 1
-// as soon as row i sits in registers (half the shared memory, so more warps
-// per SM).  MINB: the launch-bounds minimum of resident blocks per SM.
-template <class Tree, class SL, class LS, class OutT, int VEC, int NV, int RO, int NSTAT, int FULL, int NB = 2, int MINB = 1>
+// The first and last elements of a unit that lie outside its whole 16-byte
+// granules: lanes 0 .. 15 hold the head, lanes 16 .. 31 the tail (raw bits,
+// one register pair per leaf at most).
+template <int I, class... S> struct RowEdge;
+template <int I> struct RowEdge<I> {
+    template <class A> static XTG_DI void load(u64*, const A&, const unsigned*, int) {}
+    template <class A> static XTG_DI void store(const u64*, const A&, const unsigned*, unsigned char*, const unsigned*, int) {}
+};
+template <int I, class S0, class... S> struct RowEdge<I, S0, S...> {
+    typedef typename S0::type T;
+    // this lane's element as a byte offset into the unit, or -1
+    static XTG_DI int place(const unsigned char* a, unsigned bytes, int lane) {
+        const unsigned ph = (unsigned)((u64)a & 15);
+        const unsigned head = (16 - ph) & 15, tail = (ph + bytes) & 15;
+        const unsigned k = (unsigned)(lane & 15) * (unsigned)sizeof(T);
+        if (lane < 16) return k < head ? (int)k : -1;
+        return k < tail ? (int)(bytes - tail + k) : -1;
+    }
+    template <class A> static XTG_DI void load(u64* ev, const A& src, const unsigned* bytes, int lane) {
+        const int at = place(src[I], bytes[I], lane);
+        if (at >= 0) {
+            union { T t; u64 u; } x;
+            x.u = 0;
+            x.t = *reinterpret_cast<const T*>(src[I] + at);
+            ev[I] = x.u;
+        }
+        RowEdge<I + 1, S...>::load(ev, src, bytes, lane);
+    }
+    template <class A>
+    static XTG_DI void store(const u64* ev, const A& src, const unsigned* bytes, unsigned char* buf, const unsigned* loff, int lane) {
+        const int at = place(src[I], bytes[I], lane);
+        if (at >= 0) {
+            union { T t; u64 u; } x;
+            x.u = ev[I];
+            *reinterpret_cast<T*>(buf + loff[I] + (unsigned)((u64)src[I] & 15) + at) = x.t;
+        }
+        RowEdge<I + 1, S...>::store(ev, src, bytes, buf, loff, lane);
+    }
+};
+template <class LS> struct RowEdges;
+template <class... S> struct RowEdges<LeafSet<S...>> {
+    typedef RowEdge<0, S...> E;
+};
+
+// NB = 2 (GROUP 32 without EDGE): a double buffer per warp, row i + 1 copied
+// while row i is reduced from shared memory.  NB = 1: one buffer, refilled
+// with the next unit as soon as this one sits in registers (half the shared
+// memory, so more warps per SM).  MINB: the launch-bounds minimum of resident
+// blocks per SM.  NF: the first NF of a lane's NV vectors lie inside the row
+// for every lane.
+template <class Tree, class SL, class LS, class OutT, int VEC, int NV, int RO, int NSTAT, int NF, int GROUP, bool EDGE,
+          int NB = 2, int MINB = 1>
 __global__ void __launch_bounds__(128, MINB) k_rowfused_tma(const RowParams p) {
     pdl_wait();
+    static_assert(NB == 1 || (GROUP == 32 && !EDGE), "the double buffer is the aligned one-row form");
     typedef typename LS::template R<VEC>::type RG;
+    constexpr bool BLK = GROUP > 32;          // a block of 128 per row
+    constexpr int UR = BLK ? 1 : 32 / GROUP;  // rows per unit
     extern __shared__ __align__(128) unsigned char dsmem[];
     __shared__ __align__(16) unsigned char red_smem[32 * 48];
     __shared__ u64 bars[8];
     const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
-    const int nw = (int)blockDim.x >> 5;
-    u64* mybar = bars + 2 * warp;
-    unsigned char* const buf0 = dsmem + (size_t)(NB * warp) * p.buf_bytes;  // buffer b at buf0 + b * buf_bytes
-    if (lane == 0) {
+    const int owner = BLK ? 0 : warp;  // whose buffer and barrier
+    const int nw = BLK ? 1 : (int)blockDim.x >> 5;
+    const int gl = BLK ? (int)threadIdx.x : lane % GROUP;  // lane in the row's group
+    const bool copier = BLK ? threadIdx.x == 0 : lane == 0;
+    auto sync = [&]() {
+        if (BLK) __syncthreads();
+        else __syncwarp();
+    };
+    u64* mybar = bars + 2 * owner;
+    unsigned char* const buf0 = dsmem + (size_t)(NB * owner) * p.buf_bytes;  // buffer b at buf0 + b * buf_bytes
+    if (copier) {
         mbar_init(&mybar[0], 1);
         mbar_init(&mybar[1], 1);
         fence_mbar_init();
     }
-    __syncwarp();
+    sync();
     Ctx<NSTAT> c;
     c.scal = p.scal;
-    const i64 gid = (i64)blockIdx.x * nw + warp;
+    const int len = (int)p.row_len;
+    const i64 n_units = (p.n_rows + UR - 1) / UR;
+    const i64 gid = (i64)blockIdx.x * nw + owner;
     const i64 ng = (i64)gridDim.x * nw;
-    auto issue = [&](i64 row, int b) {
-        if (lane == 0) {
-            i64 ko[RO];
-            decode_dims<RO, true>(p.oshape, (const FastDiv*)0, row, ko);
-            mbar_expect_tx(&mybar[b], p.buf_bytes);
+    u64 edge[XTG_KMAX_LEAVES];
+    // first byte and bytes of a unit of every leaf
+    auto place = [&](i64 unit, const unsigned char* (&src)[XTG_KMAX_LEAVES], unsigned(&bytes)[XTG_KMAX_LEAVES]) {
+        const i64 row = unit * UR;
+        i64 ko[RO];
+        decode_dims<RO, true>(p.oshape, (const FastDiv*)0, row, ko);
+        const unsigned rows = UR == 1 ? 1u : (unsigned)(p.n_rows - row < UR ? p.n_rows - row : UR);
+#pragma unroll
+        for (int l = 0; l < LS::N; ++l) {
+            i64 o = 0;
+#pragma unroll
+            for (int d = 0; d < RO; ++d) o += ko[d] * p.lo[l][d];
+            src[l] = reinterpret_cast<const unsigned char*>(p.leaf[l]) + o * p.lsize[l];
+            bytes[l] = rows * p.lbytes[l];
+        }
+    };
+    auto issue = [&](i64 unit, int b) {
+        if (!copier && !(EDGE && warp == owner)) return;
+        const unsigned char* src[XTG_KMAX_LEAVES];
+        unsigned bytes[XTG_KMAX_LEAVES];
+        place(unit, src, bytes);
+        if (EDGE) RowEdges<LS>::E::load(edge, src, bytes, lane);
+        if (!copier) return;
+        if (!EDGE) {
+            unsigned total = 0;
+#pragma unroll
+            for (int l = 0; l < LS::N; ++l) total += bytes[l];
+            mbar_expect_tx(&mybar[b], total);
+#pragma unroll
+            for (int l = 0; l < LS::N; ++l)
+                bulk_g2s(buf0 + (size_t)b * p.buf_bytes + p.loff[l], src[l], bytes[l], &mybar[b]);
+        } else {
+            // whole granules [lo, hi) of each leaf's unit (a unit has at least 16 bytes, so hi >= lo)
+            unsigned total = 0;
 #pragma unroll
             for (int l = 0; l < LS::N; ++l) {
-                i64 o = 0;
+                const u64 a = (u64)src[l];
+                total += (unsigned)(((a + bytes[l]) & ~15ull) - ((a + 15) & ~15ull));
+            }
+            mbar_expect_tx(&mybar[b], total);
 #pragma unroll
-                for (int d = 0; d < RO; ++d) o += ko[d] * p.lo[l][d];
-                const unsigned char* src = reinterpret_cast<const unsigned char*>(p.leaf[l]) + o * (p.lbytes[l] / p.row_len);
-                bulk_g2s(buf0 + (size_t)b * p.buf_bytes + p.loff[l], src, p.lbytes[l], &mybar[b]);
+            for (int l = 0; l < LS::N; ++l) {
+                const u64 a = (u64)src[l];
+                const u64 lo = (a + 15) & ~15ull, hi = (a + bytes[l]) & ~15ull;
+                if (hi > lo)
+                    bulk_g2s(buf0 + p.loff[l] + ((unsigned)(a & 15) + (unsigned)(lo - a)), (const void*)lo,
+                             (unsigned)(hi - lo), &mybar[b]);
             }
         }
     };
     int it = 0;
-    if (gid < p.n_rows) issue(gid, 0);
-    for (i64 row = gid; row < p.n_rows; row += ng, ++it) {
+    if (gid < n_units) issue(gid, 0);
+    for (i64 unit = gid; unit < n_units; unit += ng, ++it) {
         const int b = NB == 2 ? (it & 1) : 0;
-        if (NB == 2 && row + ng < p.n_rows) issue(row + ng, b ^ 1);
+        if (NB == 2 && unit + ng < n_units) issue(unit + ng, b ^ 1);
         const unsigned parity = NB == 2 ? ((unsigned)(it >> 1) & 1u) : ((unsigned)it & 1u);
+        unsigned loff[XTG_KMAX_LEAVES];
+        const i64 row = unit * UR + (BLK ? 0 : lane / GROUP);
+        {
+            const unsigned char* src[XTG_KMAX_LEAVES];
+            unsigned bytes[XTG_KMAX_LEAVES];
+            if (EDGE) {
+                place(unit, src, bytes);
+                if (warp == owner) RowEdges<LS>::E::store(edge, src, bytes, buf0, p.loff, lane);
+            }
+#pragma unroll
+            for (int l = 0; l < LS::N; ++l) {
+                loff[l] = p.loff[l];
+                if (EDGE) loff[l] += (unsigned)((u64)src[l] & 15);
+                if (UR > 1) loff[l] += (unsigned)(lane / GROUP) * p.lbytes[l];
+            }
+        }
         bool done = false;
         for (int k = 0; k < (1 << 22); ++k) {
             if (mbar_try_wait(&mybar[b], parity)) {
@@ -3779,40 +3906,45 @@ __global__ void __launch_bounds__(128, MINB) k_rowfused_tma(const RowParams p) {
                 break;
             }
         }
-        // one decision for the whole warp: a lane that gave up must not
-        // leave while the others go on into full-mask shuffles
-        done = __all_sync(0xffffffffu, done);
+        // one decision for everyone who shares the buffer: a lane that gave
+        // up must not leave while the others go on into full shuffles
+        // (this is also the barrier that makes the edge elements visible)
+        if (BLK) done = __syncthreads_and(done) != 0;
+        else done = __all_sync(0xffffffffu, done) != 0;
+        if (EDGE && !BLK) __syncwarp();
         if (!done) {
             // give up: flag it, wait (bounded) for the copy into the other
             // buffer if one was issued, and leave.  The copy that timed out
             // may still be in flight into this block's shared memory when
             // the block exits; the error word tells the host that the
             // launch's results (and the device state) are not to be trusted.
-            if (lane == 0) atomicExch(p.err, 1);
-            if (NB == 2 && row + ng < p.n_rows) {
+            if (copier) atomicExch(p.err, 1);
+            if (NB == 2 && unit + ng < n_units) {
                 const unsigned par2 = (unsigned)((it + 1) >> 1) & 1u;
                 for (int k = 0; k < (1 << 22); ++k)
                     if (mbar_try_wait(&mybar[b ^ 1], par2)) break;
             }
             return;
         }
+        const bool live = UR == 1 || row < p.n_rows;
         RG rg[NV];
         bool ok[NV][VEC];
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const i64 e0 = ((i64)n * 32 + lane) * VEC;
+            const int e0 = (n * GROUP + gl) * VEC;
 #pragma unroll
-            for (int j = 0; j < VEC; ++j) ok[n][j] = FULL || (e0 + j) < p.row_len;
-            if (FULL || e0 < p.row_len) LoadRowSmem<LS>::template run<VEC>(rg[n], buf0 + (size_t)b * p.buf_bytes, p.loff, e0);
+            for (int j = 0; j < VEC; ++j) ok[n][j] = live && (n < NF || (e0 + j) < len);
+            if (live && (n < NF || e0 < len))
+                LoadRowSmem<LS>::template run<VEC>(rg[n], buf0 + (size_t)b * p.buf_bytes, loff, e0);
         }
         if (NB == 1) {
-            // the row is in registers: refill the buffer with the next one
+            // the unit is in registers: refill the buffer with the next one
             fence_proxy_async_smem();
-            __syncwarp();
-            if (row + ng < p.n_rows) issue(row + ng, 0);
+            sync();
+            if (unit + ng < n_units) issue(unit + ng, 0);
         }
         c.fixmask = 0;
-        Stats<SL>::template run<32, VEC, NV>(rg, ok, c, p, (void*)red_smem);
+        Stats<SL>::template run<GROUP, VEC, NV>(rg, ok, c, p, (void*)red_smem);
         Prep<Tree>::run(rg[0], c);
         i64 ko[RO];
         decode_dims<RO, true>(p.oshape, (const FastDiv*)0, row, ko);
@@ -3821,8 +3953,8 @@ __global__ void __launch_bounds__(128, MINB) k_rowfused_tma(const RowParams p) {
         for (int d = 0; d < RO; ++d) ob += ko[d] * p.oo[d];
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const i64 e0 = ((i64)n * 32 + lane) * VEC;
-            if (FULL || e0 < p.row_len) {
+            const int e0 = (n * GROUP + gl) * VEC;
+            if (live && (n < NF || e0 < len)) {
                 OutT v[VEC];
 #pragma unroll
                 for (int j = 0; j < VEC; ++j) v[j] = cvt<OutT>(Tree::ev(rg[n], j, c));

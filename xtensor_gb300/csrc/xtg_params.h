@@ -142,7 +142,8 @@ struct RowParams {
     float frow_len;             // row_len as float
     // bulk-copy (TMA) variant: per-warp buffer layout in shared memory
     unsigned loff[XTG_KMAX_LEAVES];   // byte offset of each leaf's row inside a buffer
-    unsigned lbytes[XTG_KMAX_LEAVES]; // bytes of one row of each leaf (multiple of 16)
+    unsigned lbytes[XTG_KMAX_LEAVES]; // bytes of one row of each leaf
+    unsigned lsize[XTG_KMAX_LEAVES];  // bytes of one element of each leaf
     unsigned buf_bytes;               // bytes of one buffer (all leaves)
     int* err;                         // set to 1 when a bounded wait gives up
 };
