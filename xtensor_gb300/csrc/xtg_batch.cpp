@@ -303,6 +303,7 @@ xtg_status xtg_batch_add(xtg_batch* b, const xtg_array* leaves, int32_t n_leaves
         if (out->rank == 2 && out->shape[0] == 1) I.ors = out->strides[1];
         I.ocs = 0;
         I.divisor = (double)cols;
+        I.rdivisor = 1.0 / I.divisor;
         bytes += rows * dt(out->dtype).size;
     } else {
         if (out->rank == 2) {

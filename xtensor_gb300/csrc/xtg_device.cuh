@@ -821,6 +821,12 @@ template <class A, int MAXOP> struct AccSelFast {
         const bool keep = MAXOP ? Cmp<A>::gt(v, a) : Cmp<A>::lt(v, a);
         if (!keep) v = a;
     }
+    XTG_DI void merge(const AccSelFast& o) {
+        odd |= o.odd;
+        const bool keep = MAXOP ? Cmp<A>::gt(v, o.v) : Cmp<A>::lt(v, o.v);
+        if (!keep) v = o.v;
+    }
+    XTG_DI bool nan() const { return odd; }
     XTG_DI bool exact() const { return odd || (IsFloat<A>::value && v == A(0)); }
     XTG_DI void to(AccSel<A, MAXOP>& s) const {
         s.v = v;
@@ -840,6 +846,8 @@ template <int MAXOP> struct AccSelFast<float, MAXOP> {
     float v;
     template <class P> XTG_DI void init(const P& p) { v = (float)p.init_f; }
     template <class X> XTG_DI void add(X x, i64) { v = fsel_nan(v, cvt<float>(x), MAXOP); }
+    XTG_DI void merge(const AccSelFast& o) { v = fsel_nan(v, o.v, MAXOP); }
+    XTG_DI bool nan() const { return !(v == v); }
     XTG_DI bool exact() const { return !(v == v) || v == 0.f; }
     XTG_DI void to(AccSel<float, MAXOP>& s) const {
         s.v = v;
@@ -868,6 +876,12 @@ template <int MAXOP> struct AccSelFast<double, MAXOP> {
         const i64 ka = key64(b);
         if (MAXOP ? (ka >= kv) : (ka <= kv)) kv = ka;
     }
+    XTG_DI void merge(const AccSelFast& o) {
+        mh = mh > o.mh ? mh : o.mh;
+        odd |= o.odd;
+        if (MAXOP ? (o.kv >= kv) : (o.kv <= kv)) kv = o.kv;
+    }
+    XTG_DI bool nan() const { return mh >= 0x7ff00000u; }  // (or an infinity)
     XTG_DI bool exact() const { return odd || mh >= 0x7ff00000u || kv == 0 || kv == -1; }
     XTG_DI void to(AccSel<double, MAXOP>& s) const {
         s.kv = kv;
@@ -1287,6 +1301,93 @@ template <int MAXOP> struct AccArg<double, MAXOP> {
     }
 };
 
+// The fast pass of an arg-reduction over a row (as AccSelFast for amax /
+// amin): the strict compare and two selects per element, positions as 32-bit
+// offsets, from the type's lowest (highest) value at the lane's first
+// position; equal values keep the smaller position.  A NaN anywhere (it is
+// only ever taken as the very first element) and, for float64 keys, an
+// infinity or a best value of zero ask for the exact pass.
+template <class A, int MAXOP> struct AccArgFast {
+    A v;
+    u32 off;
+    bool odd;
+    template <class P> XTG_DI void init(const P&) {
+        v = ends();
+        off = 0xffffffffu;
+        odd = false;
+    }
+    static XTG_DI A ends() {  // what nothing but a NaN is below (above)
+        if constexpr (IsFloat<A>::value) return MAXOP ? A(-__int_as_float(0x7f800000)) : A(__int_as_float(0x7f800000));
+        else return MAXOP ? Lim<A>::lowest() : Lim<A>::maxv();
+    }
+    XTG_DI void start_at(u32 first) { off = first; }
+    template <class X> XTG_DI void add(X x, i64 ps) {
+        const A a = cvt<A>(x);
+        if (IsFloat<A>::value) odd |= !(a == a);
+        if (MAXOP ? Cmp<A>::gt(a, v) : Cmp<A>::lt(a, v)) {
+            v = a;
+            off = (u32)ps;
+        }
+    }
+    XTG_DI void merge(const AccArgFast& o) {
+        odd |= o.odd;
+        const bool better = MAXOP ? Cmp<A>::gt(o.v, v) : Cmp<A>::lt(o.v, v);
+        const bool worse = MAXOP ? Cmp<A>::gt(v, o.v) : Cmp<A>::lt(v, o.v);
+        if (better || (!worse && o.off < off)) {
+            v = o.v;
+            off = o.off;
+        }
+    }
+    XTG_DI bool nan() const { return false; }  // the exact pass does not depend on the order
+    XTG_DI bool exact() const { return odd; }
+    XTG_DI void to(AccArg<A, MAXOP>& s) const {
+        s.v = v;
+        s.idx = off;
+    }
+};
+template <int MAXOP> struct AccArgFast<double, MAXOP> {
+    i64 kv;
+    u32 off;
+    unsigned mh;  // largest (high word & 0x7fffffff) seen
+    template <class P> XTG_DI void init(const P&) {
+        kv = MAXOP ? XTG_KEY_MIN : XTG_KEY_MAX;
+        off = 0xffffffffu;
+        mh = 0;
+    }
+    XTG_DI void start_at(u32 first) { off = first; }
+    template <class X> XTG_DI void add(X x, i64 ps) {
+        const i64 b = __double_as_longlong(cvt<double>(x));
+        const unsigned h = (unsigned)(b >> 32) & 0x7fffffffu;
+        mh = mh > h ? mh : h;
+        const i64 ka = key64(b);
+        if (MAXOP ? (ka > kv) : (ka < kv)) {
+            kv = ka;
+            off = (u32)ps;
+        }
+    }
+    XTG_DI void merge(const AccArgFast& o) {
+        mh = mh > o.mh ? mh : o.mh;
+        if ((MAXOP ? (o.kv > kv) : (o.kv < kv)) || (o.kv == kv && o.off < off)) {
+            kv = o.kv;
+            off = o.off;
+        }
+    }
+    XTG_DI bool nan() const { return false; }
+    XTG_DI bool exact() const { return mh >= 0x7ff00000u || kv == 0 || kv == -1; }
+    XTG_DI void to(AccArg<double, MAXOP>& s) const {
+        s.kv = kv;
+        s.idx = off;
+    }
+};
+template <class A, int M> struct FastSel<AccArg<A, M>> { enum { value = 1 }; typedef AccArgFast<A, M> F; };
+// The fast pass of a row starts at the lane's first position.
+template <class F> struct FastStart {
+    static XTG_DI void at(F&, u32) {}
+};
+template <class A, int M> struct FastStart<AccArgFast<A, M>> {
+    static XTG_DI void at(AccArgFast<A, M>& f, u32 first) { f.start_at(first); }
+};
+
 // ---------------------------------------------------------------------------
 // Reduction parameters.  Output space = kept dims (rank RO), reduced space =
 // reduced dims (rank RR).  For the ROW strategy the innermost reduced dim is
@@ -1359,6 +1460,25 @@ template <class Tree, class Acc, int VEC> struct ColStep {
     }
 };
 
+// a / b for a divisor b that is the same in the whole launch, r = 1 / b rounded
+// to nearest (the host's): q = a r is within 2 ulp, a first remainder and
+// correction bring it within 1, and from there the second gives the correctly
+// rounded quotient (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990; the one exception, a
+// divisor whose 53 significand bits are all ones, is no count of elements).
+// Five FP64 operations.  Zeros, infinities, NaNs and values near the ends of
+// the range, where a remainder could be inexact, divide.
+XTG_DI double div_by(double a, double b, double r) {
+    const double q = a * r;
+    const unsigned eq = ((unsigned)__double2hiint(q) >> 20) & 0x7ff;
+    const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ff;
+    if (eq - 128u < 1792u && ea - 128u < 1792u) {
+        const double q1 = fma(fma(-q, b, a), r, q);
+        return fma(fma(-q1, b, a), r, q1);
+    }
+    return a / b;
+}
+
 // Finalisation: accumulator state -> output element (merging xt::initial
 // last, as xreducer_stepper::aggregate does, xreducer.hpp:1778-1799).
 template <class Out, class A> struct Fin;
@@ -1403,11 +1523,10 @@ template <class Out, class C, int MODE> struct Fin<Out, AccMom<C, MODE>> {
     template <class P> static XTG_DI Out go(const AccMom<C, MODE>& a, const P& p) {
         double s1, s2;
         mom_sums(a, s1, s2);
-        if (MODE == 0) return cvt<Out>(s1 / p.divisor);
-        double n = (double)p.n_red;
-        double m2 = s2 - s1 * (s1 / n);
+        if (MODE == 0) return cvt<Out>(div_by(s1, p.divisor, p.rdivisor));
+        double m2 = s2 - s1 * div_by(s1, (double)p.n_red, p.rn_red);
         if (m2 < 0.0) m2 = 0.0;
-        double var = m2 / p.divisor;
+        double var = div_by(m2, p.divisor, p.rdivisor);
         return cvt<Out>(MODE == 2 ? sqrt(var) : var);
     }
 };
@@ -1425,7 +1544,7 @@ template <class Out, class A, int MAXOP> struct Fin<Out, AccArg<A, MAXOP>> {
 // mean divisor in double (mean_division, include/xtensor/core/xmath.hpp:1828-1835).
 template <int POST, class Out, class V, class P> XTG_DI Out post(V v, const P& p) {
     if (POST == 1) return cvt<Out>(m_sqrt(cvt<double>(v)));
-    if (POST == 2) return cvt<Out>(cvt<double>(v) / p.divisor);
+    if (POST == 2) return cvt<Out>(div_by(cvt<double>(v), p.divisor, p.rdivisor));
     return cvt<Out>(v);
 }
 // Value type handed from Fin to post: POST 2 keeps the sum in double.
@@ -1451,9 +1570,12 @@ template <class TS, class TM, class TV, class TN, int POST> struct Store<StatsOu
         pm.initial_f = 0.0;
         pm.initial_i = 0;
         pm.divisor = p.divisor;
+        pm.rdivisor = p.rdivisor;
+        pm.rn_red = p.rn_red;
         pm.n_red = p.n_red;
         FinP pv = pm;  // the variance's divisor
         pv.divisor = p.divisor2;
+        pv.rdivisor = p.rdivisor2;
         if (p.out) reinterpret_cast<TS*>(p.out)[oo] = finish<TS, AccSumC, 0>(a.s, pm);
         if (p.out_more[0]) reinterpret_cast<TM*>(p.out_more[0])[oo] = finish<TM, AccSumC, 2>(a.s, pm);
         if (p.out_more[1]) reinterpret_cast<TV*>(p.out_more[1])[oo] = finish<TV, AccMom<float, 1>, 0>(a.m, pv);
@@ -1580,10 +1702,31 @@ template <class... S, int VEC> struct Ring<LeafSet<S...>, VEC> {
 struct ArrVal {
     template <class RG, class C> static XTG_DI auto ev(const RG& r, int j, const C&) { return r[j]; }
 };
-// ES: 0 reduce only; 1 also store each evaluated vector, contiguous and
-// aligned, into p.eout (type ET); 2 the same with element-wise strided stores.
-// PK: 1 = the packed working accumulator (Work<Acc>) for double-float
-// states, 0 = the stored state's own add.
+// Rows are finished G at a time by a group of G lanes: lane i keeps the state
+// of the group's i-th row since the last finish (group_reduce leaves the
+// total in every lane), and then every lane finishes its own.  The finishers
+// work in FP64, which this part issues at 2 lanes per clock: one lane per row
+// cost float32 sums of 512-element rows as much as their memory traffic, and
+// variances of 64-element rows 40 times that.
+template <class Acc, class Out, int POST, int G> struct LaneFinish {
+    Acc kept;
+    i64 at;             // output offset of the kept state
+    bool have = false;
+    int n = 0;          // rows the group has taken since the last finish
+    template <class P> XTG_DI void take(const Acc& a, bool valid, i64 oo, int gl, const P& p) {
+        if (gl == n) {
+            kept = a;
+            at = oo;
+            have = valid;
+        }
+        if (++n == G) flush(p);
+    }
+    template <class P> XTG_DI void flush(const P& p) {
+        if (have) reinterpret_cast<Out*>(p.out)[at] = finish<Out, Acc, POST>(kept, p);
+        have = false;
+        n = 0;
+    }
+};
 template <class Tree, class LS, class Acc, class Out, int POST, int VEC, int RO, int RR, int GROUP, bool BIG, int UR = 4,
           int ES = 0, class ET = float, int PK = 1>
 __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
@@ -1592,7 +1735,7 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
     __shared__ Acc smem[32];
     Ctx<0> c;
     c.scal = p.scal;
-    const int gsz = GROUP <= 32 ? 32 : (int)blockDim.x;
+    const int gsz = GROUP <= 32 ? GROUP : (int)blockDim.x;
     const int groups_per_block = (int)blockDim.x / gsz;
     const int gtid = (int)threadIdx.x % gsz;
     const i64 gid = (i64)blockIdx.x * groups_per_block + (int)threadIdx.x / gsz;
@@ -1601,6 +1744,7 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
     i64 inner[XTG_KMAX_LEAVES];
 #pragma unroll
     for (int l = 0; l < LS::N; ++l) inner[l] = p.lrs[l][RR - 1];
+    LaneFinish<Acc, Out, POST, (GROUP <= 32 ? GROUP : 1)> fin;
     for (i64 w = gid; w < nwork; w += ngroups) {
         const i64 o = p.nsplit == 1 ? w : w / p.nsplit;
         const i64 s = w - o * p.nsplit;
@@ -1702,17 +1846,39 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
             consume(rgb, r0 + step);                                                   \
         }                                                                              \
     }
+        bool reduced = false;  // acc already holds the group's result
         if constexpr (FastSel<Acc>::value && ES == 0) {
-            // amax / amin: a position-free pass; the exact pass with
-            // positions only when some thread of the group met a NaN, a zero
-            // or (float64) another special value
+            // amax / amin: a position-free pass, arg-reductions: 32-bit
+            // positions; the exact pass only when some thread of the group met
+            // a NaN, a zero or (float64) another special value
             typename FastSel<Acc>::F fa;
             fa.init(p);
+            if (rb + gtid < re) FastStart<typename FastSel<Acc>::F>::at(fa, (u32)((rb + gtid) * VEC));
             XTG_ROW_PASS(fa)
-            bool ex = fa.exact();
-            if (GROUP <= 32) ex = __any_sync(0xffffffffu, ex);
-            else ex = __syncthreads_or(ex) != 0;
-            if (ex) XTG_ROW_PASS(acc)
+            // (a group of a warp that met a NaN: its first lane walks the whole
+            // item in order, since a fold with NaNs depends on the order)
+            bool ex, seq = false;
+            if (GROUP <= 32) {
+                fa = group_reduce<GROUP>(fa, (typename FastSel<Acc>::F*)nullptr);  // the same in every lane
+                ex = fa.exact();
+                seq = fa.nan();
+            } else {
+                ex = __syncthreads_or(fa.exact()) != 0;
+            }
+            reduced = GROUP <= 32 && !ex;
+            if (seq) {
+                if (gtid == 0)
+                    for (i64 r = rb; r < re; ++r) {
+                        i64 ri[RR];
+                        decode_dims<RR, BIG>(p.rshape, p.rfd, r, ri);
+                        ri[RR - 1] *= VEC;
+                        i64 off[XTG_KMAX_LEAVES];
+                        red_offsets<LS::N, RO, RR>(p, ko, ri, off);
+                        LoadLeavesAt<LS>::template run<VEC>(rga[0], p.leaf, off, inner);
+#pragma unroll
+                        for (int j = 0; j < VEC; ++j) acc.add(Tree::ev(rga[0], j, c), r * VEC + j);
+                    }
+            } else if (ex) XTG_ROW_PASS(acc)
             else fa.to(acc);
         } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
             // double-float states: two lanes advanced by packed instructions
@@ -1724,8 +1890,13 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
             XTG_ROW_PASS(acc)
         }
 #undef XTG_ROW_PASS
-        acc = group_reduce<GROUP>(acc, smem);
-        if (gtid == 0) {
+        if (!reduced) acc = group_reduce<GROUP>(acc, smem);
+        if (GROUP <= 32 && p.nsplit == 1) {
+            i64 oo = 0;
+#pragma unroll
+            for (int d = 0; d < RO; ++d) oo += ko[d] * p.ostr[d];
+            fin.take(acc, true, oo, gtid, p);
+        } else if (gtid == 0) {
             if (p.nsplit > 1) {
                 static_assert(sizeof(Acc) <= 32, "split partial slots are 32 bytes");
                 reinterpret_cast<Acc*>(p.partial)[w] = acc;
@@ -1738,6 +1909,7 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
         }
         if (GROUP > 32) __syncthreads();
     }
+    if (GROUP <= 32 && p.nsplit == 1) fin.flush(p);
 }
 
 // K4: COL strategy — the innermost kept dim is contiguous; each thread owns
@@ -3969,6 +4141,247 @@ __global__ void __launch_bounds__(128, MINB) k_rowfused_tma(const RowParams p) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// K3 over units: many short or odd rows.  A warp takes units of 32 / G
+// consecutive rows (G lanes per row).  The leaves in MASK are contiguous from
+// row to row: their units stream into a ring of NS buffers per warp with
+// cp.async.bulk, so rows may start at any element and NS units are in flight
+// without registers; the other leaves (a vector broadcast over the rows, a
+// value per row) are read where they lie.  A copy takes a unit's 16-byte
+// granules whole, its neighbours' bytes in the first and last one included
+// (they are rows of the same array); the first unit's head and the last
+// unit's tail, which have no such neighbour, are loaded by the lanes.
+// The fold of a row is K3's with the same G: lane gl takes vectors gl, gl + G,
+// gl + 2 G, ... in order.  ES, ET, PK as in k_reduce_row.
+template <int I, int VEC, unsigned MASK, class... S> struct UnitLoad;
+template <int I, int VEC, unsigned MASK> struct UnitLoad<I, VEC, MASK> {
+    template <class RG>
+    static XTG_DI void run(RG&, const unsigned char*, const unsigned*, const RedParams&, const i64*, int) {}
+};
+template <int I, int VEC, unsigned MASK, class S0, class... S> struct UnitLoad<I, VEC, MASK, S0, S...> {
+    template <class RG>
+    static XTG_DI void run(RG& rg, const unsigned char* buf, const unsigned* loff, const RedParams& p, const i64* kb, int e) {
+        typedef typename S0::type T;
+        if constexpr ((MASK >> I) & 1u) ld_smem<T, VEC>(rg.v, reinterpret_cast<const T*>(buf + loff[I]) + e);
+        else ld_leaf<T, S0::kind, VEC>(rg.v, reinterpret_cast<const T*>(p.leaf[I]), kb[I] + e * p.lrs[I][0], p.lrs[I][0]);
+        UnitLoad<I + 1, VEC, MASK, S...>::run(rg.rest, buf, loff, p, kb, e);
+    }
+};
+template <class LS> struct UnitLoads;
+template <class... S> struct UnitLoads<LeafSet<S...>> {
+    template <int VEC, unsigned MASK, class RG>
+    static XTG_DI void run(RG& rg, const unsigned char* buf, const unsigned* loff, const RedParams& p, const i64* kb, int e) {
+        UnitLoad<0, VEC, MASK, S...>::run(rg, buf, loff, p, kb, e);
+    }
+};
+// The elements of a unit outside its copied bytes (head of the first unit,
+// tail of the last), by plain loads.
+template <int I, unsigned MASK, class... S> struct UnitEnds;
+template <int I, unsigned MASK> struct UnitEnds<I, MASK> {
+    template <class A> static XTG_DI void run(const A&, const unsigned*, unsigned char*, const unsigned*, bool, bool, int) {}
+};
+template <int I, unsigned MASK, class S0, class... S> struct UnitEnds<I, MASK, S0, S...> {
+    template <class A>
+    static XTG_DI void run(const A& src, const unsigned* bytes, unsigned char* buf, const unsigned* loff, bool head, bool tail, int lane) {
+        if constexpr ((MASK >> I) & 1u) {
+            const int at = RowEdge<I, S0>::place(src[I], bytes[I], lane);
+            if (at >= 0 && (lane < 16 ? head : tail))
+                *reinterpret_cast<typename S0::type*>(buf + loff[I] + (unsigned)((u64)src[I] & 15) + at) =
+                    *reinterpret_cast<const typename S0::type*>(src[I] + at);
+        }
+        UnitEnds<I + 1, MASK, S...>::run(src, bytes, buf, loff, head, tail, lane);
+    }
+};
+template <unsigned MASK, class LS> struct UnitEndsOf;
+template <unsigned MASK, class... S> struct UnitEndsOf<MASK, LeafSet<S...>> {
+    typedef UnitEnds<0, MASK, S...> E;
+};
+
+template <class Tree, class LS, class Acc, class Out, int POST, int VEC, int G, unsigned MASK, int NS, int MINB, int ES = 0,
+          class ET = float, int PK = 1>
+__global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
+    pdl_wait();
+    typedef typename LS::template R<VEC>::type RG;
+    constexpr int UR = 32 / G;  // rows per unit
+    constexpr int kPolls = 1 << 22;
+    extern __shared__ __align__(128) unsigned char dsmem[];
+    __shared__ u64 bars[4 * NS];
+    const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+    const int gl = lane % G;
+    u64* const mybar = bars + NS * warp;
+    unsigned char* const bufs = dsmem + (size_t)(NS * warp) * p.buf_bytes;
+    if (lane == 0) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) mbar_init(&mybar[s], 1);
+        fence_mbar_init();
+    }
+    __syncwarp();
+    Ctx<0> c;
+    c.scal = p.scal;
+    const int nvr = (int)p.n_redv;  // vectors per row
+    const i64 n_units = (p.n_out + UR - 1) / UR;
+    const i64 first = (i64)blockIdx.x * 4 + warp;
+    const i64 ng = (i64)gridDim.x * 4;
+    auto place = [&](i64 unit, const unsigned char* (&src)[XTG_KMAX_LEAVES], unsigned(&bytes)[XTG_KMAX_LEAVES]) {
+        const i64 row = unit * UR;
+        const unsigned rows = (unsigned)(p.n_out - row < UR ? p.n_out - row : UR);
+#pragma unroll
+        for (int l = 0; l < LS::N; ++l)
+            if ((MASK >> l) & 1u) {
+                src[l] = reinterpret_cast<const unsigned char*>(p.leaf[l]) + row * p.lbytes[l];
+                bytes[l] = rows * p.lbytes[l];
+            }
+    };
+    auto issue = [&](i64 unit, int slot) {
+        if (lane != 0) return;
+        const unsigned char* src[XTG_KMAX_LEAVES];
+        unsigned bytes[XTG_KMAX_LEAVES];
+        place(unit, src, bytes);
+        u64 lo[XTG_KMAX_LEAVES], hi[XTG_KMAX_LEAVES];
+        unsigned total = 0;
+#pragma unroll
+        for (int l = 0; l < LS::N; ++l)
+            if ((MASK >> l) & 1u) {
+                const u64 a = (u64)src[l], e = a + bytes[l];
+                lo[l] = unit == 0 ? (a + 15) & ~15ull : a & ~15ull;
+                hi[l] = unit == n_units - 1 ? e & ~15ull : (e + 15) & ~15ull;
+                total += (unsigned)(hi[l] - lo[l]);
+            }
+        mbar_expect_tx(&mybar[slot], total);
+#pragma unroll
+        for (int l = 0; l < LS::N; ++l)
+            if ((MASK >> l) & 1u) {
+                // shared and global addresses agree modulo 16: the unit's granule 0 at loff
+                unsigned char* d = bufs + (size_t)slot * p.buf_bytes + p.loff[l] + (unsigned)(lo[l] - ((u64)src[l] & ~15ull));
+                if (hi[l] > lo[l]) bulk_g2s(d, (const void*)lo[l], (unsigned)(hi[l] - lo[l]), &mybar[slot]);
+            }
+    };
+    LaneFinish<Acc, Out, POST, G> fin;
+#pragma unroll 1
+    for (int s = 0; s < NS; ++s)
+        if (first + s * ng < n_units) issue(first + s * ng, s);
+    int it = 0;
+    for (i64 unit = first; unit < n_units; unit += ng, ++it) {
+        const int slot = it % NS;
+        const unsigned parity = (unsigned)(it / NS) & 1u;
+        unsigned char* const buf = bufs + (size_t)slot * p.buf_bytes;
+        const i64 row = unit * UR + lane / G;
+        const bool live = row < p.n_out;
+        unsigned loff[XTG_KMAX_LEAVES];
+        i64 kb[XTG_KMAX_LEAVES];
+        {
+            const unsigned char* src[XTG_KMAX_LEAVES];
+            unsigned bytes[XTG_KMAX_LEAVES];
+            place(unit, src, bytes);
+            if (unit == 0 || unit == n_units - 1)
+                UnitEndsOf<MASK, LS>::E::run(src, bytes, buf, p.loff, unit == 0, unit == n_units - 1, lane);
+#pragma unroll
+            for (int l = 0; l < LS::N; ++l) {
+                if ((MASK >> l) & 1u) loff[l] = p.loff[l] + (unsigned)((u64)src[l] & 15) + (unsigned)(lane / G) * p.lbytes[l];
+                else kb[l] = row * p.lks[l][0];
+            }
+        }
+        bool done = false;
+        for (int k = 0; k < kPolls; ++k) {
+            if (mbar_try_wait(&mybar[slot], parity)) {
+                done = true;
+                break;
+            }
+        }
+        // one decision for the warp (and the barrier behind the ends' stores)
+        done = __all_sync(0xffffffffu, done) != 0;
+        if (!done) {
+            // give up: flag it, wait (bounded) for the other slots' copies, leave
+            if (lane == 0) {
+                atomicExch(p.err, 1);
+                for (int s = 1; s < NS; ++s) {
+                    const i64 u = unit + s * ng;
+                    if (u < n_units)
+                        for (int k = 0; k < kPolls; ++k)
+                            if (mbar_try_wait(&mybar[(it + s) % NS], (unsigned)((it + s) / NS) & 1u)) break;
+                }
+            }
+            return;
+        }
+        Acc acc;
+        acc.init(p);
+        if (NeedsShift<Acc>::value && live) {
+            typename LS::template R<1>::type rg1;
+            UnitLoads<LS>::template run<1, MASK>(rg1, buf, loff, p, kb, 0);
+            Shift<Acc>::set(acc, Tree::ev(rg1, 0, c));
+        }
+        const int end = live ? nvr : 0;
+// One vector of the row, already loaded, into A.
+#define XTG_UNIT_ADD(A, V, r)                                                          \
+    {                                                                                  \
+        const int e = (r) * VEC;                                                       \
+        if constexpr (ES != 0) {                                                       \
+            ET ev[VEC];                                                                \
+            _Pragma("unroll") for (int j = 0; j < VEC; ++j) ev[j] = cvt<ET>(Tree::ev(V, j, c)); \
+            st_out<ET, ES == 1 ? K_CONTIG : 2, VEC>(reinterpret_cast<ET*>(p.eout),     \
+                                                    row * p.eks[0] + e * p.ers[0], p.ers[0], ev); \
+            AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, ArrVal>(A, ev, (i64)e, c); \
+        } else {                                                                       \
+            AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, Tree>(A, V, (i64)e, c); \
+        }                                                                              \
+    }
+// The pass over the row's vectors S, S + T, S + 2 T, ..., folding into A:
+// batches of four that lie inside the row for every lane, then one by one
+// (a batch under predicates would issue its FP64 work for absent vectors too:
+// float64 sums of 130-element rows 223 us, 128-element rows 142).
+#define XTG_UNIT_PASS(A, S, T)                                                         \
+    {                                                                                  \
+        int r0 = (S);                                                                  \
+        const int whole = end / ((T) * 4) * ((T) * 4);                                 \
+        for (; r0 < whole; r0 += (T) * 4) {                                            \
+            RG rg[4];                                                                  \
+            _Pragma("unroll") for (int u = 0; u < 4; ++u)                              \
+                UnitLoads<LS>::template run<VEC, MASK>(rg[u], buf, loff, p, kb, (r0 + u * (T)) * VEC); \
+            _Pragma("unroll") for (int u = 0; u < 4; ++u) XTG_UNIT_ADD(A, rg[u], r0 + u * (T)) \
+        }                                                                              \
+        _Pragma("unroll 1") for (; r0 < end; r0 += (T)) {                              \
+            RG rg;                                                                     \
+            UnitLoads<LS>::template run<VEC, MASK>(rg, buf, loff, p, kb, r0 * VEC);    \
+            XTG_UNIT_ADD(A, rg, r0)                                                    \
+        }                                                                              \
+    }
+        bool reduced = false;  // acc already holds the group's result
+        if constexpr (FastSel<Acc>::value && ES == 0) {
+            typename FastSel<Acc>::F fa;
+            fa.init(p);
+            if (gl < end) FastStart<typename FastSel<Acc>::F>::at(fa, (u32)(gl * VEC));
+            XTG_UNIT_PASS(fa, gl, G)
+            fa = group_reduce<G>(fa, (typename FastSel<Acc>::F*)nullptr);  // the same in every lane
+            reduced = !fa.exact();
+            if (reduced) {
+                fa.to(acc);
+            } else if (!fa.nan()) {
+                XTG_UNIT_PASS(acc, gl, G)
+            } else if (gl == 0) {
+                // a row with a NaN: the group's first lane walks it in order
+                // (a fold with NaNs depends on the order)
+                XTG_UNIT_PASS(acc, 0, 1)
+            }
+        } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
+            typename Work<Acc>::T wa;
+            wa.from(acc);
+            XTG_UNIT_PASS(wa, gl, G)
+            wa.to(acc);
+        } else {
+            XTG_UNIT_PASS(acc, gl, G)
+        }
+#undef XTG_UNIT_PASS
+#undef XTG_UNIT_ADD
+        // every lane has read the unit: refill its slot
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (unit + NS * ng < n_units) issue(unit + NS * ng, slot);
+        if (!reduced) acc = group_reduce<G>(acc, (Acc*)nullptr);
+        fin.take(acc, live, row * p.ostr[0], gl, p);
+    }
+    fin.flush(p);
+}
+
 // a * (1 / b) with b invariant over a row: the reciprocal is computed once
 // per row (Prep) into statistic slot KR (a division costs ~10 FP64
 // operations on GB300, and an IEEE FP32 division several instructions).
@@ -4133,6 +4546,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch_rowreduce(const BatchParams
         const BatchInst* I = p.inst + tl.inst;
         const i64 cols = I->cols;
         fp.divisor = I->divisor;
+        fp.rdivisor = I->rdivisor;
         fp.n_red = cols;
         i64 cs[XTG_KMAX_LEAVES], rsv[XTG_KMAX_LEAVES];
 #pragma unroll

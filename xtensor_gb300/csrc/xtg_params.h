@@ -107,6 +107,8 @@ struct RedParams {
     double initial_f;
     i64 initial_i;
     double divisor;  // mean / variance divisor (already integer-divided like the reference)
+    double rdivisor; // 1 / divisor
+    double rn_red;   // 1 / n_red
     // fused assign + reduce (row kernel with ES != 0): every evaluated
     // element, converted to the destination type, is also stored at
     // eout + sum(kept index * eks) + sum(reduced index * ers)
@@ -119,6 +121,11 @@ struct RedParams {
     // variance divisor (the mean's is `divisor`)
     void* out_more[3];
     double divisor2;
+    double rdivisor2;  // 1 / divisor2
+    // rows in units: per-warp buffer layout in shared memory (streamed leaves)
+    unsigned loff[XTG_KMAX_LEAVES];    // byte offset of each leaf's unit in a buffer
+    unsigned lbytes[XTG_KMAX_LEAVES];  // bytes of one row
+    unsigned buf_bytes;                // bytes of one buffer
 };
 
 struct RowParams {
@@ -209,6 +216,7 @@ struct BatchInst {
     i64 ors, ocs;             // destination strides (reductions use ors only)
     i64 rows, cols;
     double divisor;           // mean divisor of a row
+    double rdivisor;          // 1 / divisor
 };
 struct BatchTile {
     int inst;
@@ -235,6 +243,8 @@ struct FinP {
     double initial_f;
     i64 initial_i;
     double divisor;
+    double rdivisor;
+    double rn_red;
     i64 n_red;
 };
 

@@ -234,7 +234,6 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     const int64_t kept_in_stride = prim >= 0 ? K.st[1 + prim][RO - 1] : 1;
     bool row = true;
     if (n_out > 1 && kept_in_stride == 1 && red_in_stride != 1) row = false;
-    if (n_out >= 1024 && red_in_stride == 1 && Rd.shape[RR - 1] < 32 && kept_in_stride != 1 && RR == 1) row = false;
     if (opt("reduce.force_row", 0)) row = true;
     if (eout && !row) {
         if (not_fusable) *not_fusable = true;
@@ -289,6 +288,9 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
 
     p.n_out = n_out;
     p.n_red = n_red;
+    p.rdivisor = 1.0 / p.divisor;
+    p.rdivisor2 = 1.0 / p.divisor2;
+    p.rn_red = 1.0 / (double)n_red;
     for (int d = 0; d < RO; ++d) p.oshape[d] = K.shape[d];
     for (int d = 0; d < RR; ++d) p.rshape[d] = Rd.shape[d];
     if (row) p.rshape[RR - 1] /= vec;
@@ -383,7 +385,61 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         st = get_kernel(name, 288, &k, smem);  // 8 consumer warps + the producer warp
         if (st == XTG_OK) st = launch(k, grid_cap(k, nsplit), 288, &p, stream, smem, part_off);
     } else if (row) {
-        const int group = (chunk >= opt("reduce.cta_chunk", 2048)) ? 256 : 32;
+        int group = (chunk >= opt("reduce.cta_chunk", 2048)) ? 256 : 32;
+        // Lanes per row of whole rows: about 256 bytes of the row per lane
+        // (the unit of a warp is then about 8 KiB), so that short rows share a
+        // warp's merges and a long row's are few (2^26 float32: rows of 64, 335
+        // us with a warp per row, 46 with a lane pair; rows of 512, 54 and 42
+        // with 8 lanes); vectors of rows over 128 bytes take two lanes at
+        // least (rows of 64 with one: 68 us, the lanes' vectors fall on the
+        // same banks).  Fewer than 4096 warps' worth of rows spread over more
+        // lanes.
+        if (group == 32 && nsplit == 1 && RR == 1 && p.n_redv > 0) {
+            int g = 1;
+            while (g < 32 && n_red * maxsz > (int64_t)g * (vec > 1 && g == 1 ? 128 : 256)) g *= 2;
+            while (g < 32 && n_out * g < 4096 * 32 && g < p.n_redv) g *= 2;
+            group = g;
+            // single-element stores of 16 or 32 rows at once touch as many
+            // sectors: the fused form of short odd rows loses to two calls
+            // (10^6 x 27 float32: 143 us fused, 93 in two)
+            if (eout && vec == 1 && g < 4) {
+                if (not_fusable) *not_fusable = true;
+                return fail(XTG_ERR_UNSUPPORTED, kNotFusable);
+            }
+        }
+        // K3 over units: leaves contiguous from row to row are streamed, two
+        // units in flight per warp (three: slower everywhere, fewer warps
+        // fit); up to 12 KiB per unit, which leaves 8 warps per SM.  Odd rows
+        // gain most (2^26 float32 in rows of 511: 65 us by single loads, 43
+        // streamed; 2047: 62 / 39), whole vectors a little (argmax float32 of
+        // 1024 is even at 48 / 51).
+        unsigned mask = 0;
+        int64_t unit_bytes = 0;
+        if (group <= 32 && nsplit == 1 && RO == 1 && RR == 1 && n_out >= 4096 && !big && n_red > 0 && opt("reduce.units", 1)) {
+            for (int l = 0; l < NL; ++l) {
+                const int sz = dt(t.leaves[l].dtype).size;
+                if (kinds[l] != 0 || K.st[1 + l][0] != n_red || n_red * sz < 16 || !aligned(t.leaves[l].data, sz)) continue;
+                mask |= 1u << l;
+                p.loff[l] = (unsigned)unit_bytes;
+                p.lbytes[l] = (unsigned)(n_red * sz);
+                unit_bytes += (32 / group * n_red * sz + 31) / 16 * 16;
+            }
+            if (unit_bytes > 12288) mask = 0;
+        }
+        if (mask) {
+            const size_t smem = (size_t)unit_bytes * 2 * 4;
+            p.buf_bytes = (unsigned)unit_bytes;
+            XTG_TRY(device_error_word(&p.err));
+            const std::string name = "xtg::k_reduce_unit<" + tree + ", " + ls + ", " + accname + ", " + outc + ", " +
+                                     std::to_string(post) + ", " + std::to_string(vec) + ", " + std::to_string(group) +
+                                     ", " + std::to_string(mask) + ", 2, 4" +
+                                     (es ? ", " + std::to_string(es) + ", " + dt(eout->dtype).cname : std::string()) +
+                                     (opt("reduce.packed", 1) ? std::string() : std::string(es ? "" : ", 0, float") + ", 0") +
+                                     ">";
+            XTG_TRY(get_kernel(name, 128, &k, smem));
+            const int64_t units = (n_out * group + 31) / 32;
+            return launch(k, grid_cap(k, (units + 3) / 4), 128, &p, stream, smem);
+        }
         // (a copy ring as in the column kernel measured slower here: these
         // loops are instruction-bound once two register batches are in flight)
         std::string name = "xtg::k_reduce_row<" + tree + ", " + ls + ", " + accname + ", " + outc + ", " +
