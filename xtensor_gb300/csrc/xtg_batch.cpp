@@ -48,8 +48,12 @@ struct xtg_batch {
     cudaEvent_t last = nullptr;     // recorded after every upload and launch: destroy waits on it,
                                     // never on the stream (which may be gone by then)
     // configuration
-    int gl = 32, unroll = 4, cpsm = 4;
+    int gl = 32, unroll = 4, cpsm = 4;  // gl 0: the streamed form
     int vec = 1;  // reductions: elements per vector load (1: the strided form)
+    unsigned mask = 0;     // reductions: leaves that the streamed form could copy in units (0: not streamable)
+    int64_t max_cols = 0;  // widest instance
+    int block = 256;
+    size_t smem = 0;
     int64_t tile_elems = 32768;
     int tuned = 0;
     std::string kname;  // kernel name for the current group width
@@ -64,6 +68,8 @@ struct xtg_batch {
 namespace {
 
 std::mutex g_tune_mu;
+
+constexpr int kUnitSlots = 3;  // ring slots of the streamed form
 
 std::string tune_dir() {
     const char* d = getenv("XTG_CACHE_DIR");
@@ -126,12 +132,16 @@ xtg_status make_tiles(xtg_batch* b, int64_t te, std::vector<xtg::BatchTile>& til
         if (I.rows == 0 || I.cols == 0) continue;
         int64_t rpt = std::max<int64_t>(1, te / std::max<int64_t>(I.cols, 1));
         rpt = std::min<int64_t>(rpt, 1 << 20);
-        for (int64_t r = 0; r < I.rows; r += rpt) {
+        for (int64_t r = 0; r < I.rows;) {
             xtg::BatchTile t;
             t.inst = (int)i;
             t.row0 = r;
             t.nrows = (int)std::min<int64_t>(rpt, I.rows - r);
+            // streamed units: a copy may take the granule behind a tile, so
+            // what follows a tile has 16 elements at least, or joins it
+            if (b->gl == 0 && (I.rows - r - t.nrows) * I.cols < 16) t.nrows = (int)(I.rows - r);
             tiles.push_back(t);
+            r += t.nrows;
         }
     }
     return XTG_OK;
@@ -164,6 +174,9 @@ std::string kernel_name(xtg_batch* b, const Tree& t, int gl, const AccChoice* ch
     }
     ls += ">";
     const std::string tree = tree_type(t, t.root, map);
+    if (gl == 0)
+        return "xtg::k_batch_rowunits<" + tree + ", " + ls + ", " + ch->acc + ", " + dt(b->out_dtype).cname + ", " +
+               std::to_string(ch->post) + ", " + std::to_string(b->mask) + ", " + std::to_string(kUnitSlots) + ">";
     if (b->reduce)
         return "xtg::k_batch_rowreduce<" + tree + ", " + ls + ", " + ch->acc + ", " + dt(b->out_dtype).cname + ", " +
                std::to_string(ch->post) + ", " + std::to_string(gl) + ", " +
@@ -183,12 +196,29 @@ xtg_status mark(xtg_batch* b, cudaStream_t s) {
 xtg_status launch_once(xtg_batch* b, cudaStream_t s) {
     DeviceInfo* dev;
     XTG_TRY(ensure_device(&dev));
-    if (!dry_run()) XTG_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(int), s));
+    if (!dry_run() && b->gl != 0) XTG_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(int), s));
     b->stream = s;
-    int64_t cap = (int64_t)std::min(b->k->max_blocks_per_sm, b->cpsm) * dev->sm_count;
+    int64_t cap = (int64_t)std::min(b->k->max_blocks_per_sm, b->gl ? b->cpsm : 32) * dev->sm_count;
     unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(b->ntiles, cap));
-    XTG_TRY(launch(b->k, grid, 256, &b->params, s));
+    XTG_TRY(launch(b->k, grid, b->block, &b->params, s, b->smem));
     return mark(b, s);
+}
+
+// Launch shape: 256 threads, or (the streamed form) five warps and a ring of
+// slots for units of `te` elements (at least a row).
+void set_shape(xtg_batch* b, const Tree& t, int64_t te) {
+    b->block = 256;
+    b->smem = 0;
+    if (b->gl != 0) return;
+    unsigned bytes = 0;
+    for (size_t l = 0; l < t.leaves.size(); ++l)
+        if ((b->mask >> l) & 1u) {
+            b->params.loff[l] = bytes;
+            bytes += (unsigned)(((std::max(te, b->max_cols) + 16) * dt(t.leaves[l].dtype).size + 31) / 16 * 16);
+        }
+    b->params.buf_bytes = bytes;
+    b->block = 160;
+    b->smem = (size_t)bytes * kUnitSlots;
 }
 
 // The parts of a build that decide the kernel: the tree, the accumulator,
@@ -213,6 +243,30 @@ xtg_status plan_kernel(xtg_batch* b, Tree& t, AccChoice& ch, int& gl_default, st
             for (size_t l = 0; ok && l < t.leaves.size(); ++l) ok = I.cs[l] == 0 || I.cs[l] == 1;
         if (ok) b->vec = 16 / esz;
     }
+    // streamed units: the leaves that are contiguous from row to row in every
+    // instance, rows short enough for two slots of a ring
+    b->mask = 0;
+    b->max_cols = 0;
+    for (auto& I : b->inst) b->max_cols = std::max<int64_t>(b->max_cols, I.cols);
+    if (b->reduce && opt("batch.units", 1)) {
+        int64_t row_bytes = 0;
+        for (size_t l = 0; l < t.leaves.size(); ++l) {
+            const int64_t sz = dt(t.leaves[l].dtype).size;
+            bool ok = true;
+            for (auto& I : b->inst)
+                ok = ok && I.cs[l] == (I.cols == 1 ? I.cs[l] : 1) && (I.rows == 1 || I.rs[l] == I.cols) &&
+                     (uintptr_t)I.leaf[l] % sz == 0;
+            if (ok) {
+                b->mask |= 1u << l;
+                row_bytes += b->max_cols * sz;
+            }
+        }
+        if (row_bytes > 40 * 1024) b->mask = 0;
+        // (the kernel keeps the other leaves' column strides as 32-bit byte counts)
+        for (auto& I : b->inst)
+            for (size_t l = 0; l < t.leaves.size(); ++l)
+                if (I.cs[l] > (1 << 27) || I.cs[l] < -(1 << 27)) b->mask = 0;
+    }
     cols.clear();
     rows.clear();
     for (auto& I : b->inst) {
@@ -222,6 +276,11 @@ xtg_status plan_kernel(xtg_batch* b, Tree& t, AccChoice& ch, int& gl_default, st
     std::sort(cols.begin(), cols.end());
     std::sort(rows.begin(), rows.end());
     gl_default = (int)opt("batch.group_lanes", -1);
+    // the streamed form up to 2^25 elements (it runs at 0.45 of the copy rate
+    // but starts at once: 59 instances of up to 312 x 91 float32 91 us before,
+    // 4 streamed; 256 of up to 1024 x 512 209 and 83), the warp-tile form
+    // above (256 of up to 4096 x 2048: 727 us, 1460 streamed)
+    if (gl_default < 0 && b->mask && b->elements <= (1ll << 25)) gl_default = 0;
     if (gl_default < 0) gl_default = cols[cols.size() / 2] >= 512 ? 32 : (cols[cols.size() / 2] >= 128 ? 16 : 8);
     return XTG_OK;
 }
@@ -346,6 +405,7 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
         b->stream = s;
     }
     memset(&b->params, 0, sizeof b->params);
+    XTG_TRY(device_error_word(&b->params.err));
     b->params.inst = b->d_inst;
     b->params.counter = b->d_counter;
     for (size_t i = 0; i < t.scalars.size(); ++i) b->params.scal.v[i] = t.scalars[i];
@@ -357,21 +417,25 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
         b->params.initial_i = ch.initial_i;
     }
     // shape class for the tuning cache
-    const std::string base = kernel_name(b, t, 0, b->reduce ? &ch : nullptr);
+    const std::string base = kernel_name(b, t, 1, b->reduce ? &ch : nullptr);
     char cls[160];
-    snprintf(cls, sizeof cls, "|n%d|c%d|r%d|e%d|sm%d", ilog2((int64_t)b->inst.size()), ilog2(cols[cols.size() / 2]),
+    snprintf(cls, sizeof cls, "|t2|n%d|c%d|r%d|e%d|sm%d", ilog2((int64_t)b->inst.size()), ilog2(cols[cols.size() / 2]),
              ilog2(rows[rows.size() / 2]), ilog2(b->elements), dev->sm_count);
     std::string key;
     for (char c : base + cls)
         if (c != ' ') key += c;
 
     int gl = gl_default, cpsm = (int)opt("batch.ctas_per_sm", 4);
-    int64_t te = opt("batch.tile_elems", 32768);
+    // Tiles of about te elements, small enough that a small batch spreads over
+    // 16 warps per SM (a warp walks its tile row by row)
+    const int64_t te_cap = std::max<int64_t>(256, b->elements / ((int64_t)dev->sm_count * 16));
+    int64_t te = opt("batch.tile_elems", std::min<int64_t>(gl ? 32768 : 4096, te_cap));
+    if (gl == 0) te = std::min<int64_t>(te, 8192);
     b->tuned = 0;
     if (autotune && !dry_run()) {
         int tg, tc;
         int64_t tt;
-        if (tune_lookup(key, tg, tt, tc)) {
+        if (tune_lookup(key, tg, tt, tc) && (tg != 0 || b->mask)) {
             gl = tg;
             te = tt;
             cpsm = tc;
@@ -384,7 +448,9 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
             // fixed order by more than 1% to replace it, so that near-ties
             // resolve the same way on every run.
             const int gls[3] = {8, 16, 32};
-            const int64_t tes[3] = {8192, 32768, 131072};
+            std::vector<int64_t> tes;  // the three largest tile sizes that suit the batch
+            for (int64_t c : {131072, 32768, 8192, 2048, 512})
+                if (tes.size() < 3 && (c <= 2 * te_cap || c == 512)) tes.push_back(c);
             const int cps[3] = {2, 4, 8};
             struct Cand {
                 int g;
@@ -398,10 +464,12 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
             XTG_CUDA(cudaEventCreate(&e0));
             XTG_CUDA(cudaEventCreate(&e1));
             auto time_cand = [&](const Cand& cd, int reps, double* med) -> xtg_status {
+                b->gl = cd.g;
                 XTG_TRY(upload_tiles(b, cd.t, s));
                 b->params.tiles = b->d_tiles;
                 b->params.ntiles = b->ntiles;
-                XTG_TRY(get_kernel(kernel_name(b, t, cd.g, b->reduce ? &ch : nullptr), 256, &b->k));
+                set_shape(b, t, cd.t);
+                XTG_TRY(get_kernel(kernel_name(b, t, cd.g, b->reduce ? &ch : nullptr), b->block, &b->k, b->smem));
                 b->cpsm = cd.c;
                 XTG_TRY(launch_once(b, s));  // warm-up
                 std::vector<float> ms((size_t)reps);
@@ -416,14 +484,18 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
                 *med = ms[(size_t)reps / 2];
                 return XTG_OK;
             };
+            auto try_cand = [&](int g, int64_t tc, int c) -> xtg_status {
+                Cand cd{g, tc, c, 0.0};
+                XTG_TRY(time_cand(cd, 5, &cd.ms));
+                cands.push_back(cd);
+                best = std::min(best, cd.ms);
+                return XTG_OK;
+            };
+            if (b->mask)
+                for (int64_t tcand : {512, 1024, 2048, 4096}) XTG_TRY(try_cand(0, tcand, 4));
             for (int64_t tcand : tes)
                 for (int gcand : gls)
-                    for (int ccand : cps) {
-                        Cand cd{gcand, tcand, ccand, 0.0};
-                        XTG_TRY(time_cand(cd, 5, &cd.ms));
-                        cands.push_back(cd);
-                        best = std::min(best, cd.ms);
-                    }
+                    for (int ccand : cps) XTG_TRY(try_cand(gcand, tcand, ccand));
             const double cut = best * 1.03;
             int pick = -1;
             for (size_t i = 0; i < cands.size(); ++i) {
@@ -453,8 +525,9 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
     }
     b->params.tiles = b->d_tiles;
     b->params.ntiles = b->ntiles;
+    set_shape(b, t, te);
     b->kname = kernel_name(b, t, gl, b->reduce ? &ch : nullptr);
-    XTG_TRY(get_kernel(b->kname, 256, &b->k));
+    XTG_TRY(get_kernel(b->kname, b->block, &b->k, b->smem));
     b->built = true;
     XTG_TRY(mark(b, s));  // the uploads are ordered before the event destroy waits on
     return XTG_OK;

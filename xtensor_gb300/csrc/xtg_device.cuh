@@ -3925,12 +3925,14 @@ template <int I> struct RowEdge<I> {
 };
 template <int I, class S0, class... S> struct RowEdge<I, S0, S...> {
     typedef typename S0::type T;
-    // this lane's element as a byte offset into the unit, or -1
+    // this lane's element as a byte offset into the unit, or negative (a unit
+    // inside one granule has all its elements in the head, and again in the
+    // part of the tail that lies in the unit)
     static XTG_DI int place(const unsigned char* a, unsigned bytes, int lane) {
         const unsigned ph = (unsigned)((u64)a & 15);
         const unsigned head = (16 - ph) & 15, tail = (ph + bytes) & 15;
         const unsigned k = (unsigned)(lane & 15) * (unsigned)sizeof(T);
-        if (lane < 16) return k < head ? (int)k : -1;
+        if (lane < 16) return k < head && k < bytes ? (int)k : -1;
         return k < tail ? (int)(bytes - tail + k) : -1;
     }
     template <class A> static XTG_DI void load(u64* ev, const A& src, const unsigned* bytes, int lane) {
@@ -4597,6 +4599,266 @@ __global__ void __launch_bounds__(256, MINB) k_batch_rowreduce(const BatchParams
             }
             if (active && gl == 0) reinterpret_cast<Out*>(I->out)[row * I->ors] = finish<Out, Acc, POST>(acc, fp);
         }
+    }
+}
+
+// K8 over streamed units, for batches whose instances are contiguous from row
+// to row: a tile is one unit (at most the slot's bytes of every leaf in MASK),
+// a block takes a run of consecutive tiles (units of about equal size: no
+// counter, and an instance's vector stays in the SM's L1: 256 of up to 1024 x 512 float32 112 us with tiles dealt out in turn, 98 in runs).  A producer warp copies the units into a ring of NS slots with
+// cp.async.bulk, granules whole and ends by plain loads as in k_reduce_unit, so
+// rows start at any element; the 128 consumers reduce a unit's rows, g lanes
+// per row (4 .. 128, chosen per tile so that a lane folds at most 32 elements
+// and no warp idles), and finish g rows at a time.  The other leaves (the
+// vector of an instance) are read where they lie.  Waits are bounded as in
+// k_reduce_stream.
+template <int I, unsigned MASK, class... S> struct BatchUnit;
+template <int I, unsigned MASK> struct BatchUnit<I, MASK> {
+    template <class A> static XTG_DI void edges(u64*, const A&, const unsigned*, bool, bool, int) {}
+    template <class A> static XTG_DI void put_edges(const u64*, const A&, const unsigned*, unsigned char*, const unsigned*, bool, bool, int) {}
+    static XTG_DI void place(const BatchInst*, i64, int, const unsigned char**, unsigned*) {}
+    static constexpr XTG_DI int size(int) { return 0; }
+    template <class RG> static XTG_DI void load(RG&, const unsigned char*, const unsigned*, const unsigned char* const*, const int*, int) {}
+    static XTG_DI void row(const BatchInst*, i64, int, const unsigned*, unsigned*, const unsigned char**) {}
+};
+template <int I, unsigned MASK, class S0, class... S> struct BatchUnit<I, MASK, S0, S...> {
+    typedef typename S0::type T;
+    typedef BatchUnit<I + 1, MASK, S...> Next;
+    enum { streamed = (MASK >> I) & 1u };
+    static constexpr XTG_DI int size(int l) { return l == I ? (int)sizeof(T) : Next::size(l); }
+    // first byte and bytes of a unit of each streamed leaf
+    static XTG_DI void place(const BatchInst* B, i64 row0, int nrows, const unsigned char** src, unsigned* bytes) {
+        if constexpr (streamed) {
+            src[I] = reinterpret_cast<const unsigned char*>(B->leaf[I]) + row0 * B->cols * (i64)sizeof(T);
+            bytes[I] = (unsigned)(nrows * (int)B->cols * (int)sizeof(T));
+        }
+        Next::place(B, row0, nrows, src, bytes);
+    }
+    // the elements at an instance's ends that no whole granule holds: into registers, then beside the copy
+    template <class A> static XTG_DI void edges(u64* ev, const A& src, const unsigned* bytes, bool head, bool tail, int lane) {
+        if constexpr (streamed) {
+            const int at = RowEdge<I, S0>::place(src[I], bytes[I], lane);
+            if (at >= 0 && (lane < 16 ? head : tail)) {
+                union { T t; u64 u; } x;
+                x.u = 0;
+                x.t = *reinterpret_cast<const T*>(src[I] + at);
+                ev[I] = x.u;
+            }
+        }
+        Next::edges(ev, src, bytes, head, tail, lane);
+    }
+    template <class A>
+    static XTG_DI void put_edges(const u64* ev, const A& src, const unsigned* bytes, unsigned char* buf, const unsigned* loff, bool head,
+                                 bool tail, int lane) {
+        if constexpr (streamed) {
+            const int at = RowEdge<I, S0>::place(src[I], bytes[I], lane);
+            if (at >= 0 && (lane < 16 ? head : tail)) {
+                union { T t; u64 u; } x;
+                x.u = ev[I];
+                *reinterpret_cast<T*>(buf + loff[I] + (unsigned)((u64)src[I] & 15) + at) = x.t;
+            }
+        }
+        Next::put_edges(ev, src, bytes, buf, loff, head, tail, lane);
+    }
+    // where row r of the unit starts: its offset in the slot, or its address
+    static XTG_DI void row(const BatchInst* B, i64 row0, int r, const unsigned* loff, unsigned* off, const unsigned char** at) {
+        if constexpr (streamed) {
+            const unsigned a = (unsigned)(u64)B->leaf[I] + (unsigned)row0 * (unsigned)B->cols * (unsigned)sizeof(T);
+            off[I] = loff[I] + (a & 15) + r * (int)B->cols * (int)sizeof(T);
+        } else {
+            at[I] = reinterpret_cast<const unsigned char*>(B->leaf[I]) + (row0 + r) * B->rs[I] * (i64)sizeof(T);
+        }
+        Next::row(B, row0, r, loff, off, at);
+    }
+    // (column strides of the other leaves as ints, in bytes; slots by offset,
+    // so that the compiler sees shared memory)
+    template <class RG>
+    static XTG_DI void load(RG& rg, const unsigned char* buf, const unsigned* off, const unsigned char* const* at, const int* cs, int e) {
+        if constexpr (streamed) rg.v[0] = reinterpret_cast<const T*>(buf + off[I])[e];
+        else rg.v[0] = ld1<T>(reinterpret_cast<const T*>(at[I] + (i64)e * cs[I]));
+        Next::load(rg.rest, buf, off, at, cs, e);
+    }
+};
+template <unsigned MASK, class LS> struct BatchUnitOf;
+template <unsigned MASK, class... S> struct BatchUnitOf<MASK, LeafSet<S...>> {
+    typedef BatchUnit<0, MASK, S...> U;
+};
+
+template <class Tree, class LS, class Acc, class Out, int POST, unsigned MASK, int NS>
+__global__ void __launch_bounds__(160) k_batch_rowunits(const BatchParams p) {
+    pdl_wait();
+    typedef typename LS::template R<1>::type RG;
+    typedef typename BatchUnitOf<MASK, LS>::U BU;
+    constexpr int kPolls = 1 << 22;
+    extern __shared__ __align__(128) unsigned char dsmem[];
+    __shared__ u64 full[NS], empty[NS];
+    __shared__ BatchTile meta[NS];
+    __shared__ Acc part[4];
+    const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 4);
+        }
+        fence_mbar_init();
+    }
+    __syncthreads();
+    const i64 share = (p.ntiles + gridDim.x - 1) / gridDim.x;
+    const i64 t0 = (i64)blockIdx.x * share;
+    const i64 t1 = t0 + share < p.ntiles ? t0 + share : p.ntiles;
+    if (warp == 4) {
+        // the producer warp
+        i64 q = 0;
+        bool stop = false;
+        for (i64 t = t0; t < t1; ++t, ++q) {
+            const BatchTile tl = p.tiles[t];
+            const BatchInst* B = p.inst + tl.inst;
+            const unsigned char* src[XTG_KMAX_LEAVES];
+            unsigned bytes[XTG_KMAX_LEAVES];
+            u64 ev[XTG_KMAX_LEAVES];
+            BU::place(B, tl.row0, tl.nrows, src, bytes);
+            const bool head = tl.row0 == 0, tail = tl.row0 + tl.nrows == B->rows;
+            if (head || tail) BU::edges(ev, src, bytes, head, tail, lane);
+            const int slot = (int)(q % NS);
+            if (q >= NS) {
+                const unsigned par = (unsigned)(((q / NS) - 1) & 1);
+                bool ok = false;
+                for (int k = 0; k < kPolls; ++k)
+                    if (mbar_try_wait(&empty[slot], par)) {
+                        ok = true;
+                        break;
+                    }
+                if (!__all_sync(0xffffffffu, ok)) {
+                    stop = true;
+                    break;
+                }
+                fence_proxy_async_smem();  // the consumers' reads before the copy's writes
+            }
+            unsigned char* const buf = dsmem + (size_t)slot * p.buf_bytes;
+            if (head || tail) BU::put_edges(ev, src, bytes, buf, p.loff, head, tail, lane);
+            __syncwarp();
+            if (lane == 0) {
+                meta[slot] = tl;
+                u64 lo[XTG_KMAX_LEAVES], hi[XTG_KMAX_LEAVES];
+                unsigned total = 0;
+#pragma unroll
+                for (int l = 0; l < LS::N; ++l)
+                    if ((MASK >> l) & 1u) {
+                        const u64 a = (u64)src[l], e = a + bytes[l];
+                        lo[l] = head ? (a + 15) & ~15ull : a & ~15ull;
+                        hi[l] = tail ? e & ~15ull : (e + 15) & ~15ull;
+                        if (hi[l] < lo[l]) hi[l] = lo[l];  // a whole instance inside one granule: all of it is its head
+                        total += (unsigned)(hi[l] - lo[l]);
+                    }
+                mbar_expect_tx(&full[slot], total);
+#pragma unroll
+                for (int l = 0; l < LS::N; ++l)
+                    if (((MASK >> l) & 1u) && hi[l] > lo[l])
+                        bulk_g2s(buf + p.loff[l] + (unsigned)(lo[l] - ((u64)src[l] & ~15ull)), (const void*)lo[l],
+                                 (unsigned)(hi[l] - lo[l]), &full[slot]);
+            }
+        }
+        // the copies that may still be in flight: the last issued unit of each slot
+        bool drained = true;
+        for (i64 r = q > NS ? q - NS : 0; r < q; ++r) {
+            bool ok = false;
+            for (int k = 0; k < kPolls; ++k)
+                if (mbar_try_wait(&full[r % NS], (unsigned)((r / NS) & 1))) {
+                    ok = true;
+                    break;
+                }
+            drained = drained && ok;
+        }
+        if ((stop || !drained) && lane == 0) atomicExch(p.err, 1);
+        return;
+    }
+    Ctx<0> c;
+    c.scal = p.scal;
+    FinP fp;
+    fp.init_f = p.init_f;
+    fp.init_i = p.init_i;
+    fp.has_initial = p.has_initial;
+    fp.initial_f = p.initial_f;
+    fp.initial_i = p.initial_i;
+    i64 q = 0;
+    for (i64 t = t0; t < t1; ++t, ++q) {
+        const int slot = (int)(q % NS);
+        const unsigned par = (unsigned)((q / NS) & 1);
+        bool ok = false;
+        for (int k = 0; k < kPolls; ++k)
+            if (mbar_try_wait(&full[slot], par)) {
+                ok = true;
+                break;
+            }
+        if (bar_or_n<128>(!ok)) {
+            if (tid == 0) atomicExch(p.err, 1);
+            return;
+        }
+        const unsigned char* const buf = dsmem + (size_t)slot * p.buf_bytes;
+        const BatchTile tl = meta[slot];
+        const BatchInst* B = p.inst + tl.inst;
+        const int cols = (int)B->cols;
+        fp.divisor = B->divisor;
+        fp.rdivisor = B->rdivisor;
+        fp.n_red = cols;
+        int cs[XTG_KMAX_LEAVES];
+#pragma unroll
+        for (int l = 0; l < LS::N; ++l) cs[l] = (int)B->cs[l] * BU::size(l);
+        int g = 4;
+        while (g < 128 && (cols > g * 32 || tl.nrows * g < 128)) g *= 2;
+        const int gl = tid & (g - 1), rows = 128 / g;
+        Out* const out = reinterpret_cast<Out*>(B->out);
+        const i64 ors = B->ors;
+        Acc kept;
+        int kept_row = -1, n = 0;
+        for (int r0 = 0; r0 < tl.nrows; r0 += rows) {
+            const int r = r0 + tid / g;
+            const int end = r < tl.nrows ? cols : 0;
+            unsigned off[XTG_KMAX_LEAVES];
+            const unsigned char* at[XTG_KMAX_LEAVES];
+            BU::row(B, tl.row0, r, p.loff, off, at);
+            Acc acc;
+            acc.init(fp);
+            int e = gl;
+            for (; e + 3 * g < end; e += 4 * g) {
+                RG rg[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) BU::load(rg[u], buf, off, at, cs, e + u * g);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc.add(Tree::ev(rg[u], 0, c), (i64)(e + u * g));
+            }
+#pragma unroll 1
+            for (; e < end; e += g) {
+                RG rg;
+                BU::load(rg, buf, off, at, cs, e);
+                acc.add(Tree::ev(rg, 0, c), (i64)e);
+            }
+            for (int m = (g < 32 ? g : 32) / 2; m >= 1; m >>= 1) {
+                const Acc o = shfl_xor_pod(acc, m);
+                acc.merge(o);
+            }
+            if (g > 32) {
+                // the warps of the row, in order
+                bar_sync_n<128>();
+                if (lane == 0) part[warp] = acc;
+                bar_sync_n<128>();
+                const int w0 = warp & ~(g / 32 - 1);
+                acc = part[w0];
+                for (int w = 1; w < g / 32; ++w) acc.merge(part[w0 + w]);
+            }
+            if (gl == n) {
+                kept = acc;
+                kept_row = r < tl.nrows ? r : -1;
+            }
+            if (++n == g || r0 + rows >= tl.nrows) {
+                if (kept_row >= 0) out[(tl.row0 + kept_row) * ors] = finish<Out, Acc, POST>(kept, fp);
+                kept_row = -1;
+                n = 0;
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[slot]);
     }
 }
 

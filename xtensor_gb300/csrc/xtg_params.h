@@ -234,6 +234,10 @@ struct BatchParams {
     int has_initial;
     double initial_f;
     i64 initial_i;
+    // streamed units: the slot's layout, and the word a bounded wait sets
+    unsigned loff[XTG_KMAX_LEAVES];
+    unsigned buf_bytes;
+    int* err;
 };
 // Per-row finishing parameters (the fields the accumulators' finishers read).
 struct FinP {
