@@ -2863,11 +2863,14 @@ __global__ void __launch_bounds__(256) k_indexed(const IndexParams p) {
 }
 
 // K11: filters — xt::filter(e, cond) reads and filter / filtration writes
-// (include/xtensor/views/xindex_view.hpp:786-850).  Thread th of a tile owns
-// the 16 consecutive positions t*4096 + 16 th .. + 15, so the selected
-// elements come out in row-major order: (A) count per tile, (B) an
-// inclusive scan of the counts (the accumulator kernels), (C) every tile
-// again, each selected element to tile offset + its rank in the tile.
+// (include/xtensor/views/xindex_view.hpp:786-850), by tiles of 4096 positions
+// in row-major order: (A) count per tile, (B) one block scans the counts,
+// (C) every tile again, each selected element to tile offset + its rank in
+// the tile; a write of one scalar needs no ranks and runs as (C) alone.
+// Position i * 128 + 4 * lane + e of a warp's 512 belongs to lane `lane` as
+// bit 4 * i + e of its flags (i, e = 0 .. 3): loads of four neighbours per
+// lane are whole lines per warp, and the ranks follow from one warp scan of
+// the four counts packed into 8 bits each (at most 128 a group).
 template <class Tree, class LS, int R, bool BIG>
 XTG_DI bool filter_cond(const FilterParams& p, const Ctx<0>& c, i64 k, i64 (&ix)[R]) {
     typedef typename LS::template R<1>::type RG;
@@ -2886,70 +2889,70 @@ XTG_DI bool filter_cond(const FilterParams& p, const Ctx<0>& c, i64 k, i64 (&ix)
     return Tree::ev(rg, 0, c) != typename Tree::type(0);
 }
 
-// One flat dim (R == 1), every condition leaf contiguous (stride 1, 16-byte
-// aligned) or broadcast (stride 0): the 16 consecutive positions of a
-// thread are read with 16-byte loads.
-template <int I, class... S> struct LoadFlat16;
-template <int I> struct LoadFlat16<I> {
+// One flat dim (R == 1), every leaf contiguous (stride 1, 16-byte aligned) or
+// broadcast (stride 0): four neighbours by one load.  `st`: leaf strides.
+template <int I, class... S> struct LoadFlat4;
+template <int I> struct LoadFlat4<I> {
     template <class RG> static XTG_DI void run(RG&, const void* const*, i64, const i64 (*)[XTG_KMAX_RANK]) {}
 };
-template <int I, class S0, class... S> struct LoadFlat16<I, S0, S...> {
-    template <class RG> static XTG_DI void run(RG& rg, const void* const* ptr, i64 k0, const i64 (*st)[XTG_KMAX_RANK]) {
+template <int I, class S0, class... S> struct LoadFlat4<I, S0, S...> {
+    template <class RG> static XTG_DI void run(RG& rg, const void* const* ptr, i64 k, const i64 (*st)[XTG_KMAX_RANK]) {
         typedef typename S0::type T;
         const T* b = reinterpret_cast<const T*>(ptr[I]);
         if (st[I][0] != 0) {
-            constexpr int NV = (int)sizeof(T) * 16 / 16;  // 16-byte vectors for 16 elements
-            union { uint4 v[NV]; T e[16]; } u;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) u.v[q] = __ldg(reinterpret_cast<const uint4*>(b + k0) + q);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) rg.v[j] = u.e[j];
+            ld_contig<T, 4>(rg.v, b + k);
         } else {
             const T v = ld1<T>(b);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) rg.v[j] = v;
+            for (int j = 0; j < 4; ++j) rg.v[j] = v;
         }
-        LoadFlat16<I + 1, S...>::run(rg.rest, ptr, k0, st);
+        LoadFlat4<I + 1, S...>::run(rg.rest, ptr, k, st);
     }
 };
-template <class LS> struct CondFlat16;
-template <class... S> struct CondFlat16<LeafSet<S...>> {
-    template <class Tree> static XTG_DI unsigned run(const FilterParams& p, const Ctx<0>& c, i64 k0) {
-        typename LeafSet<S...>::template R<16>::type rg;
-        LoadFlat16<0, S...>::run(rg, p.cleaf, k0, p.cls);
-        unsigned f = 0;
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (Tree::ev(rg, j, c) != typename Tree::type(0)) f |= 1u << j;
-        return f;
+template <class LS> struct Flat4;
+template <class... S> struct Flat4<LeafSet<S...>> {
+    template <class RG> static XTG_DI void load(RG& rg, const void* const* ptr, i64 k, const i64 (*st)[XTG_KMAX_RANK]) {
+        LoadFlat4<0, S...>::run(rg, ptr, k, st);
     }
 };
-// The condition flags of positions k0 .. k0 + 15 (bit i: position k0 + i).
-template <class CTree, class CLS, int R, bool BIG, bool V16>
-XTG_DI unsigned filter_flags16(const FilterParams& p, const Ctx<0>& c, i64 k0) {
-    if (V16 && k0 + 16 <= p.n) return CondFlat16<CLS>::template run<CTree>(p, c, k0);
+// The condition flags of the lane's 16 positions of the warp's 512 from k0 on
+// (bit 4 i + e: position k0 + 128 i + 4 lane + e).
+template <class CTree, class CLS, int R, bool BIG, bool FLAT>
+XTG_DI unsigned filter_flags(const FilterParams& p, const Ctx<0>& c, i64 k0, int lane) {
     unsigned flags = 0;
+    if (FLAT && k0 + 512 <= p.n) {
+        typename CLS::template R<4>::type rg[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) Flat4<CLS>::load(rg[i], p.cleaf, k0 + 128 * i + 4 * lane, p.cls);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (CTree::ev(rg[i], e, c) != typename CTree::type(0)) flags |= 1u << (4 * i + e);
+        return flags;
+    }
 #pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-        const i64 k = k0 + i;
+    for (int q = 0; q < 16; ++q) {
+        const i64 k = k0 + 128 * (q >> 2) + 4 * lane + (q & 3);
         i64 ix[R];
-        if (k < p.n && filter_cond<CTree, CLS, R, BIG>(p, c, k, ix)) flags |= 1u << i;
+        if (k < p.n && filter_cond<CTree, CLS, R, BIG>(p, c, k, ix)) flags |= 1u << q;
     }
     return flags;
 }
 
-template <class CTree, class CLS, int R, bool BIG, bool V16 = false>
+// (A) a block per tile of 4096: its selected count
+template <class CTree, class CLS, int R, bool BIG, bool FLAT = false>
 __global__ void __launch_bounds__(256) k_filter_count(const FilterParams p) {
     pdl_wait();
     __shared__ int ws[8];
     Ctx<0> c;
     c.scal = p.cscal;
+    const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
     const i64 ntiles = (p.n + 4095) / 4096;
     for (i64 t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const i64 k0 = t * 4096 + (i64)threadIdx.x * 16;
-        int cnt = __popc(filter_flags16<CTree, CLS, R, BIG, V16>(p, c, k0));
+        int cnt = __popc(filter_flags<CTree, CLS, R, BIG, FLAT>(p, c, t * 4096 + warp * 512, lane));
         cnt = __reduce_add_sync(0xffffffffu, cnt);
-        if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = cnt;
+        if (lane == 0) ws[warp] = cnt;
         __syncthreads();
         if (threadIdx.x == 0) {
             int s = 0;
@@ -2960,81 +2963,192 @@ __global__ void __launch_bounds__(256) k_filter_count(const FilterParams p) {
     }
 }
 
-// MODE 0: out[j] = e[position]; MODE 1: dst[position] = dst op src[j]
+// (B) one block of 1024: exclusive prefixes of the tile counts and their
+// total, also into host memory (p.htotal) for the caller that waits for it.
+// (The general scan took three launches here: 17 us of the pass's 60 at 2^26
+// positions.)
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK) k_filter_scan(const FilterParams p) {
+    static_assert(BLOCK == 1024, "32 warps of partial sums");
+    pdl_wait();
+    __shared__ i64 ws[32];
+    const i64 ntiles = (p.n + 4095) / 4096;
+    const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+    i64 carry = 0;
+    for (i64 b = 0; b < ntiles; b += 4096) {
+        const i64 t0 = b + (i64)threadIdx.x * 4;
+        int v[4];
+        int s = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[j] = t0 + j < ntiles ? p.tcount[t0 + j] : 0;
+            s += v[j];
+        }
+        i64 inc = s;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const i64 y = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += y;
+        }
+        if (lane == 31) ws[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            i64 w = ws[lane];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const i64 y = __shfl_up_sync(0xffffffffu, w, d);
+                if (lane >= d) w += y;
+            }
+            ws[lane] = w;
+        }
+        __syncthreads();
+        i64 off = carry + (warp ? ws[warp - 1] : 0) + inc - s;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (t0 + j < ntiles) p.toff[t0 + j] = off;
+            off += v[j];
+        }
+        carry += ws[31];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        p.toff[ntiles] = carry;
+        if (p.htotal) {
+            *p.htotal = carry;
+            __threadfence_system();
+        }
+    }
+}
+
+// (C) MODE 0: out[j] = e[position], staged in shared memory so that a tile's
+// results leave as whole lines; nothing is written when the count is not the
+// destination's length (p.expect).  MODE 1: dst[position] = dst op src[j];
+// with SCAL the values do not depend on j.  VFLAT: the value leaves of a read
+// are flat like the condition's and are loaded four at a time too (in the
+// same 16 positions: where they are the condition's leaves, from L1).
 template <class CTree, class CLS, class VTree, class VLS, class VT, class DT, class CT, int MODE, int R, int OP, bool BIG,
-          bool V16 = false>
+          bool FLAT, bool VFLAT, bool SCAL>
 __global__ void __launch_bounds__(256) k_filter_tile(const FilterParams p) {
     pdl_wait();
     typedef typename VLS::template R<1>::type VRG;
     __shared__ int ws[9];
+    extern __shared__ __align__(16) unsigned char stage_raw[];
+    DT* const stage = reinterpret_cast<DT*>(stage_raw);
     Ctx<0> cc, vc;
     cc.scal = p.cscal;
     vc.scal = p.vscal;
     const i64 ntiles = (p.n + 4095) / 4096;
     const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+    if (MODE == 0 && p.toff[ntiles] != p.expect) return;
     for (i64 t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const i64 k0 = t * 4096 + (i64)threadIdx.x * 16;
-        unsigned flags = filter_flags16<CTree, CLS, R, BIG, V16>(p, cc, k0);
-        // exclusive prefix of the thread counts in thread order
-        const int cnt = __popc(flags);
-        int inc = cnt;
+        const i64 k0 = t * 4096 + warp * 512;
+        unsigned flags = filter_flags<CTree, CLS, R, BIG, FLAT>(p, cc, k0, lane);
+        unsigned before = 0;  // selected before this lane's part of each group, 8 bits per group
+        int total = 0;
+        if (!SCAL) {
+            const unsigned c4 = __popc(flags & 0xfu) | __popc(flags & 0xf0u) << 8 | __popc(flags & 0xf00u) << 16 |
+                                __popc(flags & 0xf000u) << 24;
+            unsigned inc = c4;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, inc, d);
-            if (lane >= d) inc += y;
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, inc, d);
+                if (lane >= d) inc += y;
+            }
+            const unsigned all = __shfl_sync(0xffffffffu, inc, 31);
+            before = inc - c4;
+            // the groups before each group of the warp
+            const int g0 = all & 255, g1 = (all >> 8) & 255, g2 = (all >> 16) & 255, g3 = all >> 24;
+            if (lane == 0) ws[warp] = g0 + g1 + g2 + g3;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                int s = 0;
+                for (int w = 0; w < 8; ++w) {
+                    const int v = ws[w];
+                    ws[w] = s;
+                    s += v;
+                }
+                ws[8] = s;
+            }
+            __syncthreads();
+            total = ws[8];
         }
-        if (lane == 31) ws[warp] = inc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int s = 0;
-            for (int w = 0; w < 8; ++w) {
-                const int v = ws[w];
-                ws[w] = s;
-                s += v;
+        // rank of this lane's first selected element of each group in the tile
+        int rank[4];
+        if (!SCAL) {
+            const unsigned all = __shfl_sync(0xffffffffu, before, 31);
+            const unsigned last = __shfl_sync(0xffffffffu, flags, 31);
+            int at = ws[warp];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                rank[i] = at + (int)((before >> (8 * i)) & 255);
+                at += (int)((all >> (8 * i)) & 255) + __popc((last >> (4 * i)) & 15u);
             }
         }
-        __syncthreads();
-        i64 j = (t ? (i64)p.tincl[t - 1] : 0) + ws[warp] + (inc - cnt);
-        while (flags) {
-            const int i = __ffs(flags) - 1;
-            flags &= flags - 1;
-            const i64 k = k0 + i;
-            i64 ix[R];
-            decode_dims<R, BIG>(p.shape, p.fd, k, ix);
-            i64 off[XTG_KMAX_LEAVES], inner[XTG_KMAX_LEAVES];
+        if constexpr (MODE == 0) {
+            if (VFLAT && k0 + 512 <= p.n) {
 #pragma unroll
-            for (int l = 0; l < VLS::N; ++l) {
-                inner[l] = 0;
-                if (MODE == 0) {
+                for (int i = 0; i < 4; ++i) {
+                    if ((flags >> (4 * i)) & 15u) {
+                        typename VLS::template R<4>::type rg;
+                        Flat4<VLS>::load(rg, p.vleaf, k0 + 128 * i + 4 * lane, p.vls);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if ((flags >> (4 * i + e)) & 1u) stage[rank[i]++] = cvt<DT>(cvt<VT>(VTree::ev(rg, e, vc)));
+                    }
+                }
+                flags = 0;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            unsigned f = (flags >> (4 * i)) & 15u;
+            while (f) {
+                const int e = __ffs(f) - 1;
+                f &= f - 1;
+                const i64 k = k0 + 128 * i + 4 * lane + e;
+                i64 ix[R];
+                decode_dims<R, BIG>(p.shape, p.fd, k, ix);
+                const i64 j = SCAL || MODE == 0 ? 0 : p.toff[t] + rank[i];
+                i64 off[XTG_KMAX_LEAVES], inner[XTG_KMAX_LEAVES];
+#pragma unroll
+                for (int l = 0; l < VLS::N; ++l) {
+                    inner[l] = 0;
+                    if (MODE == 0) {
+                        i64 o = 0;
+#pragma unroll
+                        for (int d = 0; d < R; ++d) o += ix[d] * p.vls[l][d];
+                        off[l] = o;
+                    } else {
+                        off[l] = j * p.vls[l][0];
+                    }
+                }
+                VRG rg;
+                LoadLeavesAt<VLS>::template run<1>(rg, p.vleaf, off, inner);
+                const VT v = cvt<VT>(VTree::ev(rg, 0, vc));
+                if constexpr (MODE == 0) {
+                    stage[rank[i]] = cvt<DT>(v);
+                } else {
+                    DT* dst = reinterpret_cast<DT*>(p.dst);
                     i64 o = 0;
 #pragma unroll
-                    for (int d = 0; d < R; ++d) o += ix[d] * p.vls[l][d];
-                    off[l] = o;
-                } else {
-                    off[l] = j * p.vls[l][0];
+                    for (int d = 0; d < R; ++d) o += ix[d] * p.ds[d];
+                    if (OP == 0) {
+                        dst[o] = cvt<DT>(v);
+                    } else {
+                        const CT a = cvt<CT>(dst[o]), b = cvt<CT>(v);
+                        const CT r = OP == 1 ? CT(a + b) : OP == 2 ? CT(a - b) : OP == 3 ? CT(a * b) : CT(a / b);
+                        dst[o] = cvt<DT>(r);
+                    }
                 }
+                if (!SCAL) ++rank[i];
             }
-            VRG rg;
-            LoadLeavesAt<VLS>::template run<1>(rg, p.vleaf, off, inner);
-            const VT v = cvt<VT>(VTree::ev(rg, 0, vc));
-            DT* dst = reinterpret_cast<DT*>(p.dst);
-            if (MODE == 0) {
-                dst[j * p.ds[0]] = cvt<DT>(v);
-            } else {
-                i64 o = 0;
-#pragma unroll
-                for (int d = 0; d < R; ++d) o += ix[d] * p.ds[d];
-                if (OP == 0) {
-                    dst[o] = cvt<DT>(v);
-                } else {
-                    const CT a = cvt<CT>(dst[o]), b = cvt<CT>(v);
-                    const CT r = OP == 1 ? CT(a + b) : OP == 2 ? CT(a - b) : OP == 3 ? CT(a * b) : CT(a / b);
-                    dst[o] = cvt<DT>(r);
-                }
-            }
-            ++j;
         }
-        __syncthreads();
+        if constexpr (MODE == 0) {
+            __syncthreads();
+            DT* const dst = reinterpret_cast<DT*>(p.dst) + p.toff[t] * p.ds[0];
+            for (int j = (int)threadIdx.x; j < total; j += 256) dst[j * p.ds[0]] = stage[j];
+        }
+        if (!SCAL) __syncthreads();
     }
 }
 

@@ -203,7 +203,9 @@ struct FilterParams {
     i64 ds[XTG_KMAX_RANK];                      // out stride in ds[0] (read) or dst strides (assign)
     Scalars cscal, vscal;
     int* tcount;                                // selected per tile
-    const long long* tincl;                     // inclusive selected count per tile
+    long long* toff;                            // selected before each tile; the total behind the last
+    long long* htotal;                          // host memory that takes the total too (null: none)
+    i64 expect;                                 // a read's destination length
 };
 
 // Batched evaluation: many instances of one expression shape, each a 2-D

@@ -9,9 +9,10 @@
 //  * index_view reads are a gather and writes a scatter over a device list of
 //    coordinates (K10 k_indexed, coordinates checked on the device);
 //  * filter(e, cond) and filtration(dst, cond) run by tiles of 4096
-//    row-major positions: per-tile counts of cond, their inclusive scan, then
-//    each tile's selected elements go to the tile's offset plus their rank
-//    in the tile — the order of argwhere (xindex_view.hpp:821-826).
+//    row-major positions: per-tile counts of cond, their scan, then each
+//    tile's selected elements go to the tile's offset plus their rank in the
+//    tile — the order of argwhere (xindex_view.hpp:821-826).  A write of one
+//    scalar needs no ranks: one pass.
 #include <algorithm>
 #include <cstring>
 #include <string>
@@ -94,17 +95,41 @@ bool same_shape(const Tree& t, const xtg_array& a) {
     return true;
 }
 
+// What a host thread needs to wait for a count: a word that the device writes
+// the total to and an event behind it.  One per thread, since the calls wait.
+struct CountWait {
+    long long* word = nullptr;
+    cudaEvent_t ev = nullptr;
+    xtg_status ready() {
+        if (!word) XTG_CUDA(cudaHostAlloc((void**)&word, 64, cudaHostAllocPortable | cudaHostAllocMapped));
+        if (!ev) XTG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        return XTG_OK;
+    }
+    ~CountWait() {
+        if (word) cudaFreeHost(word);
+        if (ev) cudaEventDestroy(ev);
+    }
+};
+CountWait& count_wait() {
+    static thread_local CountWait w;
+    return w;
+}
+
 // Filters run by tiles of 4096 row-major positions: per-tile counts of the
-// condition (K11 k_filter_count), their inclusive scan (the accumulator
-// kernels, int64), then the compaction / write kernel.  FilterRun holds the
-// scratch (counts + scan) and the condition's part of the parameters.
+// condition (K11 k_filter_count), their scan (k_filter_scan), then the
+// compaction / write kernel.  FilterRun holds the scratch (counts + offsets)
+// and the condition's part of the parameters.
+bool flat_leaf(const xtg_array& a, int64_t stride) {
+    return stride == 0 || (stride == 1 && ((uintptr_t)a.data % 16) == 0);
+}
+
 struct FilterRun {
     xtg::FilterParams p;
     Tree tc;
     void* scratch = nullptr;
     int64_t ntiles = 0;
     bool big = false;
-    bool v16 = false;  // one flat dim, condition leaves contiguous (aligned) or broadcast: 16-byte loads
+    bool flat = false;  // one flat dim, condition leaves contiguous (aligned) or broadcast: loads of four
     int rank = 1;  // of the position space after merging dims that are contiguous for every array
     std::string ctree, cls;
     std::vector<std::array<int64_t, XTG_MAX_RANK>> extra;  // the callers' position strides, merged alike
@@ -114,7 +139,7 @@ struct FilterRun {
 // addresses by position (the value leaves of a read, the destination of an
 // assignment).  Dims that are contiguous for the condition and all of them
 // merge (row-major order is kept), so a contiguous filter walks one flat dim.
-xtg_status filter_prepare(const xtg_expr* cond, int rank, const int64_t* shape, FilterRun& F, cudaStream_t stream,
+xtg_status filter_prepare(const xtg_expr* cond, int rank, const int64_t* shape, FilterRun& F,
                           const std::vector<std::array<int64_t, XTG_MAX_RANK>>& extra = {}) {
     XTG_TRY(build_tree(cond, false, F.tc));
     if (F.tc.n_rstats) return fail(XTG_ERR_UNSUPPORTED, "row statistics inside a filter condition");
@@ -152,55 +177,47 @@ xtg_status filter_prepare(const xtg_expr* cond, int rank, const int64_t* shape, 
     for (int l = 0; l < NL; ++l)
         for (int d = 0; d < D.R; ++d) F.p.cls[l][d] = D.st[l][d];
     F.extra.assign(D.st.begin() + NL, D.st.begin() + NL + extra.size());
-    F.v16 = F.rank == 1;
-    for (int l = 0; F.v16 && l < NL; ++l) {
-        const int64_t st = F.p.cls[l][0];
-        F.v16 = st == 0 || (st == 1 && ((uintptr_t)F.tc.leaves[l].data % 16) == 0);
-    }
+    F.flat = F.rank == 1;
+    for (int l = 0; F.flat && l < NL; ++l) F.flat = flat_leaf(F.tc.leaves[l], F.p.cls[l][0]);
     for (size_t i = 0; i < F.tc.scalars.size(); ++i) F.p.cscal.v[i] = F.tc.scalars[i];
     std::vector<int> map(NL);
     for (int l = 0; l < NL; ++l) map[l] = l;
     F.ctree = tree_type(F.tc, F.tc.root, map);
     F.cls = leafset_of(F.tc);
     F.ntiles = (n + 4095) / 4096;
+    return XTG_OK;
+}
+
+// The tile counts, their offsets and (wait) the total on its way to the host.
+xtg_status filter_offsets(FilterRun& F, bool wait, cudaStream_t stream) {
     if (F.ntiles == 0) return XTG_OK;
-    // scratch: int32 counts, then int64 inclusive counts
+    // scratch: int32 counts, then int64 offsets
     const size_t cbytes = (size_t)((F.ntiles * 4 + 15) / 16 * 16);
-    XTG_TRY(scratch_alloc(&F.scratch, cbytes + (size_t)F.ntiles * 8, stream));
+    XTG_TRY(scratch_alloc(&F.scratch, cbytes + (size_t)(F.ntiles + 1) * 8, stream));
     F.p.tcount = (int*)F.scratch;
-    F.p.tincl = (const long long*)((char*)F.scratch + cbytes);
+    F.p.toff = (long long*)((char*)F.scratch + cbytes);
     if (recorder()) recorder()->nocache = true;  // scratch addresses are baked into several parameter blocks
     Kernel* k;
     XTG_TRY(get_kernel("xtg::k_filter_count<" + F.ctree + ", " + F.cls + ", " + std::to_string(F.rank) + ", " +
-                           (F.big ? "true" : "false") + ", " + (F.v16 ? "true" : "false") + ">",
+                           (F.big ? "true" : "false") + ", " + (F.flat ? "true" : "false") + ">",
                        256, &k));
     XTG_TRY(launch(k, grid_n(k, F.ntiles * 256), 256, &F.p, stream));
-    // inclusive scan of the int32 counts into int64
-    xtg_expr ce;
-    memset(&ce, 0, sizeof ce);
-    xtg_array ca;
-    memset(&ca, 0, sizeof ca);
-    ca.data = F.scratch;
-    ca.dtype = XTG_INT32;
-    ca.rank = 1;
-    ca.shape[0] = F.ntiles;
-    ca.strides[0] = 1;
-    XTG_TRY(push_leaf(ce, ca));
-    xtg_array ia = ca;
-    ia.data = (void*)F.p.tincl;
-    ia.dtype = XTG_INT64;
-    return accumulate_call(&ce, XTG_ACC_CUMSUM, 0, 0, XTG_INT64, &ia, stream);
+    if (wait && !dry_run()) {
+        XTG_TRY(count_wait().ready());
+        F.p.htotal = count_wait().word;
+    }
+    XTG_TRY(get_kernel("xtg::k_filter_scan<1024>", 1024, &k));
+    XTG_TRY(launch(k, 1, 1024, &F.p, stream));
+    if (wait && !dry_run()) XTG_CUDA(cudaEventRecord(count_wait().ev, stream));
+    return XTG_OK;
 }
 
-xtg_status filter_total(const FilterRun& F, int64_t* count, cudaStream_t stream) {
-    if (F.ntiles == 0 || dry_run()) {
-        *count = 0;
-        return XTG_OK;
-    }
-    long long c = 0;
-    XTG_CUDA(cudaMemcpyAsync(&c, F.p.tincl + (F.ntiles - 1), 8, cudaMemcpyDeviceToHost, stream));
-    XTG_CUDA(cudaStreamSynchronize(stream));
-    *count = c;
+// The total that filter_offsets(wait) sent.
+xtg_status filter_total(const FilterRun& F, int64_t* count) {
+    *count = 0;
+    if (F.ntiles == 0 || dry_run()) return XTG_OK;
+    XTG_CUDA(cudaEventSynchronize(count_wait().ev));
+    *count = *(volatile long long*)count_wait().word;
     return XTG_OK;
 }
 
@@ -223,8 +240,10 @@ std::vector<std::array<int64_t, XTG_MAX_RANK>> filter_extra(const Tree& tv, int 
     return ex;
 }
 
-xtg_status filter_launch(FilterRun& F, const Tree& tv, int mode, int op, const xtg_array& dst, cudaStream_t stream) {
+xtg_status filter_launch(FilterRun& F, const Tree& tv, int mode, int op, bool scalar, const xtg_array& dst, cudaStream_t stream) {
     const int NL = (int)tv.leaves.size();
+    bool vflat = mode == 0 && F.rank == 1;
+    for (int l = 0; vflat && l < NL; ++l) vflat = flat_leaf(tv.leaves[l], F.extra[l][0]);
     for (int l = 0; l < NL; ++l) {
         F.p.vleaf[l] = tv.leaves[l].data;
         if (mode == 0) {
@@ -249,10 +268,12 @@ xtg_status filter_launch(FilterRun& F, const Tree& tv, int mode, int op, const x
     std::string name = "xtg::k_filter_tile<" + F.ctree + ", " + F.cls + ", " + tree_type(tv, tv.root, map) + ", " +
                        leafset_of(tv) + ", " + dt(vt).cname + ", " + dt(dst.dtype).cname + ", " + dt(ct).cname + ", " +
                        std::to_string(mode) + ", " + std::to_string(rank) + ", " + std::to_string(op) + ", " +
-                       (F.big ? "true" : "false") + ", " + (F.v16 ? "true" : "false") + ">";
+                       (F.big ? "true" : "false") + ", " + (F.flat ? "true" : "false") + ", " +
+                       (vflat ? "true" : "false") + ", " + (scalar ? "true" : "false") + ">";
     Kernel* k;
-    XTG_TRY(get_kernel(name, 256, &k));
-    return launch(k, grid_n(k, F.ntiles * 256), 256, &F.p, stream);
+    const size_t stage = mode == 0 ? 4096 * (size_t)dt(dst.dtype).size : 0;  // a tile's results
+    XTG_TRY(get_kernel(name, 256, &k, stage));
+    return launch(k, grid_n(k, F.ntiles * 256), 256, &F.p, stream, stage);
 }
 
 // K10 launch
@@ -361,8 +382,9 @@ xtg_status xtg_filter_count(const xtg_expr* cond, int64_t* count, xtg_stream str
     Tree tc;
     XTG_TRY(build_tree(cond, false, tc));
     FilterRun F;
-    xtg_status st = filter_prepare(cond, tc.rank, tc.shape, F, (cudaStream_t)stream);
-    if (st == XTG_OK) st = filter_total(F, count, (cudaStream_t)stream);
+    xtg_status st = filter_prepare(cond, tc.rank, tc.shape, F);
+    if (st == XTG_OK) st = filter_offsets(F, true, (cudaStream_t)stream);
+    if (st == XTG_OK) st = filter_total(F, count);
     xtg_status fs = F.scratch ? scratch_free(F.scratch, (cudaStream_t)stream) : XTG_OK;
     return st != XTG_OK ? st : fs;
 }
@@ -376,12 +398,16 @@ xtg_status xtg_filter(const xtg_expr* e, const xtg_expr* cond, const xtg_array* 
     if (t.rank < 1) return fail(XTG_ERR_INVALID, "filter of a 0-d expression");
     if (out->rank != 1) return fail(XTG_ERR_SHAPE, "filter result must be 1-D");
     FilterRun F;
-    xtg_status st = filter_prepare(cond, t.rank, t.shape, F, (cudaStream_t)stream, filter_extra(t, 0, t.rank, t.shape, *out));
+    xtg_status st = filter_prepare(cond, t.rank, t.shape, F, filter_extra(t, 0, t.rank, t.shape, *out));
+    if (st == XTG_OK) st = filter_offsets(F, true, (cudaStream_t)stream);
+    // the compaction is queued behind the offsets before the host has the
+    // count; it writes nothing when the destination has another length
+    F.p.expect = out->shape[0];
+    if (st == XTG_OK && F.ntiles) st = filter_launch(F, t, 0, 0, false, *out, (cudaStream_t)stream);
     int64_t count = 0;
-    if (st == XTG_OK) st = filter_total(F, &count, (cudaStream_t)stream);
+    if (st == XTG_OK) st = filter_total(F, &count);
     if (st == XTG_OK && !dry_run() && out->shape[0] != count)
         st = fail(XTG_ERR_SHAPE, "filter result must be 1-D of xtg_filter_count elements");
-    if (st == XTG_OK && F.ntiles) st = filter_launch(F, t, 0, 0, *out, (cudaStream_t)stream);
     xtg_status fs = F.scratch ? scratch_free(F.scratch, (cudaStream_t)stream) : XTG_OK;
     return st != XTG_OK ? st : fs;
 }
@@ -397,15 +423,16 @@ xtg_status xtg_filter_assign(const xtg_expr* src, const xtg_expr* cond, int32_t 
     if (t.rank > 1) return fail(XTG_ERR_BROADCAST, "values assigned through a filter must be 1-D or a scalar");
     if (dst->rank < 1) return fail(XTG_ERR_INVALID, "filter of a 0-d array");
     FilterRun F;
-    xtg_status st = filter_prepare(cond, dst->rank, dst->shape, F, (cudaStream_t)stream,
-                                   filter_extra(t, 1, dst->rank, dst->shape, *dst));
-    if (st == XTG_OK && t.rank == 1 && t.shape[0] != 1) {
+    xtg_status st = filter_prepare(cond, dst->rank, dst->shape, F, filter_extra(t, 1, dst->rank, dst->shape, *dst));
+    const bool scalar = t.rank == 0 || t.shape[0] == 1;
+    if (st == XTG_OK && !scalar) {
+        st = filter_offsets(F, true, (cudaStream_t)stream);
         int64_t count = 0;
-        st = filter_total(F, &count, (cudaStream_t)stream);
+        if (st == XTG_OK) st = filter_total(F, &count);
         if (st == XTG_OK && !dry_run() && t.shape[0] != count)
             st = fail(XTG_ERR_BROADCAST, "assigned values do not match the filter's length");
     }
-    if (st == XTG_OK && F.ntiles) st = filter_launch(F, t, 1, op, *dst, (cudaStream_t)stream);
+    if (st == XTG_OK && F.ntiles) st = filter_launch(F, t, 1, op, scalar, *dst, (cudaStream_t)stream);
     xtg_status fs = F.scratch ? scratch_free(F.scratch, (cudaStream_t)stream) : XTG_OK;
     return st != XTG_OK ? st : fs;
 }
