@@ -68,6 +68,11 @@ int64_t opt(const char* key, int64_t dflt);
 // Default work items a ROW reduction is split into (reduce.target_items):
 // shared by every planner of a reduction so equal calls partition alike.
 constexpr int64_t kReduceTargetItems = 2048;
+struct HotOpts {
+    int64_t gen = -1;  // option generation these were read at
+    bool dry_run = false, plan_cache = true, pdl = true;
+};
+const HotOpts& hot_opts();
 // Option "jit.dry_run": plan and compile kernels without a GPU (no launches).
 bool dry_run();
 
@@ -120,12 +125,15 @@ struct RecLaunch {
     unsigned grid, block;
     size_t smem;
     std::vector<unsigned char> params;
-    int scratch_off;
+    int scratch_off;      // byte offset of the scratch pointer in params (-1: none)
+    size_t scratch_base;  // what it points to: this far into the replay's scratch block
 };
 struct Recorder {
     std::vector<RecLaunch> launches;
+    // the call's scratch allocations back to back (each at a multiple of 256
+    // bytes); a launch with a scratch pointer uses the one made last
     size_t scratch_bytes = 0;
-    int scratch_allocs = 0;
+    size_t scratch_last = 0;
     bool nocache = false;  // a launch holds a temporary the replay could not patch
 };
 Recorder*& recorder();  // the calling thread's active recorder (nullptr: none)

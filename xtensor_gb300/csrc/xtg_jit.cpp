@@ -318,6 +318,7 @@ xtg_status launch_raw(Kernel* k, unsigned grid, unsigned block, const void* para
         l.smem = dyn_smem;
         l.params.assign((const unsigned char*)params, (const unsigned char*)params + psize);
         l.scratch_off = scratch_off;
+        l.scratch_base = rec->scratch_last;
         rec->launches.push_back(std::move(l));
     }
     t_last_kernels.push_back(k);
@@ -326,7 +327,7 @@ xtg_status launch_raw(Kernel* k, unsigned grid, unsigned block, const void* para
         return XTG_OK;
     }
     void* args[1] = {const_cast<void*>(params)};
-    if (opt("launch.pdl", 1)) {
+    if (hot_opts().pdl) {
         // programmatic dependent launch: the kernel may be set up while the
         // one before it drains (every kernel waits for its predecessors on
         // entry, griddepcontrol.wait)

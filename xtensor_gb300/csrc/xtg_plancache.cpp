@@ -9,6 +9,7 @@
 // split-reduction scratch and patching its address into the parameter
 // blocks.  Serving loops that evaluate the same request shapes over and over
 // skip the host-side planning entirely.
+#include <algorithm>
 #include <cstring>
 #include <list>
 #include <memory>
@@ -57,63 +58,74 @@ uint64_t fnv(const std::vector<unsigned char>& v) {
     return h;
 }
 
-template <class T> void put(std::vector<unsigned char>& k, const T& v) {
-    const unsigned char* p = (const unsigned char*)&v;
-    k.insert(k.end(), p, p + sizeof(T));
-}
-
-void put_array(std::vector<unsigned char>& k, const xtg_array& a) {
-    put(k, a.data);
-    put(k, a.dtype);
-    put(k, a.rank);
-    for (int d = 0; d < a.rank && d < XTG_MAX_RANK; ++d) {
-        put(k, a.shape[d]);
-        put(k, a.strides[d]);
+// Appends to a key whose buffer is already long enough.
+struct KeyWriter {
+    unsigned char* at;
+    void bytes(const void* p, size_t n) {
+        memcpy(at, p, n);
+        at += n;
     }
-}
+    template <class T> void put(const T& v) { bytes(&v, sizeof v); }
+    void array(const xtg_array& a) {
+        put(a.data);
+        put(a.dtype);
+        put(a.rank);
+        const size_t r = (size_t)std::max(0, std::min(a.rank, (int32_t)XTG_MAX_RANK));
+        bytes(a.shape, r * sizeof a.shape[0]);
+        bytes(a.strides, r * sizeof a.strides[0]);
+    }
+};
+constexpr size_t kArrayKey = 16 + 2 * XTG_MAX_RANK * sizeof(int64_t);
 
 }  // namespace
 
-bool plan_cache_enabled() { return !dry_run() && opt("plan.cache", 1) != 0; }
+bool plan_cache_enabled() { return !hot_opts().dry_run && hot_opts().plan_cache; }
 
 std::vector<unsigned char>& plan_key(int kind, const xtg_expr* e, const xtg_reduce_desc* rd, const xtg_array* out,
-                                     int32_t a0, int32_t a1, int64_t a2, const xtg_array* out2) {
+                                     int32_t a0, int32_t a1, int64_t a2, const xtg_array* const* more, int n_more) {
     // one buffer per thread, reused: no allocation on the replay path
     static thread_local std::vector<unsigned char> k;
-    k.clear();
-    k.reserve(1024);
-    put(k, kind);
-    put(k, opt_generation());
-    put(k, e->n_nodes);
-    put(k, e->n_leaves);
-    for (int i = 0; i < e->n_nodes && i < XTG_MAX_NODES; ++i) put(k, e->nodes[i]);
-    for (int i = 0; i < e->n_leaves && i < XTG_MAX_LEAVES; ++i) put_array(k, e->leaves[i]);
+    const int nn = std::max(0, std::min(e->n_nodes, (int32_t)XTG_MAX_NODES));
+    const int nl = std::max(0, std::min(e->n_leaves, (int32_t)XTG_MAX_LEAVES));
+    k.resize(256 + nn * sizeof(xtg_node) + sizeof(xtg_reduce_desc) + (nl + 1 + n_more) * kArrayKey);
+    KeyWriter w{k.data()};
+    w.put(kind);
+    w.put(opt_generation());
+    w.put(e->n_nodes);
+    w.put(e->n_leaves);
+    w.bytes(e->nodes, nn * sizeof(xtg_node));
+    for (int i = 0; i < nl; ++i) w.array(e->leaves[i]);
     if (rd) {
-        put(k, rd->op);
-        put(k, rd->n_axes);
-        for (int i = 0; i < rd->n_axes && i < XTG_MAX_RANK; ++i) put(k, rd->axes[i]);
-        put(k, rd->keep_dims);
-        put(k, rd->has_initial);
-        put(k, rd->initial);
-        put(k, rd->acc_dtype);
-        put(k, rd->precision);
-        put(k, rd->ddof);
+        w.put(rd->op);
+        w.put(rd->n_axes);
+        w.bytes(rd->axes, (size_t)std::max(0, std::min(rd->n_axes, (int32_t)XTG_MAX_RANK)) * sizeof rd->axes[0]);
+        w.put(rd->keep_dims);
+        w.put(rd->has_initial);
+        w.put(rd->initial);
+        w.put(rd->acc_dtype);
+        w.put(rd->precision);
+        w.put(rd->ddof);
     }
-    put(k, a0);
-    put(k, a1);
-    put(k, a2);
-    put_array(k, *out);
-    if (out2) put_array(k, *out2);
+    w.put(a0);
+    w.put(a1);
+    w.put(a2);
+    w.array(*out);
+    for (int i = 0; i < n_more; ++i) {
+        w.put((int32_t)(more[i] != nullptr));
+        if (more[i]) w.array(*more[i]);
+    }
+    k.resize((size_t)(w.at - k.data()));
     return k;
 }
 
 // Replays a cached plan for `key`; false if there is none.
 bool plan_replay(const std::vector<unsigned char>& key, cudaStream_t s, xtg_status* st) {
     std::shared_ptr<Plan> p;
+    const uint64_t h = fnv(key);
     {
         Cache& c = cache();
         std::lock_guard<std::mutex> lk(c.mu);
-        auto it = c.map.find(fnv(key));
+        auto it = c.map.find(h);
         if (it == c.map.end()) return false;
         for (auto& cand : it->second)
             if (cand->key == key) p = cand;
@@ -127,13 +139,18 @@ bool plan_replay(const std::vector<unsigned char>& key, cudaStream_t s, xtg_stat
     unsigned char buf[8192];
     *st = XTG_OK;
     for (const RecLaunch& l : p->launches) {
-        if (l.params.size() > sizeof buf) {
-            *st = fail(XTG_ERR_INVALID, "parameter block too large");
-            break;
+        const void* params = l.params.data();
+        if (l.scratch_off >= 0) {
+            if (l.params.size() > sizeof buf) {
+                *st = fail(XTG_ERR_INVALID, "parameter block too large");
+                break;
+            }
+            memcpy(buf, l.params.data(), l.params.size());
+            void* mine = (char*)scratch + l.scratch_base;
+            memcpy(buf + l.scratch_off, &mine, sizeof mine);
+            params = buf;
         }
-        memcpy(buf, l.params.data(), l.params.size());
-        if (l.scratch_off >= 0) memcpy(buf + l.scratch_off, &scratch, sizeof(void*));
-        *st = launch_raw(l.k, l.grid, l.block, buf, l.params.size(), s, l.smem, -1);
+        *st = launch_raw(l.k, l.grid, l.block, params, l.params.size(), s, l.smem, -1);
         if (*st != XTG_OK) break;
     }
     if (scratch) {
@@ -144,11 +161,11 @@ bool plan_replay(const std::vector<unsigned char>& key, cudaStream_t s, xtg_stat
 }
 
 void plan_store(const std::vector<unsigned char>& key, Recorder& rec) {
-    if (rec.scratch_allocs > 1 || rec.nocache) return;  // keep such calls uncached
+    if (rec.nocache) return;
     auto p = std::make_shared<Plan>();
     p->key = key;
     p->launches = std::move(rec.launches);
-    p->scratch_bytes = rec.scratch_allocs ? rec.scratch_bytes : 0;
+    p->scratch_bytes = rec.scratch_bytes;
     for (auto& l : p->launches)
         if (l.scratch_off >= 0 && !p->scratch_bytes) return;
     Cache& c = cache();

@@ -824,7 +824,9 @@ xtg_status xtg_reduce_moments(const xtg_expr* e, const xtg_reduce_desc* rd, cons
     begin_call();
     if (!e) return fail(XTG_ERR_INVALID, "null expression");
     const xtg_array* outs[4] = {sum, mean, variance, norm_l2};
-    return moments_impl(e, rd, outs, (cudaStream_t)stream);
+    const xtg_array* first = sum ? sum : mean ? mean : variance ? variance : norm_l2;
+    return with_plan_cache(5, e, rd, first, 0, 0, 0, (cudaStream_t)stream,
+                           [&]() { return moments_impl(e, rd, outs, (cudaStream_t)stream); }, outs, 4);
 }
 
 xtg_status xtg_assign_reduce(const xtg_expr* e, const xtg_array* out_e, const xtg_reduce_desc* rd,
@@ -833,7 +835,7 @@ xtg_status xtg_assign_reduce(const xtg_expr* e, const xtg_array* out_e, const xt
     if (!e || !rd || !out_e || !out_r) return fail(XTG_ERR_INVALID, "null argument");
     return with_plan_cache(
         4, e, rd, out_r, 0, 0, 0, (cudaStream_t)stream,
-        [&]() { return assign_reduce_impl(e, out_e, rd, out_r, (cudaStream_t)stream); }, out_e);
+        [&]() { return assign_reduce_impl(e, out_e, rd, out_r, (cudaStream_t)stream); }, &out_e, 1);
 }
 
 xtg_status xtg_reduce_shape(const xtg_expr* e, const xtg_reduce_desc* rd, int32_t* rank, int64_t* shape,

@@ -2,6 +2,7 @@
 // reporting of the C ABI.  xtensor reports failures by exceptions
 // (XTENSOR_THROW, include/xtensor/core/xtensor_config.hpp:27-33); across a C
 // ABI they become xtg_status codes plus a thread-local message.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -107,7 +108,7 @@ static xtg_status init_locked(int device) {
     return XTG_OK;
 }
 
-bool dry_run() { return opt("jit.dry_run", 0) != 0; }
+bool dry_run() { return hot_opts().dry_run; }
 
 xtg_status ensure_device(DeviceInfo** info) {
     if (dry_run()) {
@@ -143,17 +144,60 @@ int64_t opt(const char* key, int64_t dflt) {
     return it == g_opts.end() ? dflt : it->second;
 }
 
+// The options that every call looks at, read again only after an option has
+// changed (a lookup takes the options' lock and builds a string).
+const HotOpts& hot_opts() {
+    static thread_local HotOpts h;
+    const int64_t gen = opt_generation();
+    if (h.gen != gen) {
+        h.dry_run = opt("jit.dry_run", 0) != 0;
+        h.plan_cache = opt("plan.cache", 1) != 0;
+        h.pdl = opt("launch.pdl", 1) != 0;
+        h.gen = gen;
+    }
+    return h;
+}
+
+// Scratch comes from a stream-ordered pool of the library's own that keeps up
+// to scratch.keep_mib (64) of freed memory for the next call; the rest goes
+// back to the device at the next synchronisation.  (The device's default pool
+// keeps nothing: a full reduction after a synchronisation waited 180 us for
+// its few kilobytes.)  Allocation and free are ordered by their streams, so
+// calls on several streams and threads share the pool safely.
+static std::mutex g_pool_mu;
+static std::atomic<cudaMemPool_t> g_pool{nullptr};
+
+static xtg_status scratch_pool(cudaMemPool_t* pool) {
+    if ((*pool = g_pool.load(std::memory_order_acquire))) return XTG_OK;
+    DeviceInfo* dev;
+    XTG_TRY(ensure_device(&dev));
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if ((*pool = g_pool.load(std::memory_order_acquire))) return XTG_OK;
+    cudaMemPoolProps pr;
+    memset(&pr, 0, sizeof pr);
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.location.type = cudaMemLocationTypeDevice;
+    pr.location.id = dev->device;
+    XTG_CUDA(cudaMemPoolCreate(pool, &pr));
+    uint64_t keep = (uint64_t)std::max<int64_t>(0, opt("scratch.keep_mib", 64)) << 20;
+    XTG_CUDA(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    g_pool.store(*pool, std::memory_order_release);
+    return XTG_OK;
+}
+
 xtg_status scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
     if (bytes == 0) bytes = 16;
     if (Recorder* rec = recorder()) {
-        rec->scratch_bytes = bytes;
-        rec->scratch_allocs++;
+        rec->scratch_last = rec->scratch_bytes;
+        rec->scratch_bytes += (bytes + 255) & ~(size_t)255;
     }
     if (dry_run()) {
         *p = (void*)(uintptr_t)0x7f0000000000ull;
         return XTG_OK;
     }
-    XTG_CUDA(cudaMallocAsync(p, bytes, s));
+    cudaMemPool_t pool;
+    XTG_TRY(scratch_pool(&pool));
+    XTG_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, s));
     return XTG_OK;
 }
 static int* g_err_word = nullptr;

@@ -344,9 +344,11 @@ xtg_status xtg_masked_assign(const xtg_expr* src, const xtg_expr* mask, int32_t 
     }
     XTG_TRY(push_leaf(e, *dst));
     XTG_TRY(push_op(e, XTG_OP_WHERE));
-    Tree t;
-    XTG_TRY(build_tree(&e, opt("fp32_compute", 1) != 0 && dst->dtype != XTG_FLOAT64, t));
-    return assign_guarded(t, dst, (cudaStream_t)stream);
+    return with_plan_cache(6, &e, nullptr, dst, 0, 0, 0, (cudaStream_t)stream, [&]() -> xtg_status {
+        Tree t;
+        XTG_TRY(build_tree(&e, opt("fp32_compute", 1) != 0 && dst->dtype != XTG_FLOAT64, t));
+        return assign_guarded(t, dst, (cudaStream_t)stream);
+    });
 }
 
 xtg_status xtg_gather(const xtg_expr* e, const int64_t* indices, int64_t n, const xtg_array* out, xtg_stream stream) {
