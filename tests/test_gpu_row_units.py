@@ -35,9 +35,9 @@ def check(x, got, rel, what):
 @pytest.mark.parametrize("dt", ["float32", "float64"])
 @pytest.mark.parametrize("cols", [1, 3, 4, 5, 16, 17, 51, 64, 65, 127, 128, 129, 256, 257, 511, 512, 513, 777, 1023,
                                   1025, 2047, 2049, 4095])
-def test_row_lengths(dt, cols):
+@pytest.mark.parametrize("rows", [203, 5003])  # one wave of warps, and more; no multiples of the rows per unit
+def test_row_lengths(dt, cols, rows):
     g = rng(cols)
-    rows = 203  # no multiple of the rows per unit, block or vector
     flat = g.standard_normal(rows * cols + 8).astype(dt)
     d = DeviceArray.from_numpy(flat)
     for off in (0, 1, 3):  # rows from every phase of a 16-byte granule
@@ -71,7 +71,7 @@ def test_special_rows_beside_plain_ones(cols):
     """float64 rows with an infinity or NaN take the FP64 path; the rows that
     share their warp keep the fixed-point results, bit for bit."""
     g = rng(cols)
-    x = g.standard_normal((64, cols))
+    x = g.standard_normal((5003, cols))
     y = x.copy()
     y[::3, cols // 2] = np.inf
     y[1::9, 0] = np.nan

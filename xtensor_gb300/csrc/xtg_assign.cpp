@@ -99,6 +99,11 @@ static unsigned grid_for(Kernel* k, int64_t blocks_needed) {
     return (unsigned)std::max<int64_t>(g, 1);
 }
 
+static int dev_sms() {
+    DeviceInfo* dev = nullptr;
+    return ensure_device(&dev) == XTG_OK ? dev->sm_count : 1;
+}
+
 // Subtree broadcast shape (right-aligned extents of the leaves below node n).
 static void subtree_shape(const Tree& t, int n, int& rank, int64_t* sh) {
     std::vector<int> stack{n};
@@ -370,6 +375,9 @@ static xtg_status assign_rowfused(const Tree& t, const xtg_array& out, int R, co
     const int64_t most = maxsz >= 8 ? 32 : (vec > 1 ? 16 : 48);
     int group = vec > 1 ? 1 : 4;
     while (group < 32 && nvec * vec > group * most) group *= 2;
+    // few rows spread over more lanes (208 float64 rows of 128: 5.9 us with 4
+    // lanes per row, 3.0 with 32)
+    while (group < 32 && n_rows * group < 4096 * 32 && group < nvec) group *= 2;
     if (nvec > 32 * 16) group = 256;
     // A lane's vectors of the row, rounded up in steps that keep the number
     // of kernels for all row lengths small; the first `nf` of them lie inside
@@ -457,6 +465,10 @@ static xtg_status assign_rowfused(const Tree& t, const xtg_array& out, int R, co
     // of the row each, and a buffer per warp leave few warps resident (60000
     // float64 rows of 2048: 648 us with a warp, 455 with a block).
     if (tgroup == 256) tgroup = row_bytes > 8192 ? 128 : 32;
+    // rows of any alignment that one wave of warps takes at once: there is no
+    // next unit to copy meanwhile, and plain loads start sooner (4490 x 51
+    // float32: 3.4 us copied, 3.1 loaded)
+    if (edge && tgroup <= 32 && n_rows * tgroup <= (int64_t)dev_sms() * 32 * 32) tma = false;
     const int nbuf = opt("row.tma_buffers", 1) == 2 && tgroup == 32 && !edge ? 2 : 1;
     const int unit_rows = tgroup < 32 ? 32 / tgroup : 1;
     unsigned buf_bytes = 0;
