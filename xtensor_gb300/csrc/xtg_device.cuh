@@ -1918,7 +1918,37 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
 // or 16 bytes) the loads are asynchronous copies into a per-thread ring of
 // RS stages in shared memory: RS - 1 rows in flight without registers.
 // Work items: w = s * n_outv + ov (consecutive threads -> consecutive outputs).
-template <class Tree, class LS, class Acc, class Out, int POST, int VEC, int RO, int RR, int U, bool BIG, int RS = 0>
+// LSTR: rows that vectors do not divide.  A warp owns 32 * VEC consecutive
+// outputs, a thread the VEC of them 32 apart, so its loads of one row are
+// single elements but whole lines per warp, and the row's address and the loop
+// are shared by VEC elements (argmax of odd float32 rows spent two thirds of
+// the ALU on them).  Outputs past the row's end read the thread's first.
+template <int I, int VEC, class... S> struct LoadLane;
+template <int I, int VEC> struct LoadLane<I, VEC> {
+    template <class RG> static XTG_DI void run(RG&, const void* const*, const i64*, const int*) {}
+};
+template <int I, int VEC, class S0, class... S> struct LoadLane<I, VEC, S0, S...> {
+    template <class RG> static XTG_DI void run(RG& rg, const void* const* leaf, const i64* off, const int* dj) {
+        typedef typename S0::type T;
+        const T* b = reinterpret_cast<const T*>(leaf[I]) + off[I];
+        if (S0::kind == K_BCAST) {
+            const T v = ld1<T>(b);
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) rg.v[j] = v;
+        } else {
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) rg.v[j] = ld1<T>(b + dj[j]);
+        }
+        LoadLane<I + 1, VEC, S...>::run(rg.rest, leaf, off, dj);
+    }
+};
+template <class LS> struct LoadLanes;
+template <class... S> struct LoadLanes<LeafSet<S...>> {
+    template <int VEC, class RG> static XTG_DI void run(RG& rg, const void* const* leaf, const i64* off, const int* dj) {
+        LoadLane<0, VEC, S...>::run(rg, leaf, off, dj);
+    }
+};
+template <class Tree, class LS, class Acc, class Out, int POST, int VEC, int RO, int RR, int U, bool BIG, int RS = 0, bool LSTR = false>
 __global__ void __launch_bounds__(256) k_reduce_col(const RedParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
@@ -1934,7 +1964,23 @@ __global__ void __launch_bounds__(256) k_reduce_col(const RedParams p) {
         const i64 ov = w - s * p.n_outv;
         i64 ko[RO];
         decode_dims<RO, BIG>(p.oshape, p.ofd, ov, ko);
-        ko[RO - 1] *= VEC;
+        int dj[VEC];  // LSTR: this thread's outputs from its first
+        bool mine[VEC];
+        if constexpr (LSTR) {
+            const i64 col = ko[RO - 1] / 32 * (32 * VEC) + ko[RO - 1] % 32;
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) {
+                mine[j] = col + 32 * j < p.inner;
+                dj[j] = mine[j] ? 32 * j : 0;
+            }
+            ko[RO - 1] = mine[0] ? col : p.inner - 1;
+        } else {
+            ko[RO - 1] *= VEC;
+        }
+        auto load = [&](RG& rg, const i64* off) {
+            if constexpr (LSTR) LoadLanes<LS>::template run<VEC>(rg, p.leaf, off, dj);
+            else LoadLeavesAt<LS>::template run<VEC>(rg, p.leaf, off, inner);
+        };
         Acc acc[VEC];
 #pragma unroll
         for (int j = 0; j < VEC; ++j) acc[j].init(p);
@@ -1945,7 +1991,7 @@ __global__ void __launch_bounds__(256) k_reduce_col(const RedParams p) {
             i64 off[XTG_KMAX_LEAVES];
             red_offsets<LS::N, RO, RR>(p, ko, r0, off);
             RG rg;
-            LoadLeavesAt<LS>::template run<VEC>(rg, p.leaf, off, inner);
+            load(rg, off);
 #pragma unroll
             for (int j = 0; j < VEC; ++j) Shift<Acc>::set(acc[j], Tree::ev(rg, j, c));
         }
@@ -2028,35 +2074,70 @@ __global__ void __launch_bounds__(256) k_reduce_col(const RedParams p) {
             }
             cp_async_wait<0>();
         } else {
-        for (i64 r = rb; r < re; r += U) {
-            RG rg[U];
+            // held arg-updates keep 32-bit row offsets, as in the ring
+            u32 bo[VEC];
+            bool h32 = false;
+            const bool can32 = re - rb <= (i64)0xFFFFFFFF;
+            auto step = [&](const RG& rg, i64 r) {
+                if constexpr (HeldFast<Acc>::value) {
+                    if (h32) {
+                        const u32 ro = (u32)(r - rb);
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (r + u < re) {
+                        for (int j = 0; j < VEC; ++j) acc[j].add_held_off(Tree::ev(rg, j, c), ro, bo[j]);
+                        return;
+                    }
+                }
+                ColStep<Tree, Acc, VEC>::run(acc, rg, r, c, held);
+                if constexpr (HeldFast<Acc>::value) {
+                    if (held && can32) {
+                        h32 = true;
+#pragma unroll
+                        for (int j = 0; j < VEC; ++j) bo[j] = (u32)(acc[j].idx - rb);
+                    }
+                }
+            };
+            i64 r = rb;
+            for (; r + U <= re; r += U) {
+                RG rg[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
                     i64 off[XTG_KMAX_LEAVES];
                     offsets(r + u, off);
-                    LoadLeavesAt<LS>::template run<VEC>(rg[u], p.leaf, off, inner);
+                    load(rg[u], off);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) step(rg[u], r + u);
+            }
+#pragma unroll 1
+            for (; r < re; ++r) {
+                RG rg;
+                i64 off[XTG_KMAX_LEAVES];
+                offsets(r, off);
+                load(rg, off);
+                step(rg, r);
+            }
+            if constexpr (HeldFast<Acc>::value) {
+                if (h32) {
+#pragma unroll
+                    for (int j = 0; j < VEC; ++j) acc[j].idx = rb + (i64)bo[j];
                 }
             }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (r + u < re) ColStep<Tree, Acc, VEC>::run(acc, rg[u], r + u, c, held);
-            }
-        }
         }
         // flat output index of the first of the VEC outputs
         i64 ofl = 0;
 #pragma unroll
-        for (int d = 0; d < RO; ++d) ofl = ofl * (d == RO - 1 ? p.oshape[d] * VEC : p.oshape[d]) + ko[d];
+        for (int d = 0; d < RO; ++d) ofl = ofl * (d == RO - 1 ? p.inner : p.oshape[d]) + ko[d];
 #pragma unroll
         for (int j = 0; j < VEC; ++j) {
+            if (LSTR && !mine[j]) continue;
+            const int at = LSTR ? 32 * j : j;
             if (p.nsplit > 1) {
-                reinterpret_cast<Acc*>(p.partial)[(ofl + j) * p.nsplit + s] = acc[j];
+                reinterpret_cast<Acc*>(p.partial)[(ofl + at) * p.nsplit + s] = acc[j];
             } else {
                 i64 oo = 0;
 #pragma unroll
                 for (int d = 0; d < RO; ++d) oo += ko[d] * p.ostr[d];
-                oo += (i64)j * p.ostr[RO - 1];
+                oo += (i64)at * p.ostr[RO - 1];
                 reinterpret_cast<Out*>(p.out)[oo] = finish<Out, Acc, POST>(acc[j], p);
             }
         }

@@ -286,18 +286,32 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         for (int d = 0; d < RR; ++d) p.ers[d] = Rd.st[erow][d];
     }
 
+    // Columns whose rows vectors do not divide: lane-strided outputs (LSTR),
+    // two per thread and 8 rows in flight, one for 8-byte elements (200 x 400 x
+    // 1001 along axis 1: argmax float32 127 us through the ring of single
+    // elements, 143 / 87 / 69 / 64 us with 1 x 4, 2 x 4, 2 x 8, 4 x 8; sums of
+    // 256 x 512 x 777 160 us, 78 / 103 / 77 / 93; amax float64 210 us, 158 with
+    // 1 x 8, 171 with 2 x 8)
+    bool lstr = false;
+    if (!row && vec == 1 && n_red > 0 && K.shape[RO - 1] >= 32 && opt("reduce.col_lanes", 1)) {
+        lstr = true;
+        for (int l = 0; l < NL; ++l) lstr = lstr && kinds[l] != 2;
+        if (lstr) vec = maxsz <= 4 ? 2 : 1;
+    }
     p.n_out = n_out;
     p.n_red = n_red;
+    p.inner = K.shape[RO - 1];
     p.rdivisor = 1.0 / p.divisor;
     p.rdivisor2 = 1.0 / p.divisor2;
     p.rn_red = 1.0 / (double)n_red;
     for (int d = 0; d < RO; ++d) p.oshape[d] = K.shape[d];
     for (int d = 0; d < RR; ++d) p.rshape[d] = Rd.shape[d];
     if (row) p.rshape[RR - 1] /= vec;
+    else if (lstr) p.oshape[RO - 1] = (K.shape[RO - 1] + 32 * vec - 1) / (32 * vec) * 32;
     else p.oshape[RO - 1] /= vec;
     for (int d = 0; d < RO; ++d) p.ofd[d] = make_fd((uint64_t)std::max<int64_t>(p.oshape[d], 1));
     for (int d = 0; d < RR; ++d) p.rfd[d] = make_fd((uint64_t)std::max<int64_t>(p.rshape[d], 1));
-    p.n_outv = row ? n_out : n_out / vec;
+    p.n_outv = row ? n_out : n_out / K.shape[RO - 1] * p.oshape[RO - 1];
     p.n_redv = row ? n_red / vec : n_red;
     for (int l = 0; l < NL; ++l) {
         p.leaf[l] = t.leaves[l].data;
@@ -456,13 +470,13 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
             st = launch(k, grid_cap(k, need), 256, &p, stream, 0, part_off);
         }
     } else {
-        const int U = (int)opt("reduce.col_unroll", 4);
-        const int rs = async_stages(t, kinds, NL, vec, "reduce.col_async", "reduce.col_stages");
+        const int U = lstr ? 8 : (int)opt("reduce.col_unroll", 4);
+        const int rs = lstr ? 0 : async_stages(t, kinds, NL, vec, "reduce.col_async", "reduce.col_stages");
         const size_t ring = (size_t)rs * (size_t)NL * 256 * 16;
         std::string name = "xtg::k_reduce_col<" + tree + ", " + ls + ", " + accname + ", " + outc + ", " +
                            std::to_string(post) + ", " + std::to_string(vec) + ", " + std::to_string(RO) + ", " +
                            std::to_string(RR) + ", " + std::to_string(U) + ", " + (big ? "true" : "false") + ", " +
-                           std::to_string(rs) + ">";
+                           std::to_string(rs) + (lstr ? ", true>" : ">");
         st = get_kernel(name, 256, &k, ring);
         if (st == XTG_OK) {
             int64_t need = (p.n_outv * nsplit + 255) / 256;
@@ -471,7 +485,7 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     }
     if (st == XTG_OK && nsplit > 1) {
         xtg::RedParams pc = p;
-        if (!row) pc.oshape[RO - 1] *= vec;  // combine decodes flat element indices
+        if (!row) pc.oshape[RO - 1] = K.shape[RO - 1];  // combine decodes flat element indices
         // few splits: a thread per output merges them in order; many: a CTA
         const bool per_thread = nsplit <= opt("reduce.thread_combine_max", 64);
         std::string name = std::string(per_thread ? "xtg::k_reduce_combine_thread<" : "xtg::k_reduce_combine<") +
