@@ -1722,7 +1722,7 @@ template <class Acc, class Out, int POST, int G> struct LaneFinish {
         if (++n == G) flush(p);
     }
     template <class P> XTG_DI void flush(const P& p) {
-        if (have) reinterpret_cast<Out*>(p.out)[at] = finish<Out, Acc, POST>(kept, p);
+        if (have) Store<Out, Acc, POST>::put(kept, p, at);
         have = false;
         n = 0;
     }
@@ -1809,6 +1809,14 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
                 }
             }
         };
+        // element e of a full reduction of one run (p.tail elements behind the
+        // whole vectors; the last item's first lane takes them)
+        auto tail_load = [&](typename LS::template R<1>::type& rg1, i64 e) {
+            i64 off[XTG_KMAX_LEAVES];
+#pragma unroll
+            for (int l = 0; l < LS::N; ++l) off[l] = kbase[l] + e * p.lrs[l][RR - 1];
+            LoadLeavesAt<LS>::template run<1>(rg1, p.leaf, off, inner);
+        };
 // the reduction pass over the work item, folding into accumulator A
 #define XTG_ROW_PASS(A)                                                                \
     {                                                                                  \
@@ -1845,6 +1853,19 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
             if (r0 + 2 * step < re) load(rga, r0 + 2 * step);                          \
             consume(rgb, r0 + step);                                                   \
         }                                                                              \
+        if (VEC > 1 && p.tail && w == nwork - 1 && gtid == 0)                          \
+            _Pragma("unroll 1") for (int i = 0; i < p.tail; ++i) {                     \
+                const i64 e = p.n_redv * VEC + i;                                      \
+                typename LS::template R<1>::type rg1;                                  \
+                tail_load(rg1, e);                                                     \
+                if constexpr (ES != 0) {                                               \
+                    ET ev[1] = {cvt<ET>(Tree::ev(rg1, 0, c))};                         \
+                    reinterpret_cast<ET*>(p.eout)[ebase + e * p.ers[RR - 1]] = ev[0];  \
+                    AddVec<HasAdd2<decltype(A)>::value != 0>::template run<1, ArrVal>(A, ev, e, c); \
+                } else {                                                               \
+                    AddVec<HasAdd2<decltype(A)>::value != 0>::template run<1, Tree>(A, rg1, e, c); \
+                }                                                                      \
+            }                                                                          \
     }
         bool reduced = false;  // acc already holds the group's result
         if constexpr (FastSel<Acc>::value && ES == 0) {
@@ -1878,6 +1899,13 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
 #pragma unroll
                         for (int j = 0; j < VEC; ++j) acc.add(Tree::ev(rga[0], j, c), r * VEC + j);
                     }
+                if (VEC > 1 && p.tail && w == nwork - 1 && gtid == 0)
+                    for (int i = 0; i < p.tail; ++i) {
+                        const i64 e = p.n_redv * VEC + i;
+                        typename LS::template R<1>::type rg1;
+                        tail_load(rg1, e);
+                        acc.add(Tree::ev(rg1, 0, c), e);
+                    }
             } else if (ex) XTG_ROW_PASS(acc)
             else fa.to(acc);
         } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
@@ -1898,13 +1926,13 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
             fin.take(acc, true, oo, gtid, p);
         } else if (gtid == 0) {
             if (p.nsplit > 1) {
-                static_assert(sizeof(Acc) <= 32, "split partial slots are 32 bytes");
+                static_assert(sizeof(Acc) <= 64, "split partial slots are 32 bytes, 64 for the one-pass moments");
                 reinterpret_cast<Acc*>(p.partial)[w] = acc;
             } else {
                 i64 oo = 0;
 #pragma unroll
                 for (int d = 0; d < RO; ++d) oo += ko[d] * p.ostr[d];
-                reinterpret_cast<Out*>(p.out)[oo] = finish<Out, Acc, POST>(acc, p);
+                Store<Out, Acc, POST>::put(acc, p, oo);
             }
         }
         if (GROUP > 32) __syncthreads();
@@ -2152,6 +2180,7 @@ __global__ void __launch_bounds__(256) k_reduce_combine_thread(const RedParams p
     const Acc* part = reinterpret_cast<const Acc*>(p.partial);
     for (i64 o = (i64)blockIdx.x * blockDim.x + threadIdx.x; o < p.n_out; o += (i64)gridDim.x * blockDim.x) {
         Acc a = part[o * p.nsplit];
+#pragma unroll 8
         for (i64 s = 1; s < p.nsplit; ++s) a.merge(part[o * p.nsplit + s]);
         i64 ko[RO];
         decode_dims<RO, true>(p.oshape, p.ofd, o, ko);
@@ -3914,17 +3943,20 @@ template <int NT> XTG_DI bool bar_or_n(bool v) {
 // gives up when a slot is not released in time, and before it returns it
 // waits (bounded) for its copies still in flight, so the block's shared
 // memory outlives every copy.
-template <class T> struct SmemVec16 {
-    template <int VEC> static XTG_DI void get(T (&dst)[VEC], const unsigned char* p) {
-        union {
-            uint4 q;
-            T e[VEC];
-        } u;
-        u.q = *reinterpret_cast<const uint4*>(p);
+template <class T, int VEC>
+XTG_DI void ld_smem(T (&dst)[VEC], const T* p) {
+    const int B = (int)sizeof(T) * VEC;
+    if (B == 16 || B == 8 || B == 4) {
+        typedef typename VecT<B>::t V;
+        union { V v; T e[VEC]; } u;
+        u.v = *reinterpret_cast<const V*>(p);
 #pragma unroll
         for (int j = 0; j < VEC; ++j) dst[j] = u.e[j];
+    } else {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) dst[j] = p[j];
     }
-};
+}
 // K3's block tree (group_reduce<256>) over the 256 consumer threads.
 template <class A> XTG_DI A consumer_reduce(A a, A* smem) {
 #pragma unroll
@@ -3943,18 +3975,24 @@ template <class A> XTG_DI A consumer_reduce(A a, A* smem) {
     }
     return a;
 }
-template <class Tree, class LS, class TL, class Acc, class Out, int POST, int VEC, int NS>
-__global__ void __launch_bounds__(288) k_reduce_stream(const RedParams p) {
+// Two blocks per SM as the register bound: without one the compiler stopped at
+// 40 registers and spilled (one-pass moments of 2^28 float32 193 us; 196 bound
+// to three blocks, 186 to two).
+template <class Tree, class LS, class TL, class Acc, class Out, int POST, int VEC, bool TAIL, int NS>
+__global__ void __launch_bounds__(288, 2) k_reduce_stream(const RedParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
-    constexpr unsigned SB = 16384;  // stage bytes: 1024 vectors
+    constexpr int VB = VEC * (int)sizeof(TL);       // bytes of a vector
+    constexpr int SV = 16384 / VB;                  // vectors per stage
+    constexpr unsigned SB = VB == 16 ? 16384 : 16384 + 32;  // a slot: with room for the granules at both ends
     constexpr int kPolls = 1 << 22;
     extern __shared__ __align__(128) unsigned char sbuf[];
     __shared__ u64 full[NS], empty[NS];
     __shared__ Acc smem[8];
     const int tid = (int)threadIdx.x;
     const i64 nitems = p.nsplit;
-    const char* base = reinterpret_cast<const char*>(p.leaf[0]);
+    const unsigned char* const base = reinterpret_cast<const unsigned char*>(p.leaf[0]);
+    const unsigned char* const end = base + p.n_redv * VB;
     auto item_len = [&](i64 w) -> i64 {
         const i64 rb = w * p.chunk;
         const i64 re = rb + p.chunk < p.n_redv ? rb + p.chunk : p.n_redv;
@@ -3976,7 +4014,7 @@ __global__ void __launch_bounds__(288) k_reduce_stream(const RedParams p) {
         bool stop = false;
         for (i64 w = blockIdx.x; w < nitems && !stop; w += gridDim.x) {
             const i64 len = item_len(w);
-            for (i64 v0 = 0; v0 < len; v0 += 1024) {
+            for (i64 v0 = 0; v0 < len; v0 += SV) {
                 const int slot = (int)(q % NS);
                 if (q >= NS) {
                     const unsigned par = (unsigned)(((q / NS) - 1) & 1);
@@ -3991,11 +4029,34 @@ __global__ void __launch_bounds__(288) k_reduce_stream(const RedParams p) {
                         break;
                     }
                 }
-                const i64 nv = len - v0 < 1024 ? len - v0 : 1024;
-                const unsigned bytes = (unsigned)(nv * 16);
+                const i64 nv = len - v0 < SV ? len - v0 : SV;
                 if (q >= NS) fence_proxy_async_smem();  // the consumers' reads before the copy's writes
-                mbar_expect_tx(&full[slot], bytes);
-                bulk_g2s(sbuf + (size_t)slot * SB, base + (w * p.chunk + v0) * 16, bytes, &full[slot]);
+                const unsigned char* const a = base + (w * p.chunk + v0) * VB;
+                unsigned char* const d = sbuf + (size_t)slot * SB;
+                if (VB == 16) {
+                    const unsigned bytes = (unsigned)(nv * 16);
+                    mbar_expect_tx(&full[slot], bytes);
+                    bulk_g2s(d, a, bytes, &full[slot]);
+                } else {
+                    // whole granules, the neighbouring elements in the first
+                    // and last included; at the array's own ends by plain loads
+                    const unsigned char* const e = a + nv * VB;
+                    const u64 a16 = (u64)a & ~15ull;
+                    u64 lo = a16, hi = ((u64)e + 15) & ~15ull;
+                    if (a == base && ((u64)a & 15)) {
+                        lo = a16 + 16 < (u64)e ? a16 + 16 : (u64)e;
+                        for (u64 x = (u64)a; x < lo; x += sizeof(TL))
+                            *reinterpret_cast<TL*>(d + (x - a16)) = *reinterpret_cast<const TL*>(x);
+                    }
+                    if (hi > (u64)end) {
+                        hi = (u64)e & ~15ull;
+                        for (u64 x = hi > lo ? hi : lo; x < (u64)e; x += sizeof(TL))
+                            *reinterpret_cast<TL*>(d + (x - a16)) = *reinterpret_cast<const TL*>(x);
+                    }
+                    if (hi < lo) hi = lo;
+                    mbar_expect_tx(&full[slot], (unsigned)(hi - lo));
+                    if (hi > lo) bulk_g2s(d + (lo - a16), (const void*)lo, (unsigned)(hi - lo), &full[slot]);
+                }
                 ++q;
             }
         }
@@ -4031,7 +4092,7 @@ __global__ void __launch_bounds__(288) k_reduce_stream(const RedParams p) {
         typename Work<Acc>::T wa;
         wa.from(acc);
         const i64 len = item_len(w);
-        const i64 ns = (len + 1023) / 1024;
+        const i64 ns = (len + SV - 1) / SV;
         for (i64 s = 0; s < ns; ++s, ++q) {
             const int slot = (int)(q % NS);
             if (!bad) {
@@ -4046,15 +4107,16 @@ __global__ void __launch_bounds__(288) k_reduce_stream(const RedParams p) {
             }
             if (!bad) {
                 const unsigned char* buf = sbuf + (size_t)slot * SB;
-                const i64 nvs = len - s * 1024 < 1024 ? len - s * 1024 : 1024;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                if (VB != 16) buf += (unsigned)((u64)(base + (w * p.chunk + s * SV) * VB) & 15);
+                const i64 nvs = len - s * SV < SV ? len - s * SV : SV;
+#pragma unroll 4
+                for (int j = 0; j < SV / 256; ++j) {
                     const int v = tid + 256 * j;
                     if (v < nvs) {
                         RG rg;
-                        SmemVec16<TL>::template get<VEC>(RegAt<0>::get(rg), buf + (size_t)v * 16);
+                        ld_smem<TL, VEC>(RegAt<0>::get(rg), reinterpret_cast<const TL*>(buf + (size_t)v * VB));
                         AddVec<HasAdd2<typename Work<Acc>::T>::value != 0>::template run<VEC, Tree>(
-                            wa, rg, (w * p.chunk + s * 1024 + v) * VEC, c);
+                            wa, rg, (w * p.chunk + s * SV + v) * VEC, c);
                     }
                 }
             }
@@ -4062,6 +4124,17 @@ __global__ void __launch_bounds__(288) k_reduce_stream(const RedParams p) {
             if (__any_sync(0xffffffffu, bad)) bad = true;
             __syncwarp();
             if (!bad && (tid & 31) == 0) mbar_arrive(&empty[slot]);
+        }
+        if (TAIL && w == nitems - 1 && tid == 0) {
+            // the elements behind the whole vectors (a variant of its own: the
+            // registers of this loop cost the others 3%)
+#pragma unroll 1
+            for (int i = 0; i < p.tail; ++i) {
+                const i64 e = p.n_redv * VEC + i;
+                typename LS::template R<1>::type rg1;
+                RegAt<0>::get(rg1)[0] = reinterpret_cast<const TL*>(base)[e];
+                AddVec<HasAdd2<typename Work<Acc>::T>::value != 0>::template run<1, Tree>(wa, rg1, e, c);
+            }
         }
         wa.to(acc);
         if (bar_or_n<256>(bad)) {
@@ -4078,20 +4151,6 @@ __global__ void __launch_bounds__(288) k_reduce_stream(const RedParams p) {
 }
 
 
-template <class T, int VEC>
-XTG_DI void ld_smem(T (&dst)[VEC], const T* p) {
-    const int B = (int)sizeof(T) * VEC;
-    if (B == 16 || B == 8 || B == 4) {
-        typedef typename VecT<B>::t V;
-        union { V v; T e[VEC]; } u;
-        u.v = *reinterpret_cast<const V*>(p);
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) dst[j] = u.e[j];
-    } else {
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) dst[j] = p[j];
-    }
-}
 template <int I, int VEC, class... S> struct SmemLoad;
 template <int I, int VEC> struct SmemLoad<I, VEC> {
     template <class RG> static XTG_DI void run(RG&, const unsigned char*, const unsigned*, i64) {}

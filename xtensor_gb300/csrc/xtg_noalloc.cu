@@ -148,7 +148,7 @@ extern "C" xtg_status xtg_sum_f32_noalloc(const float* x, int64_t n, float* out,
     // The same plan as xtg_reduce(XTG_RED_SUM, all axes) on a contiguous
     // float32 array: vector width, fixed chunking, warp/CTA groups.
     int vec = 4;
-    while (vec > 1 && ((n % vec) != 0 || ((uintptr_t)x % (uintptr_t)(vec * 4)) != 0)) vec >>= 1;
+    while (vec > 1 && (n < vec || ((uintptr_t)x % (uintptr_t)(vec * 4)) != 0)) vec >>= 1;
     if (n == 0) vec = 1;
     const int64_t nv = n / vec;
     if (nv > 0xFFFFFFF0ll) return fail(XTG_ERR_UNSUPPORTED, "xtg_sum_f32_noalloc: more than 2^32 vectors");
@@ -177,6 +177,7 @@ extern "C" xtg_status xtg_sum_f32_noalloc(const float* x, int64_t n, float* out,
     p.n_outv = 1;
     p.n_red = n;
     p.n_redv = nv;
+    p.tail = (int)(n % vec);
     p.chunk = chunk;
     p.nsplit = nsplit;
     p.leaf[0] = x;
@@ -198,7 +199,7 @@ extern "C" xtg_status xtg_sum_f32_noalloc(const float* x, int64_t n, float* out,
     else group == 256 ? launch_row<1, 256>(p, grid, st) : launch_row<1, 32>(p, grid, st);
     XTG_CUDA(cudaGetLastError());
     count_launch();
-    if (nsplit > 1 && nsplit <= opt("reduce.thread_combine_max", 64)) {
+    if (nsplit > 1 && nsplit <= std::min<int64_t>(8, opt("reduce.thread_combine_max", 64))) {
         XTG_NOALLOC_COMBINE_THREAD<<<1, 256, 0, st>>>(p);
         XTG_CUDA(cudaGetLastError());
         count_launch();

@@ -92,6 +92,7 @@ struct RedParams {
     i64 n_outv;     // output vectors (COL) or outputs (ROW)
     i64 n_red;      // reduced elements per output
     i64 inner;      // outputs along the innermost kept dim
+    int tail;       // full reductions of one run: elements behind the whole vectors
     i64 n_redv;     // reduced vectors (ROW) or elements (COL)
     i64 chunk;      // reduced vectors/elements per split
     i64 nsplit;

@@ -177,9 +177,10 @@ static int kind_of(int64_t s) { return s == 1 ? 0 : (s == 0 ? 1 : 2); }
 // launch, and the caller evaluates in two calls instead.
 static const char* kNotFusable = "fused assign + reduce: not a row reduction plan";
 // One-pass moments (xtg_reduce_moments): the accumulator is xtg::AccStats and
-// `outc` names the xtg::StatsOut of the four result types; only the streaming
-// kernel (K13) takes it — any other plan returns XTG_ERR_UNSUPPORTED before a
-// launch (with *not_fusable set) and the caller runs the four reductions.
+// `outc` names the xtg::StatsOut of the four result types; full reductions by
+// the row strategy or the streaming kernel (K13) take it — any other plan
+// returns XTG_ERR_UNSUPPORTED before a launch (with *not_fusable set) and the
+// caller runs the four reductions.
 struct StatsSpec {
     std::string outc;
     bool has_sum;  // the sum's destination is `out` (else `out` only shapes the plan)
@@ -250,9 +251,13 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     // be, so that the fold matches a later reduction of it
     if (eout) maxsz = std::max(maxsz, dt(eout->dtype).size);
     int vec = 16 / maxsz;
+    // a full reduction of one run takes the elements behind its whole vectors
+    // one by one, so its length does not narrow them (2^28 - 1 bfloat16, all
+    // moments: 391 us by single elements, 125 by vectors)
+    const bool one_run = row && n_out == 1 && RR == 1;
     auto vec_ok = [&](int v) {
         if (v == 1) return true;
-        if (row ? (Rd.shape[RR - 1] % v) : (K.shape[RO - 1] % v)) return false;
+        if (one_run ? Rd.shape[RR - 1] < v : row ? (Rd.shape[RR - 1] % v) : (K.shape[RO - 1] % v)) return false;
         for (int l = 0; l < NL; ++l) {
             if (kinds[l] != 0) continue;
             if (!aligned(t.leaves[l].data, (int64_t)v * dt(t.leaves[l].dtype).size)) return false;
@@ -301,6 +306,7 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     p.n_out = n_out;
     p.n_red = n_red;
     p.inner = K.shape[RO - 1];
+    p.tail = one_run ? (int)(n_red % vec) : 0;
     p.rdivisor = 1.0 / p.divisor;
     p.rdivisor2 = 1.0 / p.divisor2;
     p.rn_red = 1.0 / (double)n_red;
@@ -354,17 +360,17 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     const std::string tree = tree_type(t, t.root, map);
     const std::string outc = stats ? stats->outc : std::string(dt(out_dt).cname);
 
-    // K13: a full reduction of one contiguous leaf in 16-byte vectors with a
-    // double-float accumulator streams through shared memory (the same
-    // vectors, order and tree as K3 with a 256-thread group, so the same bits)
+    // K13: a full reduction of one contiguous leaf with a double-float
+    // accumulator streams through shared memory (the same vectors, order and
+    // tree as K3 with a 256-thread group, so the same bits)
     const bool dfloat = stats || accname == "xtg::AccSumC" || accname.rfind("xtg::AccMom<float", 0) == 0 ||
                         accname.rfind("xtg::AccNormC<", 0) == 0;
     const bool k13 = row && !eout && n_out == 1 && RR == 1 && NL == 1 && kinds[0] == 0 && dfloat &&
-                     opt("reduce.packed", 1) && opt("reduce.stream", 1) && vec * dt(t.leaves[0].dtype).size == 16 &&
-                     aligned(t.leaves[0].data, 16) && chunk >= opt("reduce.cta_chunk", 2048);
-    if (stats && !k13) {
+                     opt("reduce.packed", 1) && opt("reduce.stream", 1) &&
+                     aligned(t.leaves[0].data, dt(t.leaves[0].dtype).size) && chunk >= opt("reduce.cta_chunk", 2048);
+    if (stats && !(row && n_out == 1)) {
         if (not_fusable) *not_fusable = true;
-        return fail(XTG_ERR_UNSUPPORTED, "one-pass moments: not a streaming plan");
+        return fail(XTG_ERR_UNSUPPORTED, "one-pass moments: not a full reduction by rows");
     }
 
     void* part = nullptr;
@@ -388,13 +394,13 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     xtg_status st;
     if (k13) {
         const int NS = (int)std::max<int64_t>(2, std::min<int64_t>(opt("reduce.stream_stages", 4), 6));
-        const size_t smem = (size_t)NS * 16384;
+        const size_t smem = (size_t)NS * (vec * dt(t.leaves[0].dtype).size == 16 ? 16384 : 16384 + 32);
         int* err = nullptr;
         XTG_TRY(device_error_word(&err));
         p.err = err;
         const std::string name = "xtg::k_reduce_stream<" + tree + ", " + ls + ", " + dt(t.leaves[0].dtype).cname + ", " +
                                  accname + ", " + outc + ", " + std::to_string(post) + ", " + std::to_string(vec) + ", " +
-                                 std::to_string(NS) + ">";
+                                 (p.tail ? "true" : "false") + ", " + std::to_string(NS) + ">";
         Kernel* k;
         st = get_kernel(name, 288, &k, smem);  // 8 consumer warps + the producer warp
         if (st == XTG_OK) st = launch(k, grid_cap(k, nsplit), 288, &p, stream, smem, part_off);
@@ -486,8 +492,10 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     if (st == XTG_OK && nsplit > 1) {
         xtg::RedParams pc = p;
         if (!row) pc.oshape[RO - 1] = K.shape[RO - 1];  // combine decodes flat element indices
-        // few splits: a thread per output merges them in order; many: a CTA
-        const bool per_thread = nsplit <= opt("reduce.thread_combine_max", 64);
+        // few splits of many outputs: a thread per output merges them in order;
+        // else a CTA per output (48 splits of one output: 15 us with the
+        // thread's chain, 8 with the CTA)
+        const bool per_thread = nsplit <= opt("reduce.thread_combine_max", 64) && (nsplit <= 8 || n_out >= 8192);
         std::string name = std::string(per_thread ? "xtg::k_reduce_combine_thread<" : "xtg::k_reduce_combine<") +
                            accname + ", " + outc + ", " + std::to_string(post) + ", " + std::to_string(RO) + ">";
         Kernel* kc;
