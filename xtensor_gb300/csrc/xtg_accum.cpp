@@ -327,8 +327,10 @@ xtg_status scan_launch(const Tree& t, int rt, int op, const AccPlan& P, const xt
                                std::to_string(nch) + ">";
     const std::string tail_c = ", " + svs + ", " + std::to_string(ns) + ", " + std::to_string(ipt_c) + ", " +
                                (cs ? "true" : "false") + ", " + std::to_string(nch) + ">";
+    // pass A streams float64 too
+    const size_t ring_a = nch > 1 ? (size_t)xtg::XTG_SCAN_FOLD_STAGES * 8 * 32 * ipt_a * rsz : 0;
     Kernel *ka, *kb, *kc;
-    XTG_TRY(get_kernel("xtg::k_scan_seg_reduce<" + tree + ", " + sls + ", " + rts + ", " + ops + tail_a, 256, &ka));
+    XTG_TRY(get_kernel("xtg::k_scan_seg_reduce<" + tree + ", " + sls + ", " + rts + ", " + ops + tail_a, 256, &ka, ring_a));
     XTG_TRY(get_kernel("xtg::k_scan_seg_apply<" + tree + ", " + sls + ", " + rts + ", " + ops + tail_c, 256, &kc, ring));
     const int64_t unit = 512;
     const int64_t nunits = (len + unit - 1) / unit;
@@ -340,7 +342,7 @@ xtg_status scan_launch(const Tree& t, int rt, int op, const AccPlan& P, const xt
     // pass B stages a row's segment totals in shared memory
     const size_t seg_smem = ((size_t)nseg * 16 + 15) & ~(size_t)15;
     if (seg_smem > 200 * 1024) return fail(XTG_ERR_UNSUPPORTED, "scan: too many segments per row");
-    XTG_TRY(get_kernel("xtg::k_scan_seg_offsets<" + rts + ", " + ops + ">", 256, &kb, seg_smem));
+    XTG_TRY(get_kernel("xtg::k_scan_seg_offsets<" + rts + ", " + ops + ">", 1024, &kb, seg_smem));
     p.ntiles = nunits;
     p.n_inner = (nseg << 32) | seg_units;
     // one scratch block: the segment states, then (CS) one value per lane
@@ -353,8 +355,8 @@ xtg_status scan_launch(const Tree& t, int rt, int op, const AccPlan& P, const xt
     p.agg = agg;
     const int agg_off = (int)offsetof(xtg::ScanParams, agg);
     const int64_t blocks = (n_outer * nseg + 7) / 8;  // eight warps per block
-    xtg_status st = launch(ka, grid_of(ka, blocks), 256, &p, stream, 0, agg_off);
-    if (st == XTG_OK) st = launch(kb, grid_of(kb, n_outer), 256, &p, stream, seg_smem, agg_off);
+    xtg_status st = launch(ka, grid_of(ka, blocks), 256, &p, stream, ring_a, agg_off);
+    if (st == XTG_OK) st = launch(kb, grid_of(kb, n_outer), nseg > 512 ? 1024 : 256, &p, stream, seg_smem, agg_off);
     if (st == XTG_OK) st = launch(kc, grid_of(kc, blocks), 256, &p, stream, ring, agg_off);
     xtg_status fs = scratch_free(agg, stream);
     return st != XTG_OK ? st : fs;

@@ -2632,6 +2632,74 @@ template <int VEC, int IPT> struct ScanWarpBuf {
     static constexpr int n = VEC > 1 ? 1 : 32 * IPT + IPT;
 };
 
+// A warp streams the tiles of [kb, ke) of a plain contiguous row (4- or
+// 8-byte elements, 16-byte aligned) through its ring of NS stages in shared
+// memory with cp.async: the warp copies whole lines, chunk q = m * 32 + lane
+// (16 bytes) into a slot of its owner q / CPL, whose CPL chunks are rotated
+// by its position within 128 bytes, so both the copies and the owners' reads
+// hit distinct banks.  f(v, k0, d, whole): lane's elements, tile, stage; the
+// row's last, partial tile is loaded by its lanes.  extra(t, d): more copies
+// of tile t into its stage behind the 32 x IPT elements.
+template <class RT, int IPT> struct ScanSlots {
+    static constexpr int EPC = 16 / (int)sizeof(RT);  // elements of a chunk
+    static constexpr int CPL = IPT / EPC;             // chunks of a lane
+    static constexpr int SB = 32 * IPT * (int)sizeof(RT);
+    static XTG_DI int lane() { return (int)threadIdx.x & 31; }
+    static XTG_DI int rot(int o) { return (o / (8 / CPL)) % CPL; }
+    // where chunk m * 32 + lane is, and the lane's own chunk m
+    static XTG_DI int line(int m) {
+        const int q = m * 32 + lane(), o = q / CPL;
+        return (o * CPL + (q % CPL + rot(o)) % CPL) * 16;
+    }
+    static XTG_DI int own(int m) { return (lane() * CPL + (m + rot(lane())) % CPL) * 16; }
+};
+template <class RT, int NS, int IPT, int XB, class X, class F>
+XTG_DI void scan_ring(unsigned char* wbase, const RT* src, i64 kb, i64 ke, X&& extra, F&& f) {
+    typedef ScanSlots<RT, IPT> S;
+    constexpr int WT = 32 * IPT;
+    const int lane = S::lane();
+    const i64 T = (ke - kb + WT - 1) / WT;
+    auto issue = [&](i64 t) {
+        const i64 k0 = kb + t * WT;
+        unsigned char* d = wbase + (int)(t % NS) * (S::SB + XB);
+        if (k0 + WT <= ke) {
+#pragma unroll
+            for (int m = 0; m < S::CPL; ++m) cp_async<16>(d + S::line(m), src + k0 + (m * 32 + lane) * S::EPC);
+        }
+        if (t < T) extra(t, d + S::SB);
+        cp_async_commit();
+    };
+#pragma unroll 1
+    for (int j = 0; j < NS - 1; ++j) issue(j);
+    for (i64 t = 0; t < T; ++t) {
+        // the slot of tile t + NS - 1 was read back by every lane
+        __syncwarp();
+        issue(t + NS - 1);
+        cp_async_wait<NS - 1>();
+        __syncwarp();
+        const i64 k0 = kb + t * WT, kt = k0 + (i64)lane * IPT;
+        unsigned char* const d = wbase + (int)(t % NS) * (S::SB + XB);
+        const bool whole = k0 + WT <= ke;
+        RT v[IPT];
+        if (whole) {
+#pragma unroll
+            for (int m = 0; m < S::CPL; ++m) {
+                union {
+                    uint4 q;
+                    RT e[S::EPC];
+                } u;
+                u.q = *reinterpret_cast<const uint4*>(d + S::own(m));
+#pragma unroll
+                for (int j = 0; j < S::EPC; ++j) v[m * S::EPC + j] = u.e[j];
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < IPT; ++i) v[i] = kt + i < ke ? src[kt + i] : RT(0);
+        }
+        f(v, k0, d, whole);
+    }
+}
+
 // Lane totals of pass A kept for pass C: one value per (row, warp tile, lane).
 template <class RT> XTG_DI RT* scan_csum(const ScanParams& p) {
     return reinterpret_cast<RT*>(reinterpret_cast<char*>(p.agg) + p.csum_off);
@@ -2664,8 +2732,9 @@ template <class Tree, class LS, class RT, int OP, int VEC, int IPT, bool CS, int
 __global__ void __launch_bounds__(256) k_scan_seg_reduce(const ScanParams p) {
     pdl_wait();
     typedef ScanState<RT, OP> ST;
-    constexpr int WB = ScanWarpBuf<VEC, IPT>::n, WT = 32 * IPT;
+    constexpr int WB = H > 1 ? 1 : ScanWarpBuf<VEC, IPT>::n, WT = 32 * IPT;
     __shared__ RT wbuf[8 * WB];
+    extern __shared__ __align__(16) unsigned char ring[];
     Ctx<0> c;
     c.scal = p.scal;
     const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
@@ -2679,18 +2748,68 @@ __global__ void __launch_bounds__(256) k_scan_seg_reduce(const ScanParams p) {
         const i64 kb = sg * su * XTG_SCAN_UNIT;
         const i64 ke = kb + su * XTG_SCAN_UNIT < p.len ? kb + su * XTG_SCAN_UNIT : p.len;
         ST s = ST::ident();
-        scan_walk<Tree, LS, RT, VEC, IPT>(p, c, row, kb, ke, wb, [&](RT(&v)[IPT], i64 k0) {
-            // the lane's fold of each tile (what pass C folds), then merged
-            ST hs[H];
-            lane_fold<H>(hs, v, k0 + lofs, ke);
-            if constexpr (CS) {
-                RT* cs = scan_csum<RT>(p) + ((row * tiles_per_row + k0 / WT) * 32 + lane) * H;
+        if constexpr (VEC > 1 && !CS && H == 1) {
+            // Sums and products commute: the lanes take whole lines (16 elements
+            // per lane in a row: half of every sector per load instruction,
+            // 48.9 us on 2^26 float32 against 39.6 at the copy rate)
+            typedef typename LS::template R<VEC>::type RG;
+            auto load = [&](RT(&v)[IPT], i64 k0) {
 #pragma unroll
-                for (int j = 0; j < H; ++j) cs[j] = hs[j].hi;
+                for (int m = 0; m < IPT / VEC; ++m) {
+                    i64 off[XTG_KMAX_LEAVES];
+#pragma unroll
+                    for (int l = 0; l < LS::N; ++l)
+                        off[l] = row * p.lso[l] + (k0 + (m * 32 + lane) * VEC) * p.lsa[l];
+                    RG rg;
+                    LoadLeavesAt<LS>::template run<VEC>(rg, p.leaf, off, p.lsa);
+#pragma unroll
+                    for (int j = 0; j < VEC; ++j) v[m * VEC + j] = cvt<RT>(Tree::ev(rg, j, c));
+                }
+            };
+            auto fold = [&](const RT(&v)[IPT]) {
+                ST h = ST::ident();
+#pragma unroll
+                for (int i = 0; i < IPT; ++i) h.add(v[i]);
+                s.merge(h);
+            };
+            RT va[IPT], vb[IPT];
+            i64 k0 = kb;
+            if (k0 + WT <= ke) load(va, k0);
+            for (; k0 + WT <= ke; k0 += 2 * WT) {
+                const bool two = k0 + 2 * WT <= ke;
+                if (two) load(vb, k0 + WT);
+                fold(va);
+                if (!two) {
+                    k0 += WT;
+                    break;
+                }
+                if (k0 + 3 * WT <= ke) load(va, k0 + 2 * WT);
+                fold(vb);
             }
+            ST h = ST::ident();
+            for (i64 k = k0 + lane; k < ke; k += 32) h.add(scan_elem<Tree, LS, RT>(p, c, row, k));
+            s.merge(h);
+        } else {
+            // the lane's fold of each tile (what pass C folds), then merged
+            auto fold = [&](RT(&v)[IPT], i64 k0) {
+                ST hs[H];
+                lane_fold<H>(hs, v, k0 + lofs, ke);
+                if constexpr (CS) {
+                    RT* cs = scan_csum<RT>(p) + ((row * tiles_per_row + k0 / WT) * 32 + lane) * H;
 #pragma unroll
-            for (int j = 0; j < H; ++j) s.merge(hs[j]);
-        });
+                    for (int j = 0; j < H; ++j) cs[j] = hs[j].hi;
+                }
+#pragma unroll
+                for (int j = 0; j < H; ++j) s.merge(hs[j]);
+            };
+            if constexpr (H > 1)
+                scan_ring<RT, XTG_SCAN_FOLD_STAGES, IPT, 0>(
+                    ring + (size_t)warp * XTG_SCAN_FOLD_STAGES * ScanSlots<RT, IPT>::SB,
+                    reinterpret_cast<const RT*>(p.leaf[0]) + row * p.lso[0], kb, ke, [](i64, unsigned char*) {},
+                    [&](RT(&v)[IPT], i64 k0, unsigned char*, bool) { fold(v, k0); });
+            else
+                scan_walk<Tree, LS, RT, VEC, IPT>(p, c, row, kb, ke, wb, fold);
+        }
         const ST tot = warp_inorder_scan(s);
         if (lane == 31) reinterpret_cast<ST*>(p.agg)[it] = tot;
     }
@@ -2702,27 +2821,29 @@ __global__ void __launch_bounds__(256) k_scan_seg_reduce(const ScanParams p) {
 // flight at once; thread t owns the run of
 // `per` consecutive totals from t * per: it folds them in order, one block
 // scan of the runs' totals gives each run its prefix, and the thread
-// rewrites its run from that prefix.
+// rewrites its run from that prefix.  A chain of dependent merges on one SM:
+// 1024 threads above 512 segments (256 threads: 6.5 us for 4.9K segments).
 template <class RT, int OP>
-__global__ void __launch_bounds__(256) k_scan_seg_offsets(const ScanParams p) {
+__global__ void __launch_bounds__(1024) k_scan_seg_offsets(const ScanParams p) {
     pdl_wait();
     typedef ScanState<RT, OP> ST;
-    __shared__ ST wsum[9];
+    __shared__ ST wsum[33];
     extern __shared__ __align__(16) unsigned char seg_smem[];
     ST* sa = reinterpret_cast<ST*>(seg_smem);
     const i64 nseg = nseg_of(p);
-    const i64 per = (nseg + 255) / 256;
+    const int nt = (int)blockDim.x;
+    const i64 per = (nseg + nt - 1) / nt;
     const i64 b0 = (i64)threadIdx.x * per;
     const i64 b1 = b0 + per < nseg ? b0 + per : nseg;
     for (i64 row = blockIdx.x; row < p.n_outer; row += gridDim.x) {
         ST* a = reinterpret_cast<ST*>(p.agg) + row * nseg;
         if constexpr (sizeof(ST) == 16 || sizeof(ST) == 8 || sizeof(ST) == 4) {
             // every copy in flight at once
-            for (i64 i = threadIdx.x; i < nseg; i += 256) cp_async<(int)sizeof(ST)>(&sa[i], &a[i]);
+            for (i64 i = threadIdx.x; i < nseg; i += nt) cp_async<(int)sizeof(ST)>(&sa[i], &a[i]);
             cp_async_commit();
             cp_async_wait<0>();
         } else {
-            for (i64 i = threadIdx.x; i < nseg; i += 256) sa[i] = a[i];
+            for (i64 i = threadIdx.x; i < nseg; i += nt) sa[i] = a[i];
         }
         __syncthreads();
         ST run = ST::ident();
@@ -2735,7 +2856,7 @@ __global__ void __launch_bounds__(256) k_scan_seg_offsets(const ScanParams p) {
             pre.merge(v);
         }
         __syncthreads();
-        for (i64 i = threadIdx.x; i < nseg; i += 256) a[i] = sa[i];
+        for (i64 i = threadIdx.x; i < nseg; i += nt) a[i] = sa[i];
         __syncthreads();
     }
 }
@@ -2744,15 +2865,16 @@ __global__ void __launch_bounds__(256) k_scan_seg_offsets(const ScanParams p) {
 // registers: 16-byte stores when the lane's elements are whole (VEC > 1:
 // the destination contiguous and aligned — the host checks).  NS > 0 (the
 // operand a plain contiguous array of the accumulation type, 4 or 8 bytes,
-// rows 16-byte aligned): every lane streams its own 16-byte chunks of the
-// next NS - 1 tiles into a per-warp ring in shared memory with cp.async, so
-// tiles are in flight without holding registers; a lane reads back only
-// what it copied itself (visible to it after cp.async.wait_group), so no
-// barrier is involved.  Chunk m of a lane lands in slot (m + rot) mod CPL of
-// the lane's 16-byte slots, rot = the lane's position within its 128 bytes
-// of the stage: the lanes of one 8-lane phase of a 16-byte read hit
-// distinct banks.  Four blocks per SM for 4-byte types with vector access
-// (a register bound of 64, no spill), fewer otherwise.
+// rows 16-byte aligned): tiles come in through scan_ring, so they are in
+// flight without holding registers, and results go back through the lane's
+// slots so that the warp stores whole lines.  With every lane copying and
+// storing its own 64 or 128 bytes the load-store unit bound the pass (65% of
+// L1's rate, MIO throttle): cumsum of 2^26 float32 156 us then, 141 now (119
+// at the copy rate: two reads, one write), int32 157 -> 136, float64 458 ->
+// 352, 2^22 float32 22 -> 17; what is left for floats is the double-float
+// arithmetic.  Two to six stages measure the same.  Four blocks per SM for
+// 4-byte types with vector access (a register bound of 64, no spill), fewer
+// otherwise.
 template <class Tree, class LS, class RT, int OP, int VEC, int NS, int IPT, bool CS, int H>
 __global__ void __launch_bounds__(256, VEC > 1 && sizeof(RT) <= 4 ? 4 : NS > 0 && IPT <= 8 ? 3 : 2)
     k_scan_seg_apply(const ScanParams p) {
@@ -2775,7 +2897,7 @@ __global__ void __launch_bounds__(256, VEC > 1 && sizeof(RT) <= 4 ? 4 : NS > 0 &
         const i64 ke = kb + su * XTG_SCAN_UNIT < p.len ? kb + su * XTG_SCAN_UNIT : p.len;
         ST carry = reinterpret_cast<const ST*>(p.agg)[it];
         RT* o = reinterpret_cast<RT*>(p.out) + row * p.oso;
-        auto tile = [&](RT(&v)[IPT], i64 k0, const RT* csv) {
+        auto tile = [&](RT(&v)[IPT], i64 k0, const RT* csv, bool store) {
             const i64 kt = k0 + lofs;
             // every tile but a row's last is whole: no per-element checks
             const bool full = kt + IPT <= ke;
@@ -2829,7 +2951,9 @@ __global__ void __launch_bounds__(256, VEC > 1 && sizeof(RT) <= 4 ? 4 : NS > 0 &
                     }
                 }
             }
-            if (VEC > 1 && full) {
+            if (!store) {
+                // the caller's
+            } else if (VEC > 1 && full) {
 #pragma unroll
                 for (int m = 0; m < IPT / VEC; ++m) {
                     RT w[VEC > 1 ? VEC : 1];
@@ -2845,64 +2969,45 @@ __global__ void __launch_bounds__(256, VEC > 1 && sizeof(RT) <= 4 ? 4 : NS > 0 &
             carry.merge(tile_tot);
         };
         if constexpr (NS > 0) {
-            constexpr int EPC = 16 / (int)sizeof(RT);        // elements per 16-byte chunk
-            constexpr int CPL = IPT / EPC;                   // chunks per lane
-            constexpr int SB = 32 * IPT * (int)sizeof(RT);   // bytes of a warp tile
             // a stage: the warp tile, then (CS) the 32 lanes' H folds from pass A
-            constexpr int CSB = H * (int)sizeof(RT);
-            constexpr int SBX = SB + (CS ? 32 * CSB : 0);
-            unsigned char* wbase = ring + (size_t)warp * NS * SBX;
-            unsigned char* wr = wbase + (size_t)lane * CPL * 16;
-            const int rot = (lane / (CPL >= 8 ? 1 : 8 / CPL)) % CPL;
-            const RT* src = reinterpret_cast<const RT*>(p.leaf[0]) + row * p.lso[0];
-            const i64 T = (ke - kb + WT - 1) / WT;
-            auto issue = [&](i64 t) {
-                const i64 kt = kb + t * WT + lofs;
-                if (t < T && kt + IPT <= ke) {
-                    unsigned char* d = wr + (int)(t % NS) * SBX;
+            typedef ScanSlots<RT, IPT> S;
+            constexpr int CSB = H * (int)sizeof(RT), XB = CS ? 32 * CSB : 0;
+            scan_ring<RT, NS, IPT, XB>(
+                ring + (size_t)warp * NS * (S::SB + XB), reinterpret_cast<const RT*>(p.leaf[0]) + row * p.lso[0], kb, ke,
+                [&](i64 t, unsigned char* d) {
+                    if (CS)
+                        cp_async<CSB>(d + lane * CSB,
+                                      scan_csum<RT>(p) + ((row * tiles_per_row + (kb + t * WT) / WT) * 32 + lane) * H);
+                },
+                [&](RT(&v)[IPT], i64 k0, unsigned char* d, bool whole) {
+                    RT csv[H];
 #pragma unroll
-                    for (int m = 0; m < CPL; ++m) cp_async<16>(d + ((m + rot) % CPL) * 16, src + kt + m * EPC);
-                }
-                if (CS && t < T)
-                    cp_async<CSB>(wbase + (int)(t % NS) * SBX + SB + lane * CSB,
-                                  scan_csum<RT>(p) + ((row * tiles_per_row + (kb + t * WT) / WT) * 32 + lane) * H);
-                cp_async_commit();
-            };
-#pragma unroll 1
-            for (int j = 0; j < NS - 1; ++j) issue(j);
-            for (i64 t = 0; t < T; ++t) {
-                // the slot of tile t + NS - 1 was read back (into registers
-                // already used) while tile t - 1 was scanned
-                issue(t + NS - 1);
-                cp_async_wait<NS - 1>();
-                const i64 k0 = kb + t * WT, kt = k0 + lofs;
-                RT csv[H];
+                    for (int j = 0; j < H; ++j)
+                        csv[j] = CS ? reinterpret_cast<const RT*>(d + S::SB + lane * CSB)[j] : RT(0);
+                    tile(v, k0, csv, !whole);
+                    if (whole) {
+                        // back through the lane's slots, out in whole lines
 #pragma unroll
-                for (int j = 0; j < H; ++j)
-                    csv[j] = CS ? reinterpret_cast<const RT*>(wbase + (int)(t % NS) * SBX + SB + lane * CSB)[j] : RT(0);
-                RT v[IPT];
-                if (kt + IPT <= ke) {
-                    const unsigned char* d = wr + (int)(t % NS) * SBX;
+                        for (int m = 0; m < S::CPL; ++m) {
+                            union {
+                                uint4 q;
+                                RT e[S::EPC];
+                            } u;
 #pragma unroll
-                    for (int m = 0; m < CPL; ++m) {
-                        union {
-                            uint4 q;
-                            RT e[EPC];
-                        } u;
-                        u.q = *reinterpret_cast<const uint4*>(d + ((m + rot) % CPL) * 16);
+                            for (int j = 0; j < S::EPC; ++j) u.e[j] = v[m * S::EPC + j];
+                            *reinterpret_cast<uint4*>(d + S::own(m)) = u.q;
+                        }
+                        __syncwarp();
 #pragma unroll
-                        for (int j = 0; j < EPC; ++j) v[m * EPC + j] = u.e[j];
+                        for (int m = 0; m < S::CPL; ++m)
+                            *reinterpret_cast<uint4*>(o + k0 + (m * 32 + lane) * S::EPC) =
+                                *reinterpret_cast<const uint4*>(d + S::line(m));
                     }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < IPT; ++i) v[i] = kt + i < ke ? src[kt + i] : RT(0);
-                }
-                tile(v, k0, csv);
-            }
+                });
         } else {
             static_assert(!CS, "lane totals from pass A come with the streamed form");
             scan_walk<Tree, LS, RT, VEC, IPT>(p, c, row, kb, ke, wb,
-                                              [&](RT(&v)[IPT], i64 k0) { tile(v, k0, nullptr); });
+                                              [&](RT(&v)[IPT], i64 k0) { tile(v, k0, nullptr, true); });
         }
     }
 }

@@ -159,6 +159,7 @@ struct RowParams {
 
 // Accumulators (cumsum / cumprod): the expression's iteration space as
 // (outer, axis, inner), each part collapsed to one dimension.
+enum { XTG_SCAN_FOLD_STAGES = 3 };  // the ring of the segmented scan's pass A (float64)
 struct ScanParams {
     i64 n_outer, len, n_inner;
     const void* leaf[XTG_KMAX_LEAVES];
