@@ -235,15 +235,27 @@ xtg_status scan_launch(const Tree& t, int rt, int op, const AccPlan& P, const xt
             return true;
         };
         while (vec > 1 && !vec_ok(vec)) vec >>= 1;
+        // Vectors while 131072 threads have one each (862 per SM), else one
+        // column per thread and more positions in flight the fewer threads
+        // there are (float32, 64 x 512 x 1024 along axis 1: 65536 columns
+        // 43 us with 16 ahead, 67 with 4; 16384 vectors 54 to 69.  8000
+        // columns of 512: 18 us with 32 ahead, 23 with 16.  204800 columns of
+        // 400: 99 us with 4, 113 with 16).  With many threads registers count:
+        // 8-byte types 2 ahead (511511 columns of 61 float64 82 us, 94 with 4,
+        // 88 with none ahead), float32 vectors 8 (30000 x 250: 38.8 us, 40.2
+        // with 4).
+        const int64_t ncol = n_outer * n_inner;
+        while (vec > 1 && ncol / vec < 131072) vec >>= 1;
+        int u = ncol / vec >= 131072 ? (dt(rt).size >= 8 ? 2 : vec > 1 ? 8 : 4) : ncol >= 16384 ? 16 : 32;
+        if (NL > 1) u = std::max(2, NL > 4 ? u / 8 : NL > 2 ? u / 4 : u / 2);  // their registers
         std::vector<int> kinds(NL);
         for (int l = 0; l < NL; ++l) kinds[l] = kind_of_s(p.lsi[l]);
         const int okind = p.osi == 1 ? 0 : 2;
         std::string name = "xtg::k_scan_col<" + tree + ", " + leafset_s(t, kinds) + ", " + rts + ", " + ops + ", " +
-                           std::to_string(vec) + ", " + std::to_string(okind) + ", 4>";
+                           std::to_string(vec) + ", " + std::to_string(okind) + ", " + std::to_string(u) + ">";
         Kernel* k;
-        XTG_TRY(get_kernel(name, 256, &k));
-        const int64_t work = n_outer * (n_inner / vec);
-        return launch(k, grid_of(k, (work + 255) / 256), 256, &p, stream);
+        XTG_TRY(get_kernel(name, 64, &k));
+        return launch(k, grid_of(k, (ncol / vec + 63) / 64), 64, &p, stream);
     }
 
     std::vector<int> kinds(NL, 2);
@@ -273,8 +285,14 @@ xtg_status scan_launch(const Tree& t, int rt, int op, const AccPlan& P, const xt
         const int vb = vec * dt(rt).size;
         const bool raw = opt("scan.async", 1) && NL == 1 && t.nodes[t.root].op == XTG_OP_LEAF &&
                          t.leaves[0].dtype == rt && p.lsa[0] == 1 && (vb == 4 || vb == 8 || vb == 16);
+        // Long single-element rows of one operand, a warp for most SMs: the
+        // next chunk waits in registers (32000 rows of 1001 float64 103 us,
+        // copied 147, float32 63 against 68; 4000 rows 25 against 34 — but
+        // 1000 rows 60 against 55 and 4000 rows of 65 4.9 against 3.7: there
+        // the longer instruction stream of one warp is what counts).
+        const int mode = vec == 1 && NL == 1 && len >= 256 && n_outer >= 4096 ? 2 : raw ? 1 : 0;
         std::string name = "xtg::k_scan_rows<" + tree + ", " + leafset_s(t, rk) + ", " + rts + ", " + ops + ", " +
-                           std::to_string(vec) + ", " + (raw ? "true" : "false") + ">";
+                           std::to_string(vec) + ", " + std::to_string(mode) + ">";
         Kernel* k;
         XTG_TRY(get_kernel(name, 64, &k));
         const int64_t groups = (n_outer + 31) / 32;

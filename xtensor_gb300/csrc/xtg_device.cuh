@@ -2239,11 +2239,18 @@ template <class RT, int OP> struct ScanOp {
 };
 
 // K9a: along a non-innermost axis.  A thread owns VEC adjacent inner
-// positions of one outer index and walks the axis in order (U positions'
-// loads in flight), so every output element is folded in the reference's
-// sequential order.
+// positions of one outer index and walks the axis in order, so every output
+// element is folded in the reference's sequential order.  Few threads have to
+// keep many loads in flight: U positions are loaded while the U before them
+// are folded and stored, without a check per position (a checked chunk made
+// the compiler wait for each load, and FP64 adds that a predicate switches
+// off still take their issue slots).  Four positions, checked, none loaded
+// ahead -> now: 64 x 512 x 1024 along axis 1 float32 106 -> 43 us (40 at the
+// copy rate), float64 180 -> 90 (79); 1000 x 4160 along axis 0 float32 137 ->
+// 25, float64 300 -> 85, which is its chain of 1000 dependent FP64 adds (80
+// ns each).
 template <class Tree, class LS, class RT, int OP, int VEC, int OKIND, int U>
-__global__ void __launch_bounds__(256) k_scan_col(const ScanParams p) {
+__global__ void __launch_bounds__(64) k_scan_col(const ScanParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
     Ctx<0> c;
@@ -2258,35 +2265,62 @@ __global__ void __launch_bounds__(256) k_scan_col(const ScanParams p) {
             off[l] = o * p.lso[l] + iv * VEC * p.lsi[l];
             inner[l] = p.lsi[l];
         }
-        i64 oo = o * p.oso + iv * VEC * p.osi;
+        const i64 oo = o * p.oso + iv * VEC * p.osi;
         RT acc[VEC];
-        for (i64 k0 = 0; k0 < p.len; k0 += U) {
-            RG rg[U];
+        auto load = [&](RG(&rg)[U], i64 k0) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                if (k0 + u < p.len) {
-                    i64 o2[XTG_KMAX_LEAVES];
+                i64 o2[XTG_KMAX_LEAVES];
 #pragma unroll
-                    for (int l = 0; l < LS::N; ++l) o2[l] = off[l] + (i64)u * p.lsa[l];
-                    LoadLeavesAt<LS>::template run<VEC>(rg[u], p.leaf, o2, inner);
-                }
+                for (int l = 0; l < LS::N; ++l) o2[l] = off[l] + (k0 + u) * p.lsa[l];
+                LoadLeavesAt<LS>::template run<VEC>(rg[u], p.leaf, o2, inner);
+            }
+        };
+        auto step = [&](const RG& rg, i64 k) {
+            RT v[VEC];
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) v[j] = acc[j] = ScanOp<RT, OP>::step(acc[j], cvt<RT>(Tree::ev(rg, j, c)));
+            st_out<RT, OKIND, VEC>(reinterpret_cast<RT*>(p.out), oo + k * p.osa, p.osi, v);
+        };
+        auto fold = [&](const RG(&rg)[U], i64 k0) {
+            if (k0 == 0) {
+                RT v[VEC];
+#pragma unroll
+                for (int j = 0; j < VEC; ++j) v[j] = acc[j] = ScanOp<RT, OP>::init(cvt<RT>(Tree::ev(rg[0], j, c)));
+                st_out<RT, OKIND, VEC>(reinterpret_cast<RT*>(p.out), oo, p.osi, v);
+            } else {
+                step(rg[0], k0);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (k0 + u < p.len) {
-                    RT v[VEC];
-#pragma unroll
-                    for (int j = 0; j < VEC; ++j) {
-                        const RT x = cvt<RT>(Tree::ev(rg[u], j, c));
-                        acc[j] = (k0 + u == 0) ? ScanOp<RT, OP>::init(x) : ScanOp<RT, OP>::step(acc[j], x);
-                        v[j] = acc[j];
-                    }
-                    st_out<RT, OKIND, VEC>(reinterpret_cast<RT*>(p.out), oo + (i64)u * p.osa, p.osi, v);
-                }
+            for (int u = 1; u < U; ++u) step(rg[u], k0 + u);
+        };
+        RG ra[U], rb[U];
+        i64 k0 = 0;
+        if (U <= p.len) load(ra, 0);
+        for (; k0 + U <= p.len; k0 += 2 * U) {
+            if (k0 + 2 * U <= p.len) load(rb, k0 + U);
+            fold(ra, k0);
+            if (k0 + 2 * U > p.len) {
+                k0 += U;
+                break;
             }
+            if (k0 + 3 * U <= p.len) load(ra, k0 + 2 * U);
+            fold(rb, k0 + U);
+        }
+        for (; k0 < p.len; ++k0) {
+            i64 o2[XTG_KMAX_LEAVES];
 #pragma unroll
-            for (int l = 0; l < LS::N; ++l) off[l] += (i64)U * p.lsa[l];
-            oo += (i64)U * p.osa;
+            for (int l = 0; l < LS::N; ++l) o2[l] = off[l] + k0 * p.lsa[l];
+            RG rg;
+            LoadLeavesAt<LS>::template run<VEC>(rg, p.leaf, o2, inner);
+            if (k0 == 0) {
+                RT v[VEC];
+#pragma unroll
+                for (int j = 0; j < VEC; ++j) v[j] = acc[j] = ScanOp<RT, OP>::init(cvt<RT>(Tree::ev(rg, j, c)));
+                st_out<RT, OKIND, VEC>(reinterpret_cast<RT*>(p.out), oo, p.osi, v);
+            } else {
+                step(rg, k0);
+            }
         }
     }
 }
@@ -2297,9 +2331,17 @@ __global__ void __launch_bounds__(256) k_scan_col(const ScanParams p) {
 // shared memory, lane i folds row i's elements in order, and the chunk goes
 // back the same way.  Sequential order per row (bit-identical to the
 // reference's fold).  VEC > 1 needs rows whose length and starts are
-// multiples of VEC (the host checks).
-template <class Tree, class LS, class RT, int OP, int VEC, bool RAW = false>
-__global__ void __launch_bounds__(64) k_scan_rows(const ScanParams p) {
+// multiples of VEC (the host checks).  MODE 0: loads into the tile; 1: the
+// operand is the accumulation type, copied into it; 2: the next chunk waits in
+// registers while this one is folded.  A few warps per SM, each through its
+// whole sequence per chunk: what bounds it is the length of that sequence, so
+// whole chunks and whole groups of rows carry no checks and fold 16 elements
+// at a time (two or three stages of copies ahead measure the same as none).
+// 32768 rows of 1024 float64 127 -> 101 us, 31171 of 1001 float32 103 -> 62,
+// float64 170 -> 103; a chain of dependent FP64 adds takes 80 ns each, 1024 of
+// them 82 us.
+template <class Tree, class LS, class RT, int OP, int VEC, int MODE>
+__global__ void __launch_bounds__(64, MODE == 2 ? (sizeof(RT) > 4 ? 6 : 10) : 1) k_scan_rows(const ScanParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
     constexpr int CW = 32 * VEC;        // columns per chunk
@@ -2308,22 +2350,59 @@ __global__ void __launch_bounds__(64) k_scan_rows(const ScanParams p) {
     Ctx<0> c;
     c.scal = p.scal;
     const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
-    RT* tw = tile[warp];
+    RT* const tw = tile[warp];
     const i64 ngroups = (p.n_outer + 31) / 32;
     for (i64 g = (i64)blockIdx.x * 2 + warp; g < ngroups; g += (i64)gridDim.x * 2) {
         const i64 r0 = g * 32;
         RT acc = RT(0);
+        const bool rows = r0 + 32 <= p.n_outer;
+        RG rg[MODE == 2 ? 32 : 1];
+        auto load = [&](i64 c0) {
+            // (MODE 2) a column of every row into registers
+            const i64 q = c0 + lane;
+            i64 o[XTG_KMAX_LEAVES];
+            if (rows && c0 + CW <= p.len) {
+#pragma unroll
+                for (int l = 0; l < LS::N; ++l) o[l] = r0 * p.lso[l] + q * p.lsa[l];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    LoadLeavesAt<LS>::template run<VEC>(rg[MODE == 2 ? i : 0], p.leaf, o, p.lsa);
+#pragma unroll
+                    for (int l = 0; l < LS::N; ++l) o[l] += p.lso[l];
+                }
+            } else if (q < p.len) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    if (r0 + i >= p.n_outer) continue;
+#pragma unroll
+                    for (int l = 0; l < LS::N; ++l) o[l] = (r0 + i) * p.lso[l] + q * p.lsa[l];
+                    LoadLeavesAt<LS>::template run<VEC>(rg[MODE == 2 ? i : 0], p.leaf, o, p.lsa);
+                }
+            }
+        };
+        if constexpr (MODE == 2) {
+            static_assert(VEC == 1, "a lane loads one column of every row");
+            load(0);
+        }
         for (i64 c0 = 0; c0 < p.len; c0 += CW) {
             const i64 col = c0 + (i64)lane * VEC;
-            if constexpr (RAW) {
+            if constexpr (MODE == 2) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) tw[i * RS + lane] = cvt<RT>(Tree::ev(rg[i], 0, c));
+            } else if constexpr (MODE == 1) {
                 // the operand is the accumulation type, contiguous along the
                 // rows: copy it into the tile, every row's vector in flight
-                const RT* src = reinterpret_cast<const RT*>(p.leaf[0]);
-#pragma unroll 8
-                for (int i = 0; i < 32; ++i) {
-                    const i64 r = r0 + i;
-                    if (r < p.n_outer && col < p.len)
-                        cp_async<(int)sizeof(RT) * VEC>(tw + (i64)i * RS + lane * VEC, src + r * p.lso[0] + col);
+                const RT* src = reinterpret_cast<const RT*>(p.leaf[0]) + r0 * p.lso[0] + col;
+                RT* d = tw + lane * VEC;
+                if (col < p.len) {
+                    if (rows) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) cp_async<(int)sizeof(RT) * VEC>(d + i * RS, src + i * p.lso[0]);
+                    } else {
+#pragma unroll 4
+                        for (int i = 0; i < 32; ++i)
+                            if (r0 + i < p.n_outer) cp_async<(int)sizeof(RT) * VEC>(d + i * RS, src + i * p.lso[0]);
+                    }
                 }
                 cp_async_commit();
                 cp_async_wait<0>();
@@ -2345,14 +2424,35 @@ __global__ void __launch_bounds__(64) k_scan_rows(const ScanParams p) {
             }
             }
             __syncwarp();
+            if constexpr (MODE == 2) {
+                if (c0 + CW < p.len) load(c0 + CW);
+            }
             const int lim = (p.len - c0) < CW ? (int)(p.len - c0) : CW;
             typedef typename VecT<(int)sizeof(RT) * VEC>::t VV;  // VEC * sizeof(RT) <= 16
             union VU {
                 VV vv;
                 RT e[VEC];
             };
-            if (r0 + lane < p.n_outer) {
-                RT* row = tw + lane * RS;
+            RT* const row = tw + lane * RS;
+            if (lim == CW) {
+                // a whole chunk (lanes behind the last row fold what is there)
+#pragma unroll
+                for (int k = 0; k < CW; k += 16) {
+                    VU u[16 / VEC];
+#pragma unroll
+                    for (int m = 0; m < 16 / VEC; ++m) u[m].vv = *reinterpret_cast<const VV*>(row + k + m * VEC);
+#pragma unroll
+                    for (int m = 0; m < 16 / VEC; ++m) {
+#pragma unroll
+                        for (int j = 0; j < VEC; ++j) {
+                            if (k + m + j == 0 && c0 == 0) acc = ScanOp<RT, OP>::init(u[0].e[0]);
+                            else acc = ScanOp<RT, OP>::step(acc, u[m].e[j]);
+                            u[m].e[j] = acc;
+                        }
+                        *reinterpret_cast<VV*>(row + k + m * VEC) = u[m].vv;
+                    }
+                }
+            } else if (r0 + lane < p.n_outer) {
                 for (int k = 0; k < lim; k += VEC) {
                     VU u;
                     u.vv = *reinterpret_cast<const VV*>(row + k);
@@ -2365,6 +2465,15 @@ __global__ void __launch_bounds__(64) k_scan_rows(const ScanParams p) {
                 }
             }
             __syncwarp();
+            if (rows && col < p.len) {
+                RT* o = reinterpret_cast<RT*>(p.out) + r0 * p.oso + col * p.osa;
+#pragma unroll
+                for (int i = 0; i < 32; ++i, o += p.oso) {
+                    VU u;
+                    u.vv = *reinterpret_cast<const VV*>(tw + i * RS + lane * VEC);
+                    st_out<RT, K_CONTIG, VEC>(o, 0, p.osa, u.e);
+                }
+            } else
 #pragma unroll 4
             for (int i = 0; i < 32; ++i) {
                 const i64 r = r0 + i;
