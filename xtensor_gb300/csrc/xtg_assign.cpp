@@ -189,17 +189,11 @@ xtg_status assign_tree(const Tree& t, const xtg_array* out, cudaStream_t stream)
             if (l != tl) order.push_back(l);
         std::vector<int> map(NL), kinds(NL, 2);
         for (int i = 0; i < NL; ++i) map[order[i]] = i;
-        // 64-wide tiles for <= 4-byte elements (256 B per warp row access),
-        // 32-wide for 8-byte ones
         const int esz = dt(t.leaves[tl].dtype).size;
-        const int TILE = esz <= 4 ? (int)opt("transpose.tile_small", 64) : 32;
-        const int ROWS = esz <= 4 ? 256 / TILE : 8;
         xtg::TransposeParams p;
         memset(&p, 0, sizeof p);
         p.sa = D.shape[ta];
         p.sb = D.shape[in];
-        p.ntile_a = (p.sa + TILE - 1) / TILE;
-        p.ntile_b = (p.sb + TILE - 1) / TILE;
         int nb = 0;
         int64_t nbatch = 1;
         for (int d = 0; d < RR; ++d) {
@@ -211,7 +205,52 @@ xtg_status assign_tree(const Tree& t, const xtg_array* out, cudaStream_t stream)
             ++nb;
         }
         p.nbd = nb;
+        p.nj = nb ? p.bshape[nb - 1] : 1;
+        // 64 x 64 tiles for <= 4-byte elements (256 B per warp row access), 32
+        // x 32 for 8-byte ones, five blocks per SM for extents of whole lines
+        // (256 x 256 x 1024 {2,1,0} float64 164 us, 175 with six), six else
+        // (255 x 255 x 1001 168 against 179); 32 x 64 where an extent is small
+        // (30000 x 70 x 33 {2,1,0} 201 us, 246 with 32 x 32).
+        const bool narrow = std::min(p.sa, p.sb) <= 128;
+        int TA = esz <= 4 ? (int)opt("transpose.tile_small", 64) : 32, TB = esz <= 4 ? TA : narrow ? 64 : 32, TJ = 1;
+        const int minb = esz <= 4 || narrow ? 4 : p.sa % 16 == 0 && p.sb % 16 == 0 ? 5 : 6;
+        // Extents that leave such tiles mostly empty: as many elements in a
+        // shape (of several planes) that covers less than 0.6 of the padding
+        // (34514 planes of 22 x 36 float32 59 us in 16 x 32 x 8, 102 in 64 x 64;
+        // but 30000 x 70 rows of 33 {2,1,0} 119 in 64 x 64, 153 in 16 x 256:
+        // shorter runs of bytes)
+        auto padded = [&](int a, int b) { return (double)((p.sa + a - 1) / a * a) * (double)((p.sb + b - 1) / b * b); };
+        const int area = TA * TB;
+        double best = 0.6 * padded(TA, TB);
+        for (int a = 16; a <= 64; a *= 2)
+            for (int b = 16; b <= 256; b *= 2) {
+                // one plane, or planes enough to fill the tile
+                if (a * b > area || (a * b < area && (b > 64 || p.nj * a * b < area)) || padded(a, b) > best) continue;
+                best = padded(a, b);
+                TA = a;
+                TB = b;
+                TJ = area / (a * b);
+            }
+        p.ntile_a = (p.sa + TA - 1) / TA;
+        p.ntile_b = (p.sb + TB - 1) / TB;
+        if (TJ > 1) {
+            p.oj = p.obs[nb - 1];
+            p.obs[nb - 1] *= TJ;
+            for (int i = 0; i < NL; ++i) {
+                p.lj[i] = p.lbs[i][nb - 1];
+                p.lbs[i][nb - 1] *= TJ;
+            }
+            nbatch /= p.nj;
+            p.bshape[nb - 1] = (p.nj + TJ - 1) / TJ;
+            nbatch *= p.bshape[nb - 1];
+        }
         p.n_tiles = nbatch * p.ntile_a * p.ntile_b;
+        p.big = p.n_tiles > 0xFFFFFFF0ll;
+        if (!p.big) {
+            p.fda = make_fd((uint64_t)p.ntile_a);
+            p.fdb = make_fd((uint64_t)p.ntile_b);
+            for (int d = 0; d < nb; ++d) p.bfd[d] = make_fd((uint64_t)p.bshape[d]);
+        }
         p.out = out->data;
         p.oa = D.st[0][ta];
         p.ob = D.st[0][in];
@@ -222,11 +261,12 @@ xtg_status assign_tree(const Tree& t, const xtg_array* out, cudaStream_t stream)
         }
         fill_scalars(t, p.scal);
         std::string name = "xtg::k_transpose<" + tree_type(t, t.root, map) + ", " + leafset(t, order, kinds) + ", " +
-                           dt(out_dt).cname + ", " + std::to_string(nb) + ", " + std::to_string(TILE) + ", " +
-                           std::to_string(ROWS) + ">";
+                           dt(out_dt).cname + ", " + std::to_string(nb) + ", " + std::to_string(TA) + ", " +
+                           std::to_string(TB) + ", " + std::to_string(TJ) + ", " +
+                           std::to_string(minb) + ">";
         Kernel* k;
-        XTG_TRY(get_kernel(name, TILE * ROWS, &k));
-        return launch(k, grid_for(k, p.n_tiles), TILE * ROWS, &p, stream);
+        XTG_TRY(get_kernel(name, 256, &k));
+        return launch(k, grid_for(k, p.n_tiles), 256, &p, stream);
     }
 
     // K1

@@ -3481,89 +3481,137 @@ __global__ void __launch_bounds__(256) k_filter_tile(const FilterParams p) {
 // contiguous destination — the case xtensor sends to the scalar
 // stepper_assigner, include/xtensor/core/xassign.hpp:1087, 1341).
 // Dims are in destination order after collapsing; dim B = R-1 is contiguous
-// in the destination, dim A (p.da) is the one along which leaf 0 — the
-// transposed source — is unit-stride.  A TILE x TILE tile goes through shared
-// memory: loads walk A (coalesced for leaf 0), stores walk B (coalesced for
-// the destination).  Other leaves are read directly at (a, b).
-template <class Tree, class LS, class OutT, int NB, int TILE, int ROWS>
-__global__ void __launch_bounds__(TILE * ROWS) k_transpose(const TransposeParams p) {
+// in the destination, dim A is the one along which leaf 0 — the transposed
+// source — is unit-stride.  A tile of TA x TB elements of TJ planes (of the
+// last other dim) goes through shared memory: loads walk A (coalesced for
+// leaf 0), stores walk B (coalesced for the destination).  Other leaves are
+// read directly at (a, b).  The next tile's elements wait in registers while
+// this one is stored: loads and stores taking turns, with 64-bit divisions in
+// between, kept 14 KB in flight per SM (255 x 511 x 1001 float32 {2,1,0} 287
+// us, long-scoreboard and barrier stalls at 51% of DRAM's rate; 192 now,
+// {0,2,1} 276 -> 169, {1,2,0} 263 -> 166; 256 x 512 x 1024 {2,0,1} 178 -> 174,
+// {2,1,0} 173 -> 165).
+template <int N> struct TransposeTile {
+    i64 a0, b0, j0, obo, boff[N];
+    bool full;
+};
+template <class Tree, class LS, class OutT, int NB, int TA, int TB, int TJ, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_transpose(const TransposeParams p) {
     pdl_wait();
     typedef typename LS::template R<1>::type RG;
     typedef typename RG::elem0 T0;
-    __shared__ T0 tile[TILE][TILE + 1];
+    typedef TransposeTile<LS::N> Pos;
+    // a thread's elements; rows of A (loads) and of B (stores) a step covers
+    constexpr int E = TA * TB * TJ / 256, RA = 256 / TA, RB = 256 / TB;
+    static_assert(TB % RA == 0 && TA % RB == 0, "a step stays in its plane");
+    __shared__ T0 tile[TJ * TB * (TA + 1)];
     Ctx<0> c;
     c.scal = p.scal;
-    const int tx = threadIdx.x % TILE, ty = threadIdx.x / TILE;
-    for (i64 t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
-        i64 tb = t % p.ntile_b;
-        i64 rest = t / p.ntile_b;
-        i64 ta = rest % p.ntile_a;
-        i64 bt = rest / p.ntile_a;
-        i64 boff[XTG_KMAX_LEAVES];
-        i64 obo = 0;
+    const int tid = (int)threadIdx.x;
+    const int ax = tid % TA, by = tid / TA, bx = tid % TB, ay = tid / TB;
+    const T0* const src = reinterpret_cast<const T0*>(p.leaf[0]);
+    OutT* const out = reinterpret_cast<OutT*>(p.out);
+    auto decode = [&](i64 t, Pos& q) {
+        i64 tb, ta, bt;
+        if (p.big) {
+            tb = t % p.ntile_b;
+            bt = t / p.ntile_b;
+            ta = bt % p.ntile_a;
+            bt /= p.ntile_a;
+        } else {
+            const u32 r = fdiv((u32)t, p.fdb);
+            tb = (u32)t - r * p.fdb.d;
+            bt = fdiv(r, p.fda);
+            ta = r - (u32)bt * p.fda.d;
+        }
+        q.a0 = ta * TA;
+        q.b0 = tb * TB;
+        q.j0 = 0;
+        q.obo = 0;
 #pragma unroll
-        for (int l = 0; l < LS::N; ++l) boff[l] = 0;
+        for (int l = 0; l < LS::N; ++l) q.boff[l] = 0;
 #pragma unroll
         for (int d = NB - 1; d >= 0; --d) {
-            i64 n = p.bshape[d];
-            i64 q = bt / n;
-            i64 id = bt - q * n;
-            bt = q;
-            obo += id * p.obs[d];
+            const i64 n = p.big ? bt / p.bshape[d] : (i64)fdiv((u32)bt, p.bfd[d]);
+            const i64 id = bt - n * p.bshape[d];
+            bt = n;
+            if (d == NB - 1) q.j0 = id * TJ;
+            q.obo += id * p.obs[d];
 #pragma unroll
-            for (int l = 0; l < LS::N; ++l) boff[l] += id * p.lbs[l][d];
+            for (int l = 0; l < LS::N; ++l) q.boff[l] += id * p.lbs[l][d];
         }
-        const i64 a0 = ta * TILE, b0 = tb * TILE;
-        const T0* src = reinterpret_cast<const T0*>(p.leaf[0]);
-        if (LS::N == 1 && a0 + TILE <= p.sa && b0 + TILE <= p.sb) {
-            // interior tile of a single-leaf tree: no bounds tests, and one
-            // pointer step per element instead of the 64-bit index products
-            const T0* ps = src + boff[0] + (a0 + tx) * p.la[0] + (b0 + ty) * p.lb[0];
-            const i64 sstep = (i64)ROWS * p.lb[0];
+        q.full = q.a0 + TA <= p.sa && q.b0 + TB <= p.sb && (TJ == 1 || q.j0 + TJ <= p.nj);
+    };
+    T0 v[E];
+    auto load = [&](const Pos& q) {
+        const T0* s = src + q.boff[0] + (q.a0 + ax) * p.la[0] + (q.b0 + by) * p.lb[0];
+        const i64 st = (i64)RA * p.lb[0], sj = TJ > 1 ? p.lj[0] - (i64)TB * p.lb[0] : 0;
+        if (q.full) {
 #pragma unroll
-            for (int bb = ty; bb < TILE; bb += ROWS) {
-                tile[bb][tx] = ld1<T0>(ps);
-                ps += sstep;
+            for (int k = 0; k < E; ++k) {
+                v[k] = ld1<T0>(s);
+                s += st;
+                if (TJ > 1 && (k + 1) * RA % TB == 0) s += sj;
             }
-            __syncthreads();
-            OutT* pd = reinterpret_cast<OutT*>(p.out) + obo + (a0 + ty) * p.oa + (b0 + tx) * p.ob;
-            const i64 dstep = (i64)ROWS * p.oa;
+        } else if (q.a0 + ax < p.sa) {
 #pragma unroll
-            for (int aa = ty; aa < TILE; aa += ROWS) {
-                RG rg;
-                rg.v[0] = tile[tx][aa];
-                *pd = cvt<OutT>(Tree::ev(rg, 0, c));
-                pd += dstep;
+            for (int k = 0; k < E; ++k) {
+                if (q.b0 + by + k * RA % TB < p.sb && (TJ == 1 || q.j0 + k * RA / TB < p.nj)) v[k] = ld1<T0>(s);
+                s += st;
+                if (TJ > 1 && (k + 1) * RA % TB == 0) s += sj;
             }
-            __syncthreads();
-            continue;
         }
-        {
-            const i64 a = a0 + tx;
+    };
+    auto put = [&](const Pos& q, int k, OutT* d) {
+        const int aa = ay + k * RB % TA, j = k * RB / TA;
+        RG rg;
+        rg.v[0] = tile[(j * TB + bx) * (TA + 1) + aa];
+        if constexpr (LS::N > 1) {
+            i64 off[XTG_KMAX_LEAVES], inner[XTG_KMAX_LEAVES];
 #pragma unroll
-            for (int bb = ty; bb < TILE; bb += ROWS) {
-                const i64 b = b0 + bb;
-                if (a < p.sa && b < p.sb) tile[bb][tx] = ld1<T0>(src + boff[0] + a * p.la[0] + b * p.lb[0]);
+            for (int l = 0; l < LS::N; ++l) {
+                off[l] = q.boff[l] + (q.a0 + aa) * p.la[l] + (q.b0 + bx) * p.lb[l] + (TJ > 1 ? j * p.lj[l] : 0);
+                inner[l] = 0;
+            }
+            LoadRest<LS>::run(rg, p.leaf, off, inner);
+        }
+        *d = cvt<OutT>(Tree::ev(rg, 0, c));
+    };
+    Pos cur, nxt;
+    i64 t = blockIdx.x;
+    if (t < p.n_tiles) {
+        decode(t, cur);
+        load(cur);
+    }
+    while (t < p.n_tiles) {
+#pragma unroll
+        for (int k = 0; k < E; ++k) tile[(by + k * RA) * (TA + 1) + ax] = v[k];
+        __syncthreads();
+        // the next tile's loads are in flight while this one is stored
+        t += gridDim.x;
+        if (t < p.n_tiles) {
+            decode(t, nxt);
+            load(nxt);
+        }
+        OutT* d = out + cur.obo + (cur.a0 + ay) * p.oa + (cur.b0 + bx) * p.ob;
+        const i64 st = (i64)RB * p.oa, sj = TJ > 1 ? p.oj - (i64)TA * p.oa : 0;
+        if (cur.full) {
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                put(cur, k, d);
+                d += st;
+                if (TJ > 1 && (k + 1) * RB % TA == 0) d += sj;
+            }
+        } else if (cur.b0 + bx < p.sb) {
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                if (cur.a0 + ay + k * RB % TA < p.sa && (TJ == 1 || cur.j0 + k * RB / TA < p.nj)) put(cur, k, d);
+                d += st;
+                if (TJ > 1 && (k + 1) * RB % TA == 0) d += sj;
             }
         }
         __syncthreads();
-        {
-            const i64 b = b0 + tx;
-#pragma unroll
-            for (int aa = ty; aa < TILE; aa += ROWS) {
-                const i64 a = a0 + aa;
-                if (a < p.sa && b < p.sb) {
-                    RG rg;
-                    rg.v[0] = tile[tx][aa];
-                    i64 off[XTG_KMAX_LEAVES], inner[XTG_KMAX_LEAVES];
-#pragma unroll
-                    for (int l = 0; l < LS::N; ++l) { off[l] = boff[l] + a * p.la[l] + b * p.lb[l]; inner[l] = 0; }
-                    LoadRest<LS>::run(rg, p.leaf, off, inner);
-                    reinterpret_cast<OutT*>(p.out)[obo + a * p.oa + b * p.ob] = cvt<OutT>(Tree::ev(rg, 0, c));
-                }
-            }
-        }
-        __syncthreads();
+        cur = nxt;
     }
 }
 

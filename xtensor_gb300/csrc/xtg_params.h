@@ -71,14 +71,18 @@ struct ChunkParams {
 struct TransposeParams {
     i64 sa, sb;            // extents of A and B
     i64 ntile_a, ntile_b;
-    i64 n_tiles;           // nbatch * ntile_a * ntile_b
-    i64 bshape[XTG_KMAX_RANK];  // batch dims (all except A and B), outer first
+    i64 n_tiles;           // batch tiles * ntile_a * ntile_b
+    i64 bshape[XTG_KMAX_RANK];  // batch dims (all except A and B), outer first; the last in tiles of TJ planes
+    FastDiv fda, fdb, bfd[XTG_KMAX_RANK];  // divisors of the tile decode
+    int big;               // n_tiles is beyond 32 bits: 64-bit divisions
     int nbd;
+    i64 nj;                // planes of that dim
     void* out;
     i64 oa, ob;            // destination strides along A, B
-    i64 obs[XTG_KMAX_RANK];     // destination strides over batch dims
+    i64 obs[XTG_KMAX_RANK];     // destination strides over batch dims (of TJ planes for the last)
+    i64 oj;                // destination stride of one plane
     const void* leaf[XTG_KMAX_LEAVES];
-    i64 la[XTG_KMAX_LEAVES], lb[XTG_KMAX_LEAVES];
+    i64 la[XTG_KMAX_LEAVES], lb[XTG_KMAX_LEAVES], lj[XTG_KMAX_LEAVES];
     i64 lbs[XTG_KMAX_LEAVES][XTG_KMAX_RANK];
     Scalars scal;
 };
