@@ -296,9 +296,18 @@ xtg_status assign_tree(const Tree& t, const xtg_array* out, cudaStream_t stream)
     while (vec > 1 && !vec_ok(vec)) vec >>= 1;
     xtg::AssignParams p;
     memset(&p, 0, sizeof p);
+    // Single elements of 4 bytes or less: a thread takes 4 rows of one column,
+    // so it decodes one position for four elements (255 x 511 x 1001 float32
+    // {1,0,2} 288 us with a decode per element, 167; 8-byte elements gain
+    // nothing: 3000 x 300 x 37 float64 86 us against 104)
+    int64_t all = 1;
+    for (int d = 0; d < RR; ++d) all *= d == in ? D.shape[d] / vec : D.shape[d];
+    const bool rows = vec == 1 && maxsz <= 4 && RR >= 2 && D.shape[in - 1] >= 16 && all <= 0xFFFFFFF0ll;
+    const int U = rows ? 4 : (int)opt("assign.unroll", vec * maxsz >= 16 ? 4 : 8);
+    p.rows = rows ? D.shape[in - 1] : 0;
     int64_t nvec = 1;
     for (int d = 0; d < RR; ++d) {
-        p.sp.shape[d] = d == in ? D.shape[d] / vec : D.shape[d];
+        p.sp.shape[d] = d == in ? D.shape[d] / vec : rows && d == in - 1 ? (D.shape[d] + U - 1) / U : D.shape[d];
         nvec *= p.sp.shape[d];
     }
     p.sp.nvec = nvec;
@@ -312,16 +321,17 @@ xtg_status assign_tree(const Tree& t, const xtg_array* out, cudaStream_t stream)
         for (int d = 0; d < RR; ++d) p.leaf_strides[l][d] = D.st[1 + l][d];
     }
     fill_scalars(t, p.scal);
-    const int U = (int)opt("assign.unroll", vec * maxsz >= 16 ? 4 : 8);
     const int block = (int)opt("assign.block", 256);
     std::vector<int> order(NL), map(NL);
     for (int l = 0; l < NL; ++l) order[l] = map[l] = l;
     std::string name = "xtg::k_assign<" + tree_type(t, t.root, map) + ", " + leafset(t, order, kinds) + ", " +
                        dt(out_dt).cname + ", " + std::to_string(okind) + ", " + std::to_string(vec) + ", " +
-                       std::to_string(RR) + ", " + std::to_string(U) + ", " + (big ? "true" : "false") + ">";
+                       std::to_string(RR) + ", " + std::to_string(U) + ", " + (big ? "true" : "false") +
+                       (rows ? ", true>" : ">");
     Kernel* k;
     XTG_TRY(get_kernel(name, block, &k));
-    int64_t need = (nvec + (int64_t)block * U - 1) / ((int64_t)block * U);
+    const int64_t per = rows ? block : (int64_t)block * U;
+    const int64_t need = (nvec + per - 1) / per;
     return launch(k, grid_for(k, need), block, &p, stream);
 }
 

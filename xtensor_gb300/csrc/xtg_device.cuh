@@ -285,6 +285,32 @@ template <class... S> struct LoadLeaves<LeafSet<S...>> {
     }
 };
 
+// Loads of all leaves at explicit offsets (vector along a given inner stride).
+template <int I, int VEC, class... S> struct LoadAt;
+template <int I, int VEC> struct LoadAt<I, VEC> {
+    template <class RG> static XTG_DI void run(RG&, const void* const*, const i64*, const i64*) {}
+};
+template <int I, int VEC, class S0, class... S> struct LoadAt<I, VEC, S0, S...> {
+    template <class RG> static XTG_DI void run(RG& rg, const void* const* ptr, const i64* off, const i64* inner) {
+        typedef typename S0::type T;
+        ld_leaf<T, S0::kind, VEC>(rg.v, reinterpret_cast<const T*>(ptr[I]), off[I], inner[I]);
+        LoadAt<I + 1, VEC, S...>::run(rg.rest, ptr, off, inner);
+    }
+};
+template <class LS> struct LoadLeavesAt;
+template <class... S> struct LoadLeavesAt<LeafSet<S...>> {
+    template <int VEC, class RG> static XTG_DI void run(RG& rg, const void* const* ptr, const i64* off, const i64* inner) {
+        LoadAt<0, VEC, S...>::run(rg, ptr, off, inner);
+    }
+};
+// All leaves but leaf 0 (the transposing kernel fills leaf 0 from shared memory).
+template <class LS> struct LoadRest;
+template <class S0, class... S> struct LoadRest<LeafSet<S0, S...>> {
+    template <class RG> static XTG_DI void run(RG& rg, const void* const* ptr, const i64* off, const i64* inner) {
+        LoadAt<1, 1, S...>::run(rg.rest, ptr, off, inner);
+    }
+};
+
 // ---------------------------------------------------------------------------
 // Evaluation context: scalar immediates plus row statistics (for the fused
 // row kernels).  Nodes evaluate at vector lane j.
@@ -449,12 +475,59 @@ template <class T, class Cd, class A, class B> struct Where {
 // destination and leaf strides.  Grid-stride over vectors of VEC elements;
 // each thread keeps U independent vectors in flight (U * leaves * 16 B of
 // loads outstanding) so that HBM latency is hidden with few CTAs per SM.
-template <class Tree, class LS, class OutT, int OUTKIND, int VEC, int R, int U, bool BIG>
+// ROWS: the U vectors lie along dim R - 2, one decode for all of them (single
+// elements: the index arithmetic was 63% of the issue slots at 40% of DRAM's
+// rate).
+template <class Tree, class LS, class OutT, int OUTKIND, int VEC, int R, int U, bool BIG, bool ROWS = false>
 __global__ void __launch_bounds__(256) k_assign(const AssignParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
     Ctx<0> c;
     c.scal = p.scal;
+    if constexpr (ROWS) {
+        // U rows of dim R - 2 per thread (sp counts that dim in groups of U)
+        static_assert(R >= 2 && !BIG, "groups of rows");
+        i64 inner[XTG_KMAX_LEAVES];
+#pragma unroll
+        for (int l = 0; l < LS::N; ++l) inner[l] = p.leaf_strides[l][R - 1];
+        for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < p.sp.nvec; q += (i64)gridDim.x * blockDim.x) {
+            i64 idx[R];
+            decode<R, VEC, false>(p.sp, q, idx);
+            idx[R - 2] *= U;
+            const i64 left = p.rows - idx[R - 2];
+            i64 off[XTG_KMAX_LEAVES];
+#pragma unroll
+            for (int l = 0; l < LS::N; ++l) off[l] = dot_idx<R>(idx, p.leaf_strides[l]);
+            i64 o = dot_idx<R>(idx, p.out_strides);
+            RG rg[U];
+            auto load = [&](int u) {
+                LoadLeavesAt<LS>::template run<VEC>(rg[u], p.leaf, off, inner);
+#pragma unroll
+                for (int l = 0; l < LS::N; ++l) off[l] += p.leaf_strides[l][R - 2];
+            };
+            auto put = [&](int u) {
+                OutT v[VEC];
+#pragma unroll
+                for (int j = 0; j < VEC; ++j) v[j] = cvt<OutT>(Tree::ev(rg[u], j, c));
+                st_out<OutT, OUTKIND, VEC>(reinterpret_cast<OutT*>(p.out), o, p.out_strides[R - 1], v);
+                o += p.out_strides[R - 2];
+            };
+            if (left >= U) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) load(u);
+#pragma unroll
+                for (int u = 0; u < U; ++u) put(u);
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (u < left) load(u);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (u < left) put(u);
+            }
+        }
+        return;
+    }
     const i64 step = (i64)gridDim.x * blockDim.x * U;
     for (i64 base = (i64)blockIdx.x * blockDim.x * U + threadIdx.x; base < p.sp.nvec; base += step) {
         RG rg[U];
@@ -1619,32 +1692,6 @@ XTG_DI void decode_dims(const i64* shape, const FastDiv* fd, i64 q, i64 (&idx)[R
         idx[0] = qu;
     }
 }
-
-// Loads of all leaves at explicit offsets (vector along a given inner stride).
-template <int I, int VEC, class... S> struct LoadAt;
-template <int I, int VEC> struct LoadAt<I, VEC> {
-    template <class RG> static XTG_DI void run(RG&, const void* const*, const i64*, const i64*) {}
-};
-template <int I, int VEC, class S0, class... S> struct LoadAt<I, VEC, S0, S...> {
-    template <class RG> static XTG_DI void run(RG& rg, const void* const* ptr, const i64* off, const i64* inner) {
-        typedef typename S0::type T;
-        ld_leaf<T, S0::kind, VEC>(rg.v, reinterpret_cast<const T*>(ptr[I]), off[I], inner[I]);
-        LoadAt<I + 1, VEC, S...>::run(rg.rest, ptr, off, inner);
-    }
-};
-template <class LS> struct LoadLeavesAt;
-template <class... S> struct LoadLeavesAt<LeafSet<S...>> {
-    template <int VEC, class RG> static XTG_DI void run(RG& rg, const void* const* ptr, const i64* off, const i64* inner) {
-        LoadAt<0, VEC, S...>::run(rg, ptr, off, inner);
-    }
-};
-// All leaves but leaf 0 (the transposing kernel fills leaf 0 from shared memory).
-template <class LS> struct LoadRest;
-template <class S0, class... S> struct LoadRest<LeafSet<S0, S...>> {
-    template <class RG> static XTG_DI void run(RG& rg, const void* const* ptr, const i64* off, const i64* inner) {
-        LoadAt<1, 1, S...>::run(rg.rest, ptr, off, inner);
-    }
-};
 
 // Asynchronous global -> shared copies of 4, 8 or 16 bytes (cp.async): the
 // copies are in flight without holding registers; a thread's own copies are

@@ -37,6 +37,7 @@ struct AssignParams {
     i64 out_strides[XTG_KMAX_RANK];
     const void* leaf[XTG_KMAX_LEAVES];
     i64 leaf_strides[XTG_KMAX_LEAVES][XTG_KMAX_RANK];
+    i64 rows;  // groups of rows: the extent of dim R - 2
     Scalars scal;
 };
 
