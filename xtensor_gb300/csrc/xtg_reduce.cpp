@@ -413,8 +413,10 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         // with 8 lanes); vectors of rows over 128 bytes take two lanes at
         // least (rows of 64 with one: 68 us, the lanes' vectors fall on the
         // same banks).  Fewer than 4096 warps' worth of rows spread over more
-        // lanes.
-        if (group == 32 && nsplit == 1 && RR == 1 && p.n_redv > 0) {
+        // lanes.  The same where the reduced dims do not collapse (axes 0 and 2
+        // of 20 x 100000 x 7 float32: 47 us with a warp per output, 26 with 4
+        // lanes; rows of two 8-wide chunks 457 against 32).
+        if (group == 32 && nsplit == 1 && (RR == 1 || !eout) && p.n_redv > 0) {
             int g = 1;
             while (g < 32 && n_red * maxsz > (int64_t)g * (vec > 1 && g == 1 ? 128 : 256)) g *= 2;
             while (g < 32 && n_out * g < 4096 * 32 && g < p.n_redv) g *= 2;
@@ -472,7 +474,7 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         st = get_kernel(name, 256, &k);
         if (st == XTG_OK) {
             int64_t items = n_out * nsplit;
-            int64_t need = group == 32 ? (items + 7) / 8 : items;
+            int64_t need = group <= 32 ? (items * group + 255) / 256 : items;
             st = launch(k, grid_cap(k, need), 256, &p, stream, 0, part_off);
         }
     } else {
