@@ -216,18 +216,27 @@ static xtg_status run_chunks(const Tree& t, const std::vector<const xtg_chunked*
     memset(&p, 0, sizeof p);
     p.n_cls = n_cls;
     int64_t total = 0, largest = 0;
+    // four rows per thread for single elements of at most 4 bytes, as in K1
+    for (int c = 0; c < n_cls; ++c) {
+        int64_t n = cls_count[(size_t)c];
+        for (int d = 0; d < R; ++d) n *= d == R - 1 ? cls_ext[(size_t)c][d] / vec : cls_ext[(size_t)c][d];
+        largest = std::max<int64_t>(largest, n);
+    }
+    const bool rows = vec == 1 && maxsz <= 4 && R >= 2 && !pad && G.cs[R - 2] >= 16 && largest <= (int64_t)0xFFFFFFF0ll;
+    const int U = rows ? 4 : vec * maxsz >= 16 ? 4 : 8;
     for (int c = 0; c < n_cls; ++c) {
         xtg::ChunkClass& K = p.cls[c];
         int64_t nvec = 1;
         for (int d = 0; d < R; ++d) {
-            K.sp.shape[d] = d == R - 1 ? cls_ext[(size_t)c][d] / vec : cls_ext[(size_t)c][d];
+            const int64_t ext = cls_ext[(size_t)c][d];
+            K.sp.shape[d] = d == R - 1 ? ext / vec : rows && d == R - 2 ? (ext + U - 1) / U : ext;
             nvec *= K.sp.shape[d];
         }
+        K.rows = rows ? cls_ext[(size_t)c][R - 2] : 0;
         K.sp.nvec = nvec;
         K.first = cls_first[(size_t)c];
         K.count = cls_count[(size_t)c];
         total += nvec * K.count;
-        largest = std::max<int64_t>(largest, nvec * K.count);
     }
     const bool big = largest > (int64_t)0xFFFFFFF0ll;
     if (!big)
@@ -250,17 +259,17 @@ static xtg_status run_chunks(const Tree& t, const std::vector<const xtg_chunked*
         ls_s += std::string("xtg::LeafSpec<") + dt(t.leaves[l].dtype).cname + ", " + std::to_string(kinds[l]) + ">";
     }
     ls_s += ">";
-    const int U = vec * maxsz >= 16 ? 4 : 8;
     const std::string name = "xtg::k_assign_chunks<" + tree_type(t, t.root, map) + ", " + ls_s + ", " +
                              dt(out_dtype).cname + ", " + std::to_string(okind) + ", " + std::to_string(vec) + ", " +
                              std::to_string(R) + ", " + std::to_string(U) + ", " + (big ? "true" : "false") + ", " +
-                             (pad ? "true" : "false") + ">";
+                             (pad ? "true" : "false") + (rows ? ", true>" : ">");
     Kernel* k;
     xtg_status st = get_kernel(name, 256, &k);
     if (st == XTG_OK) {
         DeviceInfo* dev;
         ensure_device(&dev);
-        const int64_t need = (total + 256 * U - 1) / (256 * U);
+        const int64_t per = rows ? 256 : 256 * U;
+        const int64_t need = (total + per - 1) / per;
         const int64_t cap = (int64_t)k->max_blocks_per_sm * dev->sm_count;
         st = launch(k, (unsigned)std::max<int64_t>(1, std::min(need, cap)), 256, &p, stream);
     }

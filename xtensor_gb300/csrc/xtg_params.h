@@ -59,6 +59,7 @@ struct ChunkClass {
     Space sp;          // one chunk of the class, innermost dim in vectors
     FastDiv fdn;       // divisor sp.nvec (32-bit launches)
     i64 first, count;
+    i64 rows;          // groups of rows: the extent of dim R - 2
 };
 struct ChunkParams {
     ChunkClass cls[XTG_KCHUNK_CLS];
