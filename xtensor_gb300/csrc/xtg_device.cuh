@@ -1362,16 +1362,19 @@ template <int M, class X> struct BlockAdd<AccMom2<M>, X> { enum { value = M != 0
 template <class A> struct IsStats2 { enum { value = 0 }; };
 template <> struct IsStats2<AccStats2> { enum { value = 1 }; };
 
+// BW: the width of those blocks; a full reduction in vectors that do not divide
+// its length or address keeps the blocks of the widest that does (1: none, its
+// means and norms stay exact to 2^-50).
 // One vector of tree values into an accumulator: in pairs where it takes
 // them, else element by element; p0 = the first element's position.
-template <bool PAIRS> struct AddVec {
+template <bool PAIRS, int BW = 64> struct AddVec {
     template <int VEC, class Tree, class A, class RG, class C>
     static XTG_DI void run(A& a, const RG& rg, i64 p0, const C& c) {
 #pragma unroll
         for (int j = 0; j < VEC; ++j) a.add(Tree::ev(rg, j, c), p0 + j);
     }
 };
-template <> struct AddVec<true> {
+template <int BW> struct AddVec<true, BW> {
     template <int VEC, class Tree, class A, class RG, class C>
     static XTG_DI void run(A& a, const RG& rg, i64 p0, const C& c) {
         typedef decltype(Tree::ev(rg, 0, c)) X;
@@ -1379,12 +1382,16 @@ template <> struct AddVec<true> {
             run<VEC, Tree>(a.s, rg, p0, c);
             run<VEC, Tree>(a.m, rg, p0, c);
             run<VEC, Tree>(a.q, rg, p0, c);
-        } else if constexpr (BlockAdd<A, X>::value != 0 && VEC > 1) {
-            float2 f[VEC / 2];
+        } else if constexpr (BlockAdd<A, X>::value != 0 && VEC > 1 && BW > 1) {
+            constexpr int W = VEC < BW ? VEC : BW;
 #pragma unroll
-            for (int j = 0; j < VEC / 2; ++j)
-                f[j] = make_float2(cvt<float>(Tree::ev(rg, 2 * j, c)), cvt<float>(Tree::ev(rg, 2 * j + 1, c)));
-            a.template addblk<VEC / 2>(f);
+            for (int k = 0; k < VEC; k += W) {
+                float2 f[W / 2];
+#pragma unroll
+                for (int j = 0; j < W / 2; ++j)
+                    f[j] = make_float2(cvt<float>(Tree::ev(rg, k + 2 * j, c)), cvt<float>(Tree::ev(rg, k + 2 * j + 1, c)));
+                a.template addblk<W / 2>(f);
+            }
         } else if (VEC % 2 == 0) {
 #pragma unroll
             for (int j = 0; j < VEC; j += 2) a.add2(Tree::ev(rg, j, c), Tree::ev(rg, j + 1, c), p0 + j);
@@ -1913,9 +1920,13 @@ template <class Acc, class Out, int POST, int G> struct LaneFinish {
         n = 0;
     }
 };
+// PK: 0 no packed states, 1 packed, 2 + k packed with blocks of 2^k elements.
+// Four blocks per SM for small states over two reduced dims (float64 sums over
+// axes 0 and 2 of 20 x 100000 x 7: 51 us with the compiler's choice of 70
+// registers, 42 with 64).
 template <class Tree, class LS, class Acc, class Out, int POST, int VEC, int RO, int RR, int GROUP, bool BIG, int UR = 4,
           int ES = 0, class ET = float, int PK = 1>
-__global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
+__global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 8 ? 4 : 0) k_reduce_row(const RedParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
     __shared__ Acc smem[32];
@@ -2021,10 +2032,10 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
                         _Pragma("unroll") for (int d = 0; d < RR; ++d) eo += ri[d] * p.ers[d]; \
                         st_out<ET, ES == 1 ? K_CONTIG : 2, VEC>(reinterpret_cast<ET*>(p.eout), eo, \
                                                                  p.ers[RR - 1], ev);   \
-                        AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, ArrVal>( \
+                        AddVec<HasAdd2<decltype(A)>::value != 0, (PK > 1 ? 1 << (PK - 2) : 64)>::template run<VEC, ArrVal>( \
                             A, ev, r * VEC, c);                                        \
                     } else {                                                           \
-                        AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, Tree>( \
+                        AddVec<HasAdd2<decltype(A)>::value != 0, (PK > 1 ? 1 << (PK - 2) : 64)>::template run<VEC, Tree>( \
                             A, rg[u], r * VEC, c);                                     \
                     }                                                                  \
                 }                                                                      \
@@ -2039,7 +2050,7 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
             if (r0 + 2 * step < re) load(rga, r0 + 2 * step);                          \
             consume(rgb, r0 + step);                                                   \
         }                                                                              \
-        if (VEC > 1 && p.tail && w == nwork - 1 && gtid == 0)                          \
+        if ((RR == 1 || GROUP > 32) && VEC > 1 && p.tail && w == nwork - 1 && gtid == 0)                          \
             _Pragma("unroll 1") for (int i = 0; i < p.tail; ++i) {                     \
                 const i64 e = p.n_redv * VEC + i;                                      \
                 typename LS::template R<1>::type rg1;                                  \
@@ -2085,7 +2096,7 @@ __global__ void __launch_bounds__(256) k_reduce_row(const RedParams p) {
 #pragma unroll
                         for (int j = 0; j < VEC; ++j) acc.add(Tree::ev(rga[0], j, c), r * VEC + j);
                     }
-                if (VEC > 1 && p.tail && w == nwork - 1 && gtid == 0)
+                if ((RR == 1 || GROUP > 32) && VEC > 1 && p.tail && w == nwork - 1 && gtid == 0)
                     for (int i = 0; i < p.tail; ++i) {
                         const i64 e = p.n_redv * VEC + i;
                         typename LS::template R<1>::type rg1;
@@ -4453,7 +4464,7 @@ template <class A> XTG_DI A consumer_reduce(A a, A* smem) {
 // Two blocks per SM as the register bound: without one the compiler stopped at
 // 40 registers and spilled (one-pass moments of 2^28 float32 193 us; 196 bound
 // to three blocks, 186 to two).
-template <class Tree, class LS, class TL, class Acc, class Out, int POST, int VEC, bool TAIL, int NS>
+template <class Tree, class LS, class TL, class Acc, class Out, int POST, int VEC, bool TAIL, int NS, int BW = 64>
 __global__ void __launch_bounds__(288, 2) k_reduce_stream(const RedParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
@@ -4590,7 +4601,7 @@ __global__ void __launch_bounds__(288, 2) k_reduce_stream(const RedParams p) {
                     if (v < nvs) {
                         RG rg;
                         ld_smem<TL, VEC>(RegAt<0>::get(rg), reinterpret_cast<const TL*>(buf + (size_t)v * VB));
-                        AddVec<HasAdd2<typename Work<Acc>::T>::value != 0>::template run<VEC, Tree>(
+                        AddVec<HasAdd2<typename Work<Acc>::T>::value != 0, BW>::template run<VEC, Tree>(
                             wa, rg, (w * p.chunk + s * SV + v) * VEC, c);
                     }
                 }

@@ -390,6 +390,11 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     // where a replayed plan patches in its fresh scratch (stream-ordered only)
     const int part_off = (part && !(scratch && scratch->fixed)) ? (int)offsetof(xtg::RedParams, partial) : -1;
 
+    // the widest vectors that divide a full reduction's length and fit its
+    // address: the blocks of its sums (AddVec)
+    int bw = vec;
+    if (one_run)
+        while (bw > 1 && (n_red % bw || (k13 && !aligned(t.leaves[0].data, (int64_t)bw * dt(t.leaves[0].dtype).size)))) bw >>= 1;
     Kernel* k;
     xtg_status st;
     if (k13) {
@@ -400,7 +405,8 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         p.err = err;
         const std::string name = "xtg::k_reduce_stream<" + tree + ", " + ls + ", " + dt(t.leaves[0].dtype).cname + ", " +
                                  accname + ", " + outc + ", " + std::to_string(post) + ", " + std::to_string(vec) + ", " +
-                                 (p.tail ? "true" : "false") + ", " + std::to_string(NS) + ">";
+                                 (p.tail ? "true" : "false") + ", " + std::to_string(NS) +
+                                 (bw < vec ? ", " + std::to_string(bw) + ">" : ">");
         Kernel* k;
         st = get_kernel(name, 288, &k, smem);  // 8 consumer warps + the producer warp
         if (st == XTG_OK) st = launch(k, grid_cap(k, nsplit), 288, &p, stream, smem, part_off);
@@ -469,8 +475,9 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
                            std::to_string(RR) + ", " + std::to_string(group) + ", " + (big ? "true" : "false") + ", " +
                            std::to_string(opt("reduce.row_unroll", 4)) +
                            (es ? ", " + std::to_string(es) + ", " + dt(eout->dtype).cname : std::string()) +
-                           (opt("reduce.packed", 1) ? std::string() :
-                            std::string(es ? "" : ", 0, float") + ", 0") + ">";
+                           (!opt("reduce.packed", 1) ? std::string(es ? "" : ", 0, float") + ", 0" :
+                            bw < vec ? std::string(es ? "" : ", 0, float") + (bw == 1 ? ", 2" : bw == 2 ? ", 3" : ", 4") :
+                            std::string()) + ">";
         st = get_kernel(name, 256, &k);
         if (st == XTG_OK) {
             int64_t items = n_out * nsplit;
@@ -496,8 +503,9 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         if (!row) pc.oshape[RO - 1] = K.shape[RO - 1];  // combine decodes flat element indices
         // few splits of many outputs: a thread per output merges them in order;
         // else a CTA per output (48 splits of one output: 15 us with the
-        // thread's chain, 8 with the CTA)
-        const bool per_thread = nsplit <= opt("reduce.thread_combine_max", 64) && (nsplit <= 8 || n_out >= 8192);
+        // thread's chain, 8 with the CTA; int32 sums of 6960 outputs in 11.9 us
+        // with CTAs, 7.2 with threads)
+        const bool per_thread = nsplit <= opt("reduce.thread_combine_max", 64) && (nsplit <= 8 || n_out >= 1024);
         std::string name = std::string(per_thread ? "xtg::k_reduce_combine_thread<" : "xtg::k_reduce_combine<") +
                            accname + ", " + outc + ", " + std::to_string(post) + ", " + std::to_string(RO) + ">";
         Kernel* kc;
