@@ -420,11 +420,14 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         // least (rows of 64 with one: 68 us, the lanes' vectors fall on the
         // same banks).  Fewer than 4096 warps' worth of rows spread over more
         // lanes.  The same where the reduced dims do not collapse (axes 0 and 2
-        // of 20 x 100000 x 7 float32: 47 us with a warp per output, 26 with 4
-        // lanes; rows of two 8-wide chunks 457 against 32).
+        // of 20 x 100000 x 7 float32: 47 us with a warp per output, 21 with 4
+        // lanes; rows of two 8-wide chunks 457 against 32); half the bytes per
+        // lane where outputs of several dims rule out the streamed units (row
+        // sums of 64 x 256 x 1024 chunks 110 us with 16 lanes, 105 with 32).
         if (group == 32 && nsplit == 1 && (RR == 1 || !eout) && p.n_redv > 0) {
             int g = 1;
-            while (g < 32 && n_red * maxsz > (int64_t)g * (vec > 1 && g == 1 ? 128 : 256)) g *= 2;
+            const int64_t lane_bytes = RO > 1 && RR == 1 ? 128 : 256;
+            while (g < 32 && n_red * maxsz > g * (vec > 1 && g == 1 ? 128 : lane_bytes)) g *= 2;
             while (g < 32 && n_out * g < 4096 * 32 && g < p.n_redv) g *= 2;
             group = g;
             // single-element stores of 16 or 32 rows at once touch as many
