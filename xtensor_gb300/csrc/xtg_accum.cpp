@@ -360,7 +360,7 @@ xtg_status scan_launch(const Tree& t, int rt, int op, const AccPlan& P, const xt
     // pass B stages a row's segment totals in shared memory
     const size_t seg_smem = ((size_t)nseg * 16 + 15) & ~(size_t)15;
     if (seg_smem > 200 * 1024) return fail(XTG_ERR_UNSUPPORTED, "scan: too many segments per row");
-    XTG_TRY(get_kernel("xtg::k_scan_seg_offsets<" + rts + ", " + ops + ">", 1024, &kb, seg_smem));
+    XTG_TRY(get_kernel("xtg::k_scan_seg_offsets<" + rts + ", " + ops + ">", 512, &kb, seg_smem));
     p.ntiles = nunits;
     p.n_inner = (nseg << 32) | seg_units;
     // one scratch block: the segment states, then (CS) one value per lane
@@ -373,8 +373,12 @@ xtg_status scan_launch(const Tree& t, int rt, int op, const AccPlan& P, const xt
     p.agg = agg;
     const int agg_off = (int)offsetof(xtg::ScanParams, agg);
     const int64_t blocks = (n_outer * nseg + 7) / 8;  // eight warps per block
+    // (2^21 float32: 16.3 us in all with 256 threads, 13.6 with 512, 12.9 with
+    // 1024; 2^19: 7.2, 7.1, 7.7; float64, whose levels are FP64 latency: 12.0,
+    // 12.5, 13.5)
+    const int kb_threads = nseg > 512 && rt != XTG_FLOAT64 ? 512 : 256;
     xtg_status st = launch(ka, grid_of(ka, blocks), 256, &p, stream, ring_a, agg_off);
-    if (st == XTG_OK) st = launch(kb, grid_of(kb, n_outer), nseg > 512 ? 1024 : 256, &p, stream, seg_smem, agg_off);
+    if (st == XTG_OK) st = launch(kb, grid_of(kb, n_outer), kb_threads, &p, stream, seg_smem, agg_off);
     if (st == XTG_OK) st = launch(kc, grid_of(kc, blocks), 256, &p, stream, ring, agg_off);
     xtg_status fs = scratch_free(agg, stream);
     return st != XTG_OK ? st : fs;
