@@ -4821,8 +4821,8 @@ __global__ void __launch_bounds__(128, MINB) k_rowfused_tma(const RowParams p) {
             }
         }
         // one decision for everyone who shares the buffer: a lane that gave
-        // up must not leave while the others go on into full shuffles
-        // (this is also the barrier that makes the edge elements visible)
+        // up must not leave while the others go on into full shuffles; the
+        // barrier makes the edge elements visible to them
         if (BLK) done = __syncthreads_and(done) != 0;
         else done = __all_sync(0xffffffffu, done) != 0;
         if (EDGE && !BLK) __syncwarp();
@@ -5030,8 +5030,9 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
                 break;
             }
         }
-        // one decision for the warp (and the barrier behind the ends' stores)
+        // one decision for the warp
         done = __all_sync(0xffffffffu, done) != 0;
+        __syncwarp();  // the ends' stores before the other lanes' reads (a vote does not order them)
         if (!done) {
             // give up: flag it, wait (bounded) for the other slots' copies, leave
             if (lane == 0) {
