@@ -1521,11 +1521,13 @@ template <int MAXOP> struct AccArg<double, MAXOP> {
 };
 
 // The fast pass of an arg-reduction over a row (as AccSelFast for amax /
-// amin): the strict compare and two selects per element, positions as 32-bit
-// offsets, from the type's lowest (highest) value at the lane's first
-// position; equal values keep the smaller position.  A NaN anywhere (it is
-// only ever taken as the very first element) and, for float64 keys, an
-// infinity or a best value of zero ask for the exact pass.
+// amin): the strict compare and two selects per element, from the type's
+// lowest (highest) value at the lane's first position.  Positions are kept
+// modulo 2^32; FastItem makes them offsets from the work item's start (the
+// planner gives an item fewer than 2^32 - 1), so that merge() can let equal
+// values keep the smaller one, and adds the start back.  A NaN anywhere (it is only ever
+// taken as the very first element) and, for float64 keys, an infinity or a
+// best value of zero ask for the exact pass.
 template <class A, int MAXOP> struct AccArgFast {
     A v;
     u32 off;
@@ -1599,12 +1601,22 @@ template <int MAXOP> struct AccArgFast<double, MAXOP> {
     }
 };
 template <class A, int M> struct FastSel<AccArg<A, M>> { enum { value = 1 }; typedef AccArgFast<A, M> F; };
-// The fast pass of a row starts at the lane's first position.
-template <class F> struct FastStart {
-    static XTG_DI void at(F&, u32) {}
+// The fast pass of a work item that starts at position `base`: a lane with
+// elements starts at its first position, its result is rebased, and the item's
+// result gets the start back.
+template <class F> struct FastItem {
+    static XTG_DI void start(F&, i64) {}
+    static XTG_DI void rebase(F&, i64) {}
+    template <class S> static XTG_DI void to(const F& f, S& s, i64) { f.to(s); }
 };
-template <class A, int M> struct FastStart<AccArgFast<A, M>> {
-    static XTG_DI void at(AccArgFast<A, M>& f, u32 first) { f.start_at(first); }
+template <class A, int M> struct FastItem<AccArgFast<A, M>> {
+    typedef AccArgFast<A, M> F;
+    static XTG_DI void start(F& f, i64 first) { f.start_at((u32)first); }
+    static XTG_DI void rebase(F& f, i64 base) { f.off -= (u32)base; }
+    template <class S> static XTG_DI void to(const F& f, S& s, i64 base) {
+        f.to(s);
+        s.idx += base;
+    }
 };
 
 // ---------------------------------------------------------------------------
@@ -2069,15 +2081,17 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
             // amax / amin: a position-free pass, arg-reductions: 32-bit
             // positions; the exact pass only when some thread of the group met
             // a NaN, a zero or (float64) another special value
-            typename FastSel<Acc>::F fa;
+            typedef typename FastSel<Acc>::F F;
+            F fa;
             fa.init(p);
-            if (rb + gtid < re) FastStart<typename FastSel<Acc>::F>::at(fa, (u32)((rb + gtid) * VEC));
+            if (rb + gtid < re) FastItem<F>::start(fa, (rb + gtid) * VEC);
             XTG_ROW_PASS(fa)
+            if (rb + gtid < re) FastItem<F>::rebase(fa, rb * VEC);
             // (a group of a warp that met a NaN: its first lane walks the whole
             // item in order, since a fold with NaNs depends on the order)
             bool ex, seq = false;
             if (GROUP <= 32) {
-                fa = group_reduce<GROUP>(fa, (typename FastSel<Acc>::F*)nullptr);  // the same in every lane
+                fa = group_reduce<GROUP>(fa, (F*)nullptr);  // the same in every lane
                 ex = fa.exact();
                 seq = fa.nan();
             } else {
@@ -2104,7 +2118,7 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
                         acc.add(Tree::ev(rg1, 0, c), e);
                     }
             } else if (ex) XTG_ROW_PASS(acc)
-            else fa.to(acc);
+            else FastItem<F>::to(fa, acc, rb * VEC);
         } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
             // double-float states: two lanes advanced by packed instructions
             typename Work<Acc>::T wa;
@@ -5090,11 +5104,12 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
     }
         bool reduced = false;  // acc already holds the group's result
         if constexpr (FastSel<Acc>::value && ES == 0) {
-            typename FastSel<Acc>::F fa;
+            typedef typename FastSel<Acc>::F F;
+            F fa;
             fa.init(p);
-            if (gl < end) FastStart<typename FastSel<Acc>::F>::at(fa, (u32)(gl * VEC));
+            if (gl < end) FastItem<F>::start(fa, gl * VEC);  // (a row is an item that starts at 0)
             XTG_UNIT_PASS(fa, gl, G)
-            fa = group_reduce<G>(fa, (typename FastSel<Acc>::F*)nullptr);  // the same in every lane
+            fa = group_reduce<G>(fa, (F*)nullptr);  // the same in every lane
             reduced = !fa.exact();
             if (reduced) {
                 fa.to(acc);

@@ -338,6 +338,8 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         // slower: the split combine's launch costs more than the parallelism
         // gains — C0's row sum 8.1 -> 14.3 µs)
         nsplit = std::max<int64_t>(1, std::min<int64_t>((target + n_out - 1) / n_out, p.n_redv / minchunk));
+        // arg-reductions keep an item's positions in 32 bits
+        if (accname.rfind("xtg::AccArg<", 0) == 0) nsplit = std::max<int64_t>(nsplit, (p.n_redv * vec >> 31) + 1);
     } else {
         const int64_t target = opt("reduce.target_threads", 131072);
         const int64_t minchunk = opt("reduce.min_col_chunk", 64);
