@@ -52,6 +52,7 @@ struct xtg_batch {
     int vec = 1;  // reductions: elements per vector load (1: the strided form)
     unsigned mask = 0;     // reductions: leaves that the streamed form could copy in units (0: not streamable)
     int64_t max_cols = 0;  // widest instance
+    int64_t unit_cap = 0;  // reductions: elements of a streamed unit whose slots fit a block's shared memory
     int block = 256;
     size_t smem = 0;
     int64_t tile_elems = 32768;
@@ -70,6 +71,8 @@ namespace {
 std::mutex g_tune_mu;
 
 constexpr int kUnitSlots = 3;  // ring slots of the streamed form
+// what a block can have (227 KiB) less the kernel's own variables
+constexpr int64_t kUnitSmem = 225 * 1024;
 
 std::string tune_dir() {
     const char* d = getenv("XTG_CACHE_DIR");
@@ -204,6 +207,13 @@ xtg_status launch_once(xtg_batch* b, cudaStream_t s) {
     return mark(b, s);
 }
 
+// Tile elements of the form `gl`: a streamed unit has 256 at least (what lies
+// before a tile that is not an instance's first then fills a granule) and as
+// many as its slots have room for.
+int64_t fit_tile(const xtg_batch* b, int gl, int64_t te) {
+    return gl != 0 ? te : std::min(std::max<int64_t>(te, 256), b->unit_cap);
+}
+
 // Launch shape: 256 threads, or (the streamed form) five warps and a ring of
 // slots for units of `te` elements (at least a row).
 void set_shape(xtg_batch* b, const Tree& t, int64_t te) {
@@ -262,6 +272,14 @@ xtg_status plan_kernel(xtg_batch* b, Tree& t, AccChoice& ch, int& gl_default, st
             }
         }
         if (row_bytes > 40 * 1024) b->mask = 0;
+        // a slot has room for 16 elements behind a unit and 31 bytes of each leaf
+        int64_t elem_bytes = 0, n = 0;
+        for (size_t l = 0; l < t.leaves.size(); ++l)
+            if ((b->mask >> l) & 1u) {
+                elem_bytes += dt(t.leaves[l].dtype).size;
+                ++n;
+            }
+        if (n) b->unit_cap = (kUnitSmem / kUnitSlots - 31 * n) / elem_bytes - 16;
         // (the kernel keeps the other leaves' column strides as 32-bit byte counts)
         for (auto& I : b->inst)
             for (size_t l = 0; l < t.leaves.size(); ++l)
@@ -276,6 +294,7 @@ xtg_status plan_kernel(xtg_batch* b, Tree& t, AccChoice& ch, int& gl_default, st
     std::sort(cols.begin(), cols.end());
     std::sort(rows.begin(), rows.end());
     gl_default = (int)opt("batch.group_lanes", -1);
+    if (gl_default == 0 && !b->mask) gl_default = -1;  // nothing to stream
     // the streamed form up to 2^25 elements (it runs at 0.45 of the copy rate
     // but starts at once: 59 instances of up to 312 x 91 float32 91 us before,
     // 4 streamed; 256 of up to 1024 x 512 209 and 83), the warp-tile form
@@ -431,13 +450,14 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
     const int64_t te_cap = std::max<int64_t>(256, b->elements / ((int64_t)dev->sm_count * 16));
     int64_t te = opt("batch.tile_elems", std::min<int64_t>(gl ? 32768 : 4096, te_cap));
     if (gl == 0) te = std::min<int64_t>(te, 8192);
+    te = fit_tile(b, gl, te);
     b->tuned = 0;
     if (autotune && !dry_run()) {
         int tg, tc;
         int64_t tt;
         if (tune_lookup(key, tg, tt, tc) && (tg != 0 || b->mask)) {
             gl = tg;
-            te = tt;
+            te = fit_tile(b, gl, tt);
             cpsm = tc;
             b->tuned = 2;
         } else {
@@ -492,7 +512,8 @@ xtg_status xtg_batch_build(xtg_batch* b, int32_t autotune, xtg_stream stream) {
                 return XTG_OK;
             };
             if (b->mask)
-                for (int64_t tcand : {512, 1024, 2048, 4096}) XTG_TRY(try_cand(0, tcand, 4));
+                for (int64_t tcand : {512, 1024, 2048, 4096})
+                    if (tcand <= b->unit_cap) XTG_TRY(try_cand(0, tcand, 4));
             for (int64_t tcand : tes)
                 for (int gcand : gls)
                     for (int ccand : cps) XTG_TRY(try_cand(gcand, tcand, ccand));
