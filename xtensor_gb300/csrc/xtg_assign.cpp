@@ -511,10 +511,31 @@ static xtg_status assign_rowfused(const Tree& t, const xtg_array& out, int R, co
             if ((D.st[1 + l][d] * sz) % 16) edge = true;
         if (n_rows > 1 && (D.R != 1 || D.st[1 + l][0] != row_len)) tgroup = std::max(tgroup, 32);
     }
-    // A block per row above 8 KiB: a warp's lanes would hold over 64 registers
-    // of the row each, and a buffer per warp leave few warps resident (60000
-    // float64 rows of 2048: 648 us with a warp, 455 with a block).
-    if (tgroup == 256) tgroup = row_bytes > 8192 ? 128 : 32;
+    // A block of 128 per row above 8 KiB or 96 elements per lane of a warp: a
+    // warp's lanes would hold over 64 registers of the row each, and a buffer
+    // per warp leave few warps resident (60000 float64 rows of 2048: 648 us
+    // with a warp, 455 with a block; 2^27 int8 elements in rows of 8192: 946
+    // and 326; 2^26 bfloat16 in rows of 2049, 72 per lane: 80 and 127).  Plain
+    // loads by 256 lanes where 128 would hold over 288 registers, integers
+    // below 4 bytes beside their converted values and bfloat16 packed (three
+    // float64 operands in rows of 6000, 288: 197 us with 128 lanes, 205; of
+    // 8192, 384: 209, 160; uint8 rows of 16384, 256: 799, 1021; of 32768, 512:
+    // 1886, 1129), and for whole vectors of 4 bytes up to 48 elements of a lane,
+    // whose lines they fetch as well (2^26 float32 in rows of 8192: 97 us with
+    // 128 lanes, 85; of 4096: 99, 95; of 16384 less their maximum: 91, 128).
+    auto lane_elems = [&](int g) { return (nvec + g - 1) / g * vec; };
+    int64_t regs128 = 0;
+    for (int l = 0; l < NL; ++l) {
+        const DTypeInfo& T = dt(t.leaves[l].dtype);
+        const int bytes = T.size >= 4 || (T.is_float && vec > 1) ? T.size : T.is_float ? 4 : 8;
+        regs128 += lane_elems(128) * bytes / 4;
+    }
+    if (group == 256) {
+        tgroup = row_bytes > 8192 || lane_elems(32) > 96 ? 128 : 32;
+        if (tgroup == 128 && (regs128 > 288 || (maxsz == 4 && !edge && lane_elems(256) <= 48))) tma = false;
+    } else if (tgroup == 32 && lane_elems(32) > 96) {
+        tgroup = 128;
+    }
     // rows of any alignment that one wave of warps takes at once: there is no
     // next unit to copy meanwhile, and plain loads start sooner (4490 x 51
     // float32: 3.4 us copied, 3.1 loaded)
@@ -537,11 +558,14 @@ static xtg_status assign_rowfused(const Tree& t, const xtg_array& out, int R, co
     // share of the row takes at most 64 registers (float64 rows of 1024: 376
     // us per 2^27 elements with 96 registers; 388 at 4 blocks, 422 at 3,
     // 519 uncapped with two buffers — the compiler then spends ~210
-    // registers; 6 blocks spill).
+    // registers; 6 blocks spill).  An element counts a register at least (2^26
+    // bfloat16 in rows of 16384, 128 per lane: 123 us at 5 blocks, 84 at 2;
+    // rows of 3001: 100, 85 at 3).
     int tnf = 0;
     const int tnv = lane_vecs(tgroup, tnf);
-    int64_t row_regs = 0;
-    for (int l = 0; l < NL; ++l) row_regs += (int64_t)tnv * vec * dt(t.leaves[l].dtype).size / 4;
+    int64_t elem_bytes = 0;
+    for (int l = 0; l < NL; ++l) elem_bytes += dt(t.leaves[l].dtype).size;
+    const int64_t row_regs = (int64_t)tnv * vec * std::max<int64_t>(4, elem_bytes) / 4;
     int64_t minb_auto = row_regs <= 64 ? 5 : (row_regs <= 96 ? 3 : 2);
     // short rows: more units in flight (float64 rows of 64: 233 us at 5, 223 at 8)
     if (tgroup < 32 && row_regs <= 32) minb_auto = 8;
