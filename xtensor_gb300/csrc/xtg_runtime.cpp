@@ -84,6 +84,21 @@ const DTypeInfo& dt(int d) { return kDT[valid_dtype(d) ? d : 0]; }
 static std::mutex g_dev_mu;
 static DeviceInfo g_dev;
 static CUcontext g_ctx = nullptr;
+static int* g_err_word = nullptr;
+
+// Scratch comes from a stream-ordered pool of the library's own that keeps up
+// to scratch.keep_mib (64) of freed memory for the next call; the rest goes
+// back to the device at the next synchronisation.  (The device's default pool
+// keeps nothing: a full reduction after a synchronisation waited 180 us for
+// its few kilobytes.)  Allocation and free are ordered by their streams, so
+// calls on several streams and threads share the pool safely.
+static std::atomic<cudaMemPool_t> g_pool{nullptr};
+
+static xtg_status set_pool_keep(int64_t mib) {
+    uint64_t keep = (uint64_t)std::max<int64_t>(0, mib) << 20;
+    if (cudaMemPool_t pool = g_pool.load()) XTG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    return XTG_OK;
+}
 
 static xtg_status init_locked(int device) {
     int n = 0;
@@ -99,6 +114,23 @@ static xtg_status init_locked(int device) {
     if (!g_ctx) return fail(XTG_ERR_CUDA, "no current CUDA context after runtime init");
     cudaDeviceProp pr;
     XTG_CUDA(cudaGetDeviceProperties(&pr, device));
+    // here and not at first use, which a stream that is being captured does
+    // not allow
+    if (!g_pool.load()) {
+        cudaMemPoolProps mp;
+        memset(&mp, 0, sizeof mp);
+        mp.allocType = cudaMemAllocationTypePinned;
+        mp.location.type = cudaMemLocationTypeDevice;
+        mp.location.id = device;
+        cudaMemPool_t pool;
+        XTG_CUDA(cudaMemPoolCreate(&pool, &mp));
+        g_pool.store(pool);
+        XTG_TRY(set_pool_keep(opt("scratch.keep_mib", 64)));
+    }
+    if (!g_err_word) {
+        XTG_CUDA(cudaMalloc((void**)&g_err_word, 256));
+        XTG_CUDA(cudaMemset(g_err_word, 0, 256));
+    }
     g_dev.device = device;
     g_dev.sm_count = pr.multiProcessorCount;
     g_dev.cc_major = pr.major;
@@ -158,33 +190,6 @@ const HotOpts& hot_opts() {
     return h;
 }
 
-// Scratch comes from a stream-ordered pool of the library's own that keeps up
-// to scratch.keep_mib (64) of freed memory for the next call; the rest goes
-// back to the device at the next synchronisation.  (The device's default pool
-// keeps nothing: a full reduction after a synchronisation waited 180 us for
-// its few kilobytes.)  Allocation and free are ordered by their streams, so
-// calls on several streams and threads share the pool safely.
-static std::mutex g_pool_mu;
-static std::atomic<cudaMemPool_t> g_pool{nullptr};
-
-static xtg_status scratch_pool(cudaMemPool_t* pool) {
-    if ((*pool = g_pool.load(std::memory_order_acquire))) return XTG_OK;
-    DeviceInfo* dev;
-    XTG_TRY(ensure_device(&dev));
-    std::lock_guard<std::mutex> lk(g_pool_mu);
-    if ((*pool = g_pool.load(std::memory_order_acquire))) return XTG_OK;
-    cudaMemPoolProps pr;
-    memset(&pr, 0, sizeof pr);
-    pr.allocType = cudaMemAllocationTypePinned;
-    pr.location.type = cudaMemLocationTypeDevice;
-    pr.location.id = dev->device;
-    XTG_CUDA(cudaMemPoolCreate(pool, &pr));
-    uint64_t keep = (uint64_t)std::max<int64_t>(0, opt("scratch.keep_mib", 64)) << 20;
-    XTG_CUDA(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    g_pool.store(*pool, std::memory_order_release);
-    return XTG_OK;
-}
-
 xtg_status scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
     if (bytes == 0) bytes = 16;
     if (Recorder* rec = recorder()) {
@@ -195,23 +200,17 @@ xtg_status scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
         *p = (void*)(uintptr_t)0x7f0000000000ull;
         return XTG_OK;
     }
-    cudaMemPool_t pool;
-    XTG_TRY(scratch_pool(&pool));
-    XTG_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, s));
+    if (!g_pool.load(std::memory_order_acquire)) XTG_TRY(ensure_device(nullptr));
+    XTG_CUDA(cudaMallocFromPoolAsync(p, bytes, g_pool.load(std::memory_order_acquire), s));
     return XTG_OK;
 }
-static int* g_err_word = nullptr;
 
 xtg_status device_error_word(int** p) {
     if (dry_run()) {
         *p = (int*)(uintptr_t)0x7e0000000000ull;
         return XTG_OK;
     }
-    std::lock_guard<std::mutex> lk(g_dev_mu);
-    if (!g_err_word) {
-        XTG_CUDA(cudaMalloc((void**)&g_err_word, 256));
-        XTG_CUDA(cudaMemset(g_err_word, 0, 256));
-    }
+    XTG_TRY(ensure_device(nullptr));
     *p = g_err_word;
     return XTG_OK;
 }
@@ -421,11 +420,13 @@ xtg_status xtg_stream_wait_event(xtg_stream stream, xtg_event ev) {
 
 xtg_status xtg_set_option(const char* key, int64_t value) {
     if (!key) return fail(XTG_ERR_INVALID, "null key");
-    std::lock_guard<std::mutex> lk(g_opt_mu);
-    if (value < 0) g_opts.erase(key);
-    else g_opts[key] = value;
-    g_opt_gen.fetch_add(1);
-    return XTG_OK;
+    {
+        std::lock_guard<std::mutex> lk(g_opt_mu);
+        if (value < 0) g_opts.erase(key);
+        else g_opts[key] = value;
+        g_opt_gen.fetch_add(1);
+    }
+    return strcmp(key, "scratch.keep_mib") ? XTG_OK : set_pool_keep(value < 0 ? 64 : value);
 }
 
 xtg_status xtg_get_option(const char* key, int64_t* value) {
