@@ -1563,7 +1563,7 @@ template <class A, int MAXOP> struct AccArgFast {
     XTG_DI bool exact() const { return odd; }
     XTG_DI void to(AccArg<A, MAXOP>& s) const {
         s.v = v;
-        s.idx = off;
+        s.idx = off == 0xffffffffu ? -1 : (i64)off;  // a lane without elements holds nothing
     }
 };
 template <int MAXOP> struct AccArgFast<double, MAXOP> {
@@ -1597,7 +1597,7 @@ template <int MAXOP> struct AccArgFast<double, MAXOP> {
     XTG_DI bool exact() const { return mh >= 0x7ff00000u || kv == 0 || kv == -1; }
     XTG_DI void to(AccArg<double, MAXOP>& s) const {
         s.kv = kv;
-        s.idx = off;
+        s.idx = off == 0xffffffffu ? -1 : (i64)off;  // (its key would be a NaN's)
     }
 };
 template <class A, int M> struct FastSel<AccArg<A, M>> { enum { value = 1 }; typedef AccArgFast<A, M> F; };
@@ -1615,7 +1615,7 @@ template <class A, int M> struct FastItem<AccArgFast<A, M>> {
     static XTG_DI void rebase(F& f, i64 base) { f.off -= (u32)base; }
     template <class S> static XTG_DI void to(const F& f, S& s, i64 base) {
         f.to(s);
-        s.idx += base;
+        if (s.idx >= 0) s.idx += base;
     }
 };
 
