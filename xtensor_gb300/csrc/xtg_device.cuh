@@ -1067,12 +1067,14 @@ template <int MAXOP> struct AccSelFast<float, MAXOP> {
     }
 };
 // double: the key order is the IEEE order except for NaNs and for -0 / +0,
-// so the pass keeps the largest high word magnitude (an infinity or NaN
-// anywhere asks for the exact pass) and asks for it too when the best key is
-// a zero's (0: +0, -1: -0), where the fold's last-visited rule decides.
+// so the pass keeps the largest high word magnitude, one more where the low
+// word is not zero: above an infinity's there is a NaN, which asks for the
+// exact pass, as does a best key that is a zero's (0: +0, -1: -0), where the
+// fold's last-visited rule decides.
+XTG_DI unsigned f64_mag_up(i64 b) { return ((unsigned)(b >> 32) & 0x7fffffffu) + ((unsigned)b != 0u ? 1u : 0u); }
 template <int MAXOP> struct AccSelFast<double, MAXOP> {
     i64 kv;
-    unsigned mh;  // largest (high word & 0x7fffffff) seen
+    unsigned mh;  // largest f64_mag_up seen
     bool odd;
     template <class P> XTG_DI void init(const P& p) {
         AccSel<double, MAXOP> s;
@@ -1083,7 +1085,7 @@ template <int MAXOP> struct AccSelFast<double, MAXOP> {
     }
     template <class X> XTG_DI void add(X x, i64) {
         const i64 b = __double_as_longlong(cvt<double>(x));
-        const unsigned h = (unsigned)(b >> 32) & 0x7fffffffu;
+        const unsigned h = f64_mag_up(b);
         mh = mh > h ? mh : h;
         const i64 ka = key64(b);
         if (MAXOP ? (ka >= kv) : (ka <= kv)) kv = ka;
@@ -1093,8 +1095,8 @@ template <int MAXOP> struct AccSelFast<double, MAXOP> {
         odd |= o.odd;
         if (MAXOP ? (o.kv >= kv) : (o.kv <= kv)) kv = o.kv;
     }
-    XTG_DI bool nan() const { return mh >= 0x7ff00000u; }  // (or an infinity)
-    XTG_DI bool exact() const { return odd || mh >= 0x7ff00000u || kv == 0 || kv == -1; }
+    XTG_DI bool nan() const { return mh > 0x7ff00000u; }
+    XTG_DI bool exact() const { return odd || nan() || kv == 0 || kv == -1; }
     XTG_DI void to(AccSel<double, MAXOP>& s) const {
         s.kv = kv;
         s.pos = -1;
@@ -1102,6 +1104,36 @@ template <int MAXOP> struct AccSelFast<double, MAXOP> {
 };
 template <class A> struct FastSel { enum { value = 0 }; typedef A F; };
 template <class A, int M> struct FastSel<AccSel<A, M>> { enum { value = 1 }; typedef AccSelFast<A, M> F; };
+// The passes over a work item that has a NaN.  The fold drops what lies before
+// a NaN (what follows replaces it), so the result is the fold of the elements
+// from the last NaN on, in which the positions stand for the order again: one
+// pass finds that NaN, one folds from there on, from the type's end (float32
+// amax, 2^27 elements with a NaN per row, rows of 1024 / 4096: one lane that
+// walks a row in order 453 / 1829 us, this 143 / 188, rows without NaNs 80 / 79).
+XTG_DI bool is_nan(double x) { return f64_isnan_bits(__double_as_longlong(x)); }
+template <class A> XTG_DI bool is_nan(A x) { return IsFloat<A>::value && !(x == x); }
+template <class S> struct LastNan;
+template <class A, int MAXOP> struct LastNan<AccSel<A, MAXOP>> {
+    i64 p;
+    template <class X> XTG_DI void add(X x, i64 ps) {
+        if (is_nan(cvt<A>(x))) p = ps;
+    }
+    XTG_DI void merge(const LastNan& o) { p = p > o.p ? p : o.p; }
+};
+template <class S> struct AccSelFrom;
+template <class A, int MAXOP> struct AccSelFrom<AccSel<A, MAXOP>> {
+    AccSel<A, MAXOP> s;
+    i64 from;
+    XTG_DI void begin(i64 first) {
+        from = first;
+        s.start(cvt<A>(MAXOP ? -__int_as_float(0x7f800000) : __int_as_float(0x7f800000)));
+    }
+    template <class X> XTG_DI void add(X x, i64 ps) {
+        if (ps >= from) s.add(cvt<A>(x), ps);
+    }
+};
+template <class S> struct IsSel { enum { value = 0 }; };
+template <class A, int M> struct IsSel<AccSel<A, M>> { enum { value = 1 }; };
 
 // Moments for mean / variance / stddev.  Data are shifted by k (the first
 // element of the output's reduction set), then sum(d) and sum(d*d) are
@@ -1525,23 +1557,25 @@ template <int MAXOP> struct AccArg<double, MAXOP> {
 // lowest (highest) value at the lane's first position.  Positions are kept
 // modulo 2^32; FastItem makes them offsets from the work item's start (the
 // planner gives an item fewer than 2^32 - 1), so that merge() can let equal
-// values keep the smaller one, and adds the start back.  A NaN anywhere (it is only ever
-// taken as the very first element) and, for float64 keys, an infinity or a
-// best value of zero ask for the exact pass.
+// values keep the smaller one, and adds the start back.  A NaN is passed over,
+// unless it is the row's very first element, which nothing then beats (first:
+// looked at behind the pass).  The exact pass is left to items whose best value
+// is the one the lanes start from while they have a NaN (its position could be
+// the NaN's) and to float64 zeros, whose two keys are one value.
 template <class A, int MAXOP> struct AccArgFast {
     A v;
     u32 off;
-    bool odd;
+    bool odd, first;
     template <class P> XTG_DI void init(const P&) {
         v = ends();
         off = 0xffffffffu;
-        odd = false;
+        odd = first = false;
     }
     static XTG_DI A ends() {  // what nothing but a NaN is below (above)
         if constexpr (IsFloat<A>::value) return MAXOP ? A(-__int_as_float(0x7f800000)) : A(__int_as_float(0x7f800000));
         else return MAXOP ? Lim<A>::lowest() : Lim<A>::maxv();
     }
-    XTG_DI void start_at(u32 first) { off = first; }
+    XTG_DI void start_at(u32 at) { off = at; }
     template <class X> XTG_DI void add(X x, i64 ps) {
         const A a = cvt<A>(x);
         if (IsFloat<A>::value) odd |= !(a == a);
@@ -1552,6 +1586,7 @@ template <class A, int MAXOP> struct AccArgFast {
     }
     XTG_DI void merge(const AccArgFast& o) {
         odd |= o.odd;
+        first |= o.first;
         const bool better = MAXOP ? Cmp<A>::gt(o.v, v) : Cmp<A>::lt(o.v, v);
         const bool worse = MAXOP ? Cmp<A>::gt(v, o.v) : Cmp<A>::lt(v, o.v);
         if (better || (!worse && o.off < off)) {
@@ -1559,45 +1594,56 @@ template <class A, int MAXOP> struct AccArgFast {
             off = o.off;
         }
     }
-    XTG_DI bool nan() const { return false; }  // the exact pass does not depend on the order
-    XTG_DI bool exact() const { return odd; }
+    XTG_DI bool any_nan() const { return odd; }
+    XTG_DI bool nan() const { return false; }  // no pass here depends on the order
+    XTG_DI bool exact() const { return IsFloat<A>::value && odd && !first && v == ends(); }
     XTG_DI void to(AccArg<A, MAXOP>& s) const {
         s.v = v;
         s.idx = off == 0xffffffffu ? -1 : (i64)off;  // a lane without elements holds nothing
+        if (IsFloat<A>::value && first) {
+            s.v = cvt<A>(__int_as_float(0x7fffffff));
+            s.idx = 0;
+        }
     }
 };
 template <int MAXOP> struct AccArgFast<double, MAXOP> {
     i64 kv;
     u32 off;
-    unsigned mh;  // largest (high word & 0x7fffffff) seen
+    unsigned mh;  // largest f64_mag_up seen
+    bool first;
     template <class P> XTG_DI void init(const P&) {
         kv = MAXOP ? XTG_KEY_MIN : XTG_KEY_MAX;
         off = 0xffffffffu;
         mh = 0;
+        first = false;
     }
-    XTG_DI void start_at(u32 first) { off = first; }
+    XTG_DI void start_at(u32 at) { off = at; }
     template <class X> XTG_DI void add(X x, i64 ps) {
         const i64 b = __double_as_longlong(cvt<double>(x));
-        const unsigned h = (unsigned)(b >> 32) & 0x7fffffffu;
+        const unsigned h = f64_mag_up(b);
         mh = mh > h ? mh : h;
         const i64 ka = key64(b);
-        if (MAXOP ? (ka > kv) : (ka < kv)) {
+        if (h <= 0x7ff00000u && (MAXOP ? (ka > kv) : (ka < kv))) {
             kv = ka;
             off = (u32)ps;
         }
     }
     XTG_DI void merge(const AccArgFast& o) {
         mh = mh > o.mh ? mh : o.mh;
+        first |= o.first;
         if ((MAXOP ? (o.kv > kv) : (o.kv < kv)) || (o.kv == kv && o.off < off)) {
             kv = o.kv;
             off = o.off;
         }
     }
+    XTG_DI bool any_nan() const { return mh > 0x7ff00000u; }
     XTG_DI bool nan() const { return false; }
-    XTG_DI bool exact() const { return mh >= 0x7ff00000u || kv == 0 || kv == -1; }
+    XTG_DI bool exact() const {
+        return !first && ((any_nan() && kv == (MAXOP ? XTG_KEY_MIN : XTG_KEY_MAX)) || kv == 0 || kv == -1);
+    }
     XTG_DI void to(AccArg<double, MAXOP>& s) const {
-        s.kv = kv;
-        s.idx = off == 0xffffffffu ? -1 : (i64)off;  // (its key would be a NaN's)
+        s.kv = first ? (MAXOP ? XTG_KEY_MAX : XTG_KEY_MIN) : kv;
+        s.idx = first ? 0 : off == 0xffffffffu ? -1 : (i64)off;  // (its key would be a NaN's)
     }
 };
 template <class A, int M> struct FastSel<AccArg<A, M>> { enum { value = 1 }; typedef AccArgFast<A, M> F; };
@@ -1605,12 +1651,14 @@ template <class A, int M> struct FastSel<AccArg<A, M>> { enum { value = 1 }; typ
 // elements starts at its first position, its result is rebased, and the item's
 // result gets the start back.
 template <class F> struct FastItem {
+    enum { arg = 0 };
     static XTG_DI void start(F&, i64) {}
     static XTG_DI void rebase(F&, i64) {}
     template <class S> static XTG_DI void to(const F& f, S& s, i64) { f.to(s); }
 };
 template <class A, int M> struct FastItem<AccArgFast<A, M>> {
     typedef AccArgFast<A, M> F;
+    enum { arg = 1 };
     static XTG_DI void start(F& f, i64 first) { f.start_at((u32)first); }
     static XTG_DI void rebase(F& f, i64 base) { f.off -= (u32)base; }
     template <class S> static XTG_DI void to(const F& f, S& s, i64 base) {
@@ -2079,46 +2127,44 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
         bool reduced = false;  // acc already holds the group's result
         if constexpr (FastSel<Acc>::value && ES == 0) {
             // amax / amin: a position-free pass, arg-reductions: 32-bit
-            // positions; the exact pass only when some thread of the group met
-            // a NaN, a zero or (float64) another special value
+            // positions; the exact pass only for what that pass cannot tell
+            // (a NaN, a zero: the accumulators say)
             typedef typename FastSel<Acc>::F F;
             F fa;
             fa.init(p);
             if (rb + gtid < re) FastItem<F>::start(fa, (rb + gtid) * VEC);
             XTG_ROW_PASS(fa)
             if (rb + gtid < re) FastItem<F>::rebase(fa, rb * VEC);
-            // (a group of a warp that met a NaN: its first lane walks the whole
-            // item in order, since a fold with NaNs depends on the order)
-            bool ex, seq = false;
+            if constexpr (FastItem<F>::arg) {
+                if (rb + gtid == 0 && fa.any_nan()) {
+                    typename LS::template R<1>::type rg1;
+                    tail_load(rg1, 0);
+                    fa.first = is_nan(Tree::ev(rg1, 0, c));
+                }
+            }
+            bool ex, nan = false;
             if (GROUP <= 32) {
                 fa = group_reduce<GROUP>(fa, (F*)nullptr);  // the same in every lane
                 ex = fa.exact();
-                seq = fa.nan();
+                nan = fa.nan();
             } else {
                 ex = __syncthreads_or(fa.exact()) != 0;
             }
             reduced = GROUP <= 32 && !ex;
-            if (seq) {
-                if (gtid == 0)
-                    for (i64 r = rb; r < re; ++r) {
-                        i64 ri[RR];
-                        decode_dims<RR, BIG>(p.rshape, p.rfd, r, ri);
-                        ri[RR - 1] *= VEC;
-                        i64 off[XTG_KMAX_LEAVES];
-                        red_offsets<LS::N, RO, RR>(p, ko, ri, off);
-                        LoadLeavesAt<LS>::template run<VEC>(rga[0], p.leaf, off, inner);
-#pragma unroll
-                        for (int j = 0; j < VEC; ++j) acc.add(Tree::ev(rga[0], j, c), r * VEC + j);
-                    }
-                if ((RR == 1 || GROUP > 32) && VEC > 1 && p.tail && w == nwork - 1 && gtid == 0)
-                    for (int i = 0; i < p.tail; ++i) {
-                        const i64 e = p.n_redv * VEC + i;
-                        typename LS::template R<1>::type rg1;
-                        tail_load(rg1, e);
-                        acc.add(Tree::ev(rg1, 0, c), e);
-                    }
-            } else if (ex) XTG_ROW_PASS(acc)
-            else FastItem<F>::to(fa, acc, rb * VEC);
+            if (nan) {
+                if constexpr (GROUP <= 32 && IsSel<Acc>::value) {
+                    LastNan<Acc> last{-1};
+                    XTG_ROW_PASS(last)
+                    AccSelFrom<Acc> rest;
+                    rest.begin(group_reduce<GROUP>(last, (LastNan<Acc>*)nullptr).p);
+                    XTG_ROW_PASS(rest)
+                    acc = rest.s;
+                }
+            } else if (ex) {
+                XTG_ROW_PASS(acc)
+            } else {
+                FastItem<F>::to(fa, acc, rb * VEC);
+            }
         } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
             // double-float states: two lanes advanced by packed instructions
             typename Work<Acc>::T wa;
@@ -5082,21 +5128,21 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
             AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, Tree>(A, V, (i64)e, c); \
         }                                                                              \
     }
-// The pass over the row's vectors S, S + T, S + 2 T, ..., folding into A:
+// The pass over the row's vectors gl, gl + G, gl + 2 G, ..., folding into A:
 // batches of four that lie inside the row for every lane, then one by one
 // (a batch under predicates would issue its FP64 work for absent vectors too:
 // float64 sums of 130-element rows 223 us, 128-element rows 142).
-#define XTG_UNIT_PASS(A, S, T)                                                         \
+#define XTG_UNIT_PASS(A)                                                               \
     {                                                                                  \
-        int r0 = (S);                                                                  \
-        const int whole = end / ((T) * 4) * ((T) * 4);                                 \
-        for (; r0 < whole; r0 += (T) * 4) {                                            \
+        int r0 = gl;                                                                   \
+        const int whole = end / (G * 4) * (G * 4);                                     \
+        for (; r0 < whole; r0 += G * 4) {                                              \
             RG rg[4];                                                                  \
             _Pragma("unroll") for (int u = 0; u < 4; ++u)                              \
-                UnitLoads<LS>::template run<VEC, MASK>(rg[u], buf, loff, p, kb, (r0 + u * (T)) * VEC); \
-            _Pragma("unroll") for (int u = 0; u < 4; ++u) XTG_UNIT_ADD(A, rg[u], r0 + u * (T)) \
+                UnitLoads<LS>::template run<VEC, MASK>(rg[u], buf, loff, p, kb, (r0 + u * G) * VEC); \
+            _Pragma("unroll") for (int u = 0; u < 4; ++u) XTG_UNIT_ADD(A, rg[u], r0 + u * G) \
         }                                                                              \
-        _Pragma("unroll 1") for (; r0 < end; r0 += (T)) {                              \
+        _Pragma("unroll 1") for (; r0 < end; r0 += G) {                                \
             RG rg;                                                                     \
             UnitLoads<LS>::template run<VEC, MASK>(rg, buf, loff, p, kb, r0 * VEC);    \
             XTG_UNIT_ADD(A, rg, r0)                                                    \
@@ -5108,25 +5154,37 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
             F fa;
             fa.init(p);
             if (gl < end) FastItem<F>::start(fa, gl * VEC);  // (a row is an item that starts at 0)
-            XTG_UNIT_PASS(fa, gl, G)
+            XTG_UNIT_PASS(fa)
+            if constexpr (FastItem<F>::arg) {
+                if (gl == 0 && fa.any_nan()) {
+                    typename LS::template R<1>::type rg1;
+                    UnitLoads<LS>::template run<1, MASK>(rg1, buf, loff, p, kb, 0);
+                    fa.first = is_nan(Tree::ev(rg1, 0, c));
+                }
+            }
             fa = group_reduce<G>(fa, (F*)nullptr);  // the same in every lane
             reduced = !fa.exact();
             if (reduced) {
                 fa.to(acc);
-            } else if (!fa.nan()) {
-                XTG_UNIT_PASS(acc, gl, G)
-            } else if (gl == 0) {
-                // a row with a NaN: the group's first lane walks it in order
-                // (a fold with NaNs depends on the order)
-                XTG_UNIT_PASS(acc, 0, 1)
+            } else if (fa.nan()) {
+                if constexpr (IsSel<Acc>::value) {
+                    LastNan<Acc> last{-1};
+                    XTG_UNIT_PASS(last)
+                    AccSelFrom<Acc> rest;
+                    rest.begin(group_reduce<G>(last, (LastNan<Acc>*)nullptr).p);
+                    XTG_UNIT_PASS(rest)
+                    acc = rest.s;
+                }
+            } else {
+                XTG_UNIT_PASS(acc)
             }
         } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
             typename Work<Acc>::T wa;
             wa.from(acc);
-            XTG_UNIT_PASS(wa, gl, G)
+            XTG_UNIT_PASS(wa)
             wa.to(acc);
         } else {
-            XTG_UNIT_PASS(acc, gl, G)
+            XTG_UNIT_PASS(acc)
         }
 #undef XTG_UNIT_PASS
 #undef XTG_UNIT_ADD
