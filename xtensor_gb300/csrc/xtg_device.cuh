@@ -1434,6 +1434,122 @@ template <int BW> struct AddVec<true, BW> {
     }
 };
 
+// Working forms of the float64 sums for the lanes of a narrow group, which fold
+// up to 32 elements of a row each where a whole warp's would fold a few: a batch
+// of four vectors is summed as a tree and the batches go to two sums in turn,
+// vectors behind the last batch to a third; the squared deviations of the
+// moments, one fma each, go to four chains instead.  The rounding error of a
+// row stays what a warp's lanes make of it (rms over random rows, in one chain
+// per lane / so: 64 elements 1.53 / 1.00 of the warp's, 128 1.35 / 1.00, 255
+// 1.17 / 1.00, 63 1.60 / 1.04) for two additions per lane and row, five for the
+// moments (2^27 elements in rows of 64: sums 280 -> 296 us, variances 821 -> 851).
+// A lane that has its row to itself folds under 32 elements in order.
+template <int N> struct Tree64 {
+    static XTG_DI double sum(const double* v) { return Tree64<N / 2>::sum(v) + Tree64<N - N / 2>::sum(v + N / 2); }
+};
+template <> struct Tree64<1> {
+    static XTG_DI double sum(const double* v) { return v[0]; }
+};
+struct Sum64 {
+    double e, o, t;
+    XTG_DI void from(double s) {
+        e = s;
+        o = t = 0.0;
+    }
+    XTG_DI double total() const { return (e + t) + o; }
+    template <int N> XTG_DI void batch(const double (&v)[N]) {
+        const double x = e + Tree64<N>::sum(v);
+        e = o;
+        o = x;
+    }
+    template <int N> XTG_DI void rest(const double (&v)[N]) { t += Tree64<N>::sum(v); }
+};
+template <class A> struct Batch64 { enum { value = 0 }; typedef A T; };
+struct AccPlainB {
+    Sum64 s;
+    XTG_DI void from(const AccPlain<double, 0>& a) { s.from(a.s); }
+    XTG_DI void to(AccPlain<double, 0>& a) const { a.s = s.total(); }
+    template <class X> XTG_DI void add(X x, i64) {
+        const X v[1][1] = {{x}};
+        addv(v);
+    }
+    // M vectors of V elements: a batch, or (M == 1) one behind the last batch
+    template <int M, int V, class X> XTG_DI void addv(const X (&x)[M][V]) {
+        double v[M * V];
+#pragma unroll
+        for (int i = 0; i < M * V; ++i) v[i] = cvt<double>(x[i / V][i % V]);
+        if (M > 1) s.batch(v);
+        else s.rest(v);
+    }
+};
+template <int NK> struct AccNormB {
+    Sum64 s;
+    XTG_DI void from(const AccNorm<double, NK>& a) { s.from(a.s); }
+    XTG_DI void to(AccNorm<double, NK>& a) const { a.s = s.total(); }
+    template <class X> XTG_DI void add(X x, i64) {
+        const X v[1][1] = {{x}};
+        addv(v);
+    }
+    template <int M, int V, class X> XTG_DI void addv(const X (&x)[M][V]) {
+        double v[M * V];
+#pragma unroll
+        for (int i = 0; i < M * V; ++i) {
+            const X f = x[i / V][i % V];
+            v[i] = NK == 1 ? (double)m_abs(f) : (double)(f * f);
+        }
+        if (M > 1) s.batch(v);
+        else s.rest(v);
+    }
+};
+template <int MODE> struct AccMomB {
+    double k;
+    Sum64 s;
+    double q[MODE != 0 ? 4 : 1];
+    XTG_DI void from(const AccMom<double, MODE>& a) {
+        k = a.k;
+        s.from(a.s1);
+        q[0] = a.s2;
+#pragma unroll
+        for (int u = 1; u < (MODE != 0 ? 4 : 1); ++u) q[u] = 0.0;
+    }
+    XTG_DI void to(AccMom<double, MODE>& a) const {
+        a.k = k;
+        a.s1 = s.total();
+        if constexpr (MODE != 0) a.s2 = (q[0] + q[2]) + (q[1] + q[3]);
+        else a.s2 = q[0];
+    }
+    template <class X> XTG_DI void add(X x, i64) {
+        const X v[1][1] = {{x}};
+        addv(v);
+    }
+    template <int M, int V, class X> XTG_DI void addv(const X (&x)[M][V]) {
+        double v[M * V];
+#pragma unroll
+        for (int i = 0; i < M * V; ++i) v[i] = cvt<double>(x[i / V][i % V]) - k;
+        if (M > 1) s.batch(v);
+        else s.rest(v);
+        if constexpr (MODE != 0) {
+#pragma unroll
+            for (int i = 0; i < M * V; ++i) q[i / V % 4] = fma(v[i], v[i], q[i / V % 4]);
+            if (M == 1) {  // the next vector to the next chain
+                const double r = q[0];
+                q[0] = q[1];
+                q[1] = q[2];
+                q[2] = q[3];
+                q[3] = r;
+            }
+        }
+    }
+};
+template <> struct Batch64<AccPlain<double, 0>> { enum { value = 1 }; typedef AccPlainB T; };
+template <> struct Batch64<AccNorm<double, 1>> { enum { value = 1 }; typedef AccNormB<1> T; };
+template <> struct Batch64<AccNorm<double, 2>> { enum { value = 1 }; typedef AccNormB<2> T; };
+template <int MODE> struct Batch64<AccMom<double, MODE>> { enum { value = 1 }; typedef AccMomB<MODE> T; };
+template <class T> struct IsBatch64 { enum { value = 0 }; };
+template <> struct IsBatch64<AccPlainB> { enum { value = 1 }; };
+template <int NK> struct IsBatch64<AccNormB<NK>> { enum { value = 1 }; };
+template <int MODE> struct IsBatch64<AccMomB<MODE>> { enum { value = 1 }; };
+
 // Arg-reductions (include/xtensor/misc/xsort.hpp:1158-1296): strict compare,
 // first index wins; NaN never wins unless it is the very first element (the
 // reference then returns 0 because nothing compares greater than NaN).
@@ -1955,6 +2071,9 @@ template <class... S, int VEC> struct Ring<LeafSet<S...>, VEC> {
 struct ArrVal {
     template <class RG, class C> static XTG_DI auto ev(const RG& r, int j, const C&) { return r[j]; }
 };
+// The type an accumulator takes its values in: the stored one or the tree's.
+template <bool STORED, class ET, class V> struct EvalAs { typedef V T; };
+template <class ET, class V> struct EvalAs<true, ET, V> { typedef ET T; };
 // Rows are finished G at a time by a group of G lanes: lane i keeps the state
 // of the group's i-th row since the last finish (group_reduce leaves the
 // total in every lane), and then every lane finishes its own.  The finishers
@@ -2074,24 +2193,46 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
             for (int l = 0; l < LS::N; ++l) off[l] = kbase[l] + e * p.lrs[l][RR - 1];
             LoadLeavesAt<LS>::template run<1>(rg1, p.leaf, off, inner);
         };
+        // the values of vector r as the accumulator takes them, stored too if ES
+        typedef typename EvalAs<ES != 0, ET, decltype(Tree::ev(*(const RG*)0, 0, c))>::T X;
+        auto values = [&](X(&x)[VEC], const RG& rg, i64 r) {
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) x[j] = cvt<X>(Tree::ev(rg, j, c));
+            if constexpr (ES != 0) {
+                i64 ri[RR];
+                decode_dims<RR, BIG>(p.rshape, p.rfd, r, ri);
+                ri[RR - 1] *= VEC;
+                i64 eo = ebase;
+#pragma unroll
+                for (int d = 0; d < RR; ++d) eo += ri[d] * p.ers[d];
+                st_out<ET, ES == 1 ? K_CONTIG : 2, VEC>(reinterpret_cast<ET*>(p.eout), eo, p.ers[RR - 1], x);
+            }
+        };
 // the reduction pass over the work item, folding into accumulator A
 #define XTG_ROW_PASS(A)                                                                \
     {                                                                                  \
         auto consume = [&](const RG(&rg)[U], i64 r0) {                                 \
+            if constexpr (IsBatch64<decltype(A)>::value != 0) {                        \
+                if (r0 - gtid + step <= re) {                                          \
+                    X x[U][VEC];                                                       \
+                    _Pragma("unroll") for (int u = 0; u < U; ++u)                      \
+                        values(x[u], rg[u], r0 + (i64)u * gsz);                        \
+                    A.addv(x);                                                         \
+                } else {                                                               \
+                    _Pragma("unroll") for (int u = 0; u < U; ++u) {                    \
+                        if (r0 + (i64)u * gsz >= re) break;                            \
+                        X x[1][VEC];                                                   \
+                        values(x[0], rg[u], r0 + (i64)u * gsz);                        \
+                        A.addv(x);                                                     \
+                    }                                                                  \
+                }                                                                      \
+            } else {                                                                   \
             _Pragma("unroll") for (int u = 0; u < U; ++u) {                            \
                 const i64 r = r0 + (i64)u * gsz;                                       \
                 if (r < re) {                                                          \
                     if constexpr (ES != 0) {                                           \
                         ET ev[VEC];                                                    \
-                        _Pragma("unroll") for (int j = 0; j < VEC; ++j)                \
-                            ev[j] = cvt<ET>(Tree::ev(rg[u], j, c));                    \
-                        i64 ri[RR];                                                    \
-                        decode_dims<RR, BIG>(p.rshape, p.rfd, r, ri);                  \
-                        ri[RR - 1] *= VEC;                                             \
-                        i64 eo = ebase;                                                \
-                        _Pragma("unroll") for (int d = 0; d < RR; ++d) eo += ri[d] * p.ers[d]; \
-                        st_out<ET, ES == 1 ? K_CONTIG : 2, VEC>(reinterpret_cast<ET*>(p.eout), eo, \
-                                                                 p.ers[RR - 1], ev);   \
+                        values(ev, rg[u], r);                                          \
                         AddVec<HasAdd2<decltype(A)>::value != 0, (PK > 1 ? 1 << (PK - 2) : 64)>::template run<VEC, ArrVal>( \
                             A, ev, r * VEC, c);                                        \
                     } else {                                                           \
@@ -2099,6 +2240,7 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
                             A, rg[u], r * VEC, c);                                     \
                     }                                                                  \
                 }                                                                      \
+            }                                                                          \
             }                                                                          \
         };                                                                             \
         i64 r0 = rb + gtid;                                                            \
@@ -2165,6 +2307,11 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
             } else {
                 FastItem<F>::to(fa, acc, rb * VEC);
             }
+        } else if constexpr (GROUP > 1 && GROUP < 32 && Batch64<Acc>::value != 0) {
+            typename Batch64<Acc>::T wa;
+            wa.from(acc);
+            XTG_ROW_PASS(wa)
+            wa.to(acc);
         } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
             // double-float states: two lanes advanced by packed instructions
             typename Work<Acc>::T wa;
@@ -5114,15 +5261,26 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
             Shift<Acc>::set(acc, Tree::ev(rg1, 0, c));
         }
         const int end = live ? nvr : 0;
+        // the values of the vector at element e as the accumulator takes them, stored too if ES
+        typedef typename EvalAs<ES != 0, ET, decltype(Tree::ev(*(const RG*)0, 0, c))>::T X;
+        auto values = [&](X(&x)[VEC], const RG& rg, int e) {
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) x[j] = cvt<X>(Tree::ev(rg, j, c));
+            if constexpr (ES != 0)
+                st_out<ET, ES == 1 ? K_CONTIG : 2, VEC>(reinterpret_cast<ET*>(p.eout), row * p.eks[0] + e * p.ers[0],
+                                                        p.ers[0], x);
+        };
 // One vector of the row, already loaded, into A.
 #define XTG_UNIT_ADD(A, V, r)                                                          \
     {                                                                                  \
         const int e = (r) * VEC;                                                       \
-        if constexpr (ES != 0) {                                                       \
+        if constexpr (IsBatch64<decltype(A)>::value != 0) {                            \
+            X x[1][VEC];                                                               \
+            values(x[0], V, e);                                                        \
+            A.addv(x);                                                                 \
+        } else if constexpr (ES != 0) {                                                \
             ET ev[VEC];                                                                \
-            _Pragma("unroll") for (int j = 0; j < VEC; ++j) ev[j] = cvt<ET>(Tree::ev(V, j, c)); \
-            st_out<ET, ES == 1 ? K_CONTIG : 2, VEC>(reinterpret_cast<ET*>(p.eout),     \
-                                                    row * p.eks[0] + e * p.ers[0], p.ers[0], ev); \
+            values(ev, V, e);                                                          \
             AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, ArrVal>(A, ev, (i64)e, c); \
         } else {                                                                       \
             AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, Tree>(A, V, (i64)e, c); \
@@ -5140,7 +5298,14 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
             RG rg[4];                                                                  \
             _Pragma("unroll") for (int u = 0; u < 4; ++u)                              \
                 UnitLoads<LS>::template run<VEC, MASK>(rg[u], buf, loff, p, kb, (r0 + u * G) * VEC); \
-            _Pragma("unroll") for (int u = 0; u < 4; ++u) XTG_UNIT_ADD(A, rg[u], r0 + u * G) \
+            if constexpr (IsBatch64<decltype(A)>::value != 0) {                        \
+                X x[4][VEC];                                                           \
+                _Pragma("unroll") for (int u = 0; u < 4; ++u)                          \
+                    values(x[u], rg[u], (r0 + u * G) * VEC);                           \
+                A.addv(x);                                                             \
+            } else {                                                                   \
+                _Pragma("unroll") for (int u = 0; u < 4; ++u) XTG_UNIT_ADD(A, rg[u], r0 + u * G) \
+            }                                                                          \
         }                                                                              \
         _Pragma("unroll 1") for (; r0 < end; r0 += G) {                                \
             RG rg;                                                                     \
@@ -5178,6 +5343,11 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
             } else {
                 XTG_UNIT_PASS(acc)
             }
+        } else if constexpr (G > 1 && G < 32 && Batch64<Acc>::value != 0) {
+            typename Batch64<Acc>::T wa;
+            wa.from(acc);
+            XTG_UNIT_PASS(wa)
+            wa.to(acc);
         } else if constexpr (Work<Acc>::packed != 0 && PK != 0) {
             typename Work<Acc>::T wa;
             wa.from(acc);
@@ -5634,20 +5804,37 @@ __global__ void __launch_bounds__(160) k_batch_rowunits(const BatchParams p) {
             BU::row(B, tl.row0, r, p.loff, off, at);
             Acc acc;
             acc.init(fp);
+            typename Batch64<Acc>::T wa;
+            if constexpr (Batch64<Acc>::value != 0) wa.from(acc);
+            else wa = acc;
             int e = gl;
             for (; e + 3 * g < end; e += 4 * g) {
                 RG rg[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) BU::load(rg[u], buf, off, at, cs, e + u * g);
+                if constexpr (Batch64<Acc>::value != 0) {
+                    decltype(Tree::ev(rg[0], 0, c)) x[4][1];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) acc.add(Tree::ev(rg[u], 0, c), (i64)(e + u * g));
+                    for (int u = 0; u < 4; ++u) x[u][0] = Tree::ev(rg[u], 0, c);
+                    wa.addv(x);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) wa.add(Tree::ev(rg[u], 0, c), (i64)(e + u * g));
+                }
             }
 #pragma unroll 1
             for (; e < end; e += g) {
                 RG rg;
                 BU::load(rg, buf, off, at, cs, e);
-                acc.add(Tree::ev(rg, 0, c), (i64)e);
+                if constexpr (Batch64<Acc>::value != 0) {
+                    decltype(Tree::ev(rg, 0, c)) x[1][1] = {{Tree::ev(rg, 0, c)}};
+                    wa.addv(x);
+                } else {
+                    wa.add(Tree::ev(rg, 0, c), (i64)e);
+                }
             }
+            if constexpr (Batch64<Acc>::value != 0) wa.to(acc);
+            else acc = wa;
             for (int m = (g < 32 ? g : 32) / 2; m >= 1; m >>= 1) {
                 const Acc o = shfl_xor_pod(acc, m);
                 acc.merge(o);

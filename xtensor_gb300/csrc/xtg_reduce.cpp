@@ -430,6 +430,7 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
             int g = 1;
             const int64_t lane_bytes = RO > 1 && RR == 1 ? 128 : 256;
             while (g < 32 && n_red * maxsz > g * (vec > 1 && g == 1 ? 128 : lane_bytes)) g *= 2;
+            if (g == 1 && maxsz == 8 && n_red >= 32) g = 2;  // (32 elements at an odd one: float64 sums in one chain)
             while (g < 32 && n_out * g < 4096 * 32 && g < p.n_redv) g *= 2;
             group = g;
             // single-element stores of 16 or 32 rows at once touch as many
