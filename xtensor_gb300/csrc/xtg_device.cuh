@@ -4461,7 +4461,37 @@ template <int K, int MODE, class C, class Sub, class... Rest> struct Stats<StatL
                     const C m = RowFin<C>::mean(sum, p);
                     A q;
                     RS::zero(q);
-                    if constexpr (sizeof(C) == 4) {
+                    if constexpr (sizeof(C) == 4 && (GROUP < 32 || VEC == 1 || GROUP == 128)) {
+                        // lanes that hold more of a row than a warp's (a
+                        // block's, of single elements) lanes would: pairs of
+                        // squares into two packed double-float sums, so a
+                        // lane's share does not add to the error (rms of the
+                        // variance over random rows, in the four chains below
+                        // / so, in ulps: 131 elements 0.74 / 0.63, 64 0.60 /
+                        // 0.48; with a warp per row 0.64, 0.50)
+                        constexpr int NE = NV * VEC;
+                        float2 hi = make_float2(0.f, 0.f), lo = hi;
+#pragma unroll
+                        for (int i = 0; i < NE; i += 4) {
+                            float d[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const int n = (i + u < NE ? i + u : 0) / VEC, j = (i + u < NE ? i + u : 0) % VEC;
+                                d[u] = i + u < NE && ok[n][j] ? cvt<float>(Sub::ev(rg[n], j, c)) - m : 0.f;
+                            }
+                            const float2 d0 = make_float2(d[0], d[1]), d1 = make_float2(d[2], d[3]);
+                            float2 sm, er;
+                            two_sum2(hi, p_fma(d1, d1, p_mul(d0, d0)), sm, er);
+                            hi = sm;
+                            lo = p_add(lo, er);
+                        }
+                        A r;
+                        q.hi = hi.x;
+                        q.lo = lo.x;
+                        r.hi = hi.y;
+                        r.lo = lo.y;
+                        q.merge(r);
+                    } else if constexpr (sizeof(C) == 4) {
                         // squared deviations are all >= 0 (no cancellation):
                         // four interleaved FP32 fma chains per lane (relative
                         // error below (n/(4*lanes) + 2) ulp), then compensated
