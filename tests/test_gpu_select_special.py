@@ -73,6 +73,29 @@ def test_other_axes(axes, shape):
         np.testing.assert_array_equal(got[n], want[n])
 
 
+@pytest.mark.parametrize("dt", ["float32", "float64"])
+@pytest.mark.parametrize("rows,cols", [(4104, 5), (1500, 9), (4104, 21), (4104, 64), (4101, 301), (40, 33), (40, 301), (4101, 1024)])
+@pytest.mark.parametrize("form", ["dense", "strided", "in place"])
+def test_fused_with_the_assignment(form, rows, cols, dt):
+    """Stored and reduced in one call: the same as assigned and then reduced."""
+    x = special_rows(rng(cols), rows, cols, dt)
+    d = DeviceArray.from_numpy(x)
+    for op in ("amax", "amin"):
+        if form == "in place":
+            d = out = DeviceArray.from_numpy(x)
+        elif form == "dense":
+            out = DeviceArray.empty((rows, cols), dt)
+        else:
+            out = DeviceArray.from_numpy(np.zeros((rows, cols + 3), dt))[:, 1:cols + 1]
+        r = ops.assign_reduce(out, d + d, op, axes=[1]).to_numpy()
+        got, want = out.to_numpy(), O.reduce(op, HostArray(x + x), [1])
+        np.testing.assert_array_equal(got, x + x)
+        np.testing.assert_array_equal(r, want, err_msg=op)
+        np.testing.assert_array_equal(r, ops.reduce(op, out, [1]).to_numpy())
+        n = ~np.isnan(want)
+        np.testing.assert_array_equal(np.signbit(r[n]), np.signbit(want[n]), err_msg=op)
+
+
 @pytest.mark.parametrize("dt,special", [("float64", -np.inf), ("float64", np.nan), ("float32", np.nan)])
 def test_cost(dt, special):
     """One special value per row of 1024: three passes over a cached row where

@@ -1132,8 +1132,31 @@ template <class A, int MAXOP> struct AccSelFrom<AccSel<A, MAXOP>> {
         if (ps >= from) s.add(cvt<A>(x), ps);
     }
 };
-template <class S> struct IsSel { enum { value = 0 }; };
-template <class A, int M> struct IsSel<AccSel<A, M>> { enum { value = 1 }; };
+template <class S> struct IsSel { enum { value = 0, nans = 0 }; };
+template <class A, int M> struct IsSel<AccSel<A, M>> { enum { value = 1, nans = IsFloat<A>::value }; };
+// The pass that also stores the elements (fused assign + reduce) folds and
+// takes down whether there was a NaN; the two passes above then go over what
+// was stored (an operand may be gone by then: it can be the destination).
+template <class S> struct AccSelNote;
+template <class A, int MAXOP> struct AccSelNote<AccSel<A, MAXOP>> {
+    AccSel<A, MAXOP> s;
+    bool nan;
+    template <class X> XTG_DI void add(X x, i64 ps) {
+        const A a = cvt<A>(x);
+        nan |= is_nan(a);
+        s.add(a, ps);
+    }
+};
+template <int MAXOP> struct AccSelNote<AccSel<double, MAXOP>> {
+    AccSel<double, MAXOP> s;
+    bool nan;
+    template <class X> XTG_DI void add(X x, i64 ps) {
+        const double a = cvt<double>(x);
+        const i64 b = __double_as_longlong(a);
+        if (f64_special(b)) nan |= f64_isnan_bits(b);  // where the fold leaves its short path, too
+        s.add(a, ps);
+    }
+};
 
 // Moments for mean / variance / stddev.  Data are shifted by k (the first
 // element of the output's reduction set), then sum(d) and sum(d*d) are
@@ -2294,7 +2317,9 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
             }
             reduced = GROUP <= 32 && !ex;
             if (nan) {
-                if constexpr (GROUP <= 32 && IsSel<Acc>::value) {
+                if constexpr (GROUP == 1) {
+                    XTG_ROW_PASS(acc)  // in order
+                } else if constexpr (GROUP <= 32 && IsSel<Acc>::value) {
                     LastNan<Acc> last{-1};
                     XTG_ROW_PASS(last)
                     AccSelFrom<Acc> rest;
@@ -2306,6 +2331,35 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
                 XTG_ROW_PASS(acc)
             } else {
                 FastItem<F>::to(fa, acc, rb * VEC);
+            }
+        } else if constexpr (IsSel<Acc>::nans && GROUP > 1 && GROUP <= 32) {
+            AccSelNote<Acc> note{acc, false};
+            XTG_ROW_PASS(note)
+            acc = note.s;
+            if (__any_sync(group_mask<GROUP>(), note.nan)) {
+// the pass over the stored elements, by the lanes that stored them
+#define XTG_STORED_PASS(A)                                                             \
+    {                                                                                  \
+        for (i64 r = rb + gtid; r < re; r += gsz) {                                    \
+            i64 ri[RR];                                                                \
+            decode_dims<RR, BIG>(p.rshape, p.rfd, r, ri);                              \
+            ri[RR - 1] *= VEC;                                                         \
+            i64 eo = ebase;                                                            \
+            _Pragma("unroll") for (int d = 0; d < RR; ++d) eo += ri[d] * p.ers[d];     \
+            _Pragma("unroll") for (int j = 0; j < VEC; ++j)                            \
+                A.add(reinterpret_cast<const ET*>(p.eout)[eo + j * p.ers[RR - 1]], r * VEC + j); \
+        }                                                                              \
+        if (RR == 1 && w == nwork - 1 && gtid == 0)                                    \
+            for (i64 e = p.n_redv * VEC; e < p.n_redv * VEC + p.tail; ++e)             \
+                A.add(reinterpret_cast<const ET*>(p.eout)[ebase + e * p.ers[RR - 1]], e); \
+    }
+                LastNan<Acc> last{-1};
+                XTG_STORED_PASS(last)
+                AccSelFrom<Acc> rest;
+                rest.begin(group_reduce<GROUP>(last, (LastNan<Acc>*)nullptr).p);
+                XTG_STORED_PASS(rest)
+                acc = rest.s;
+#undef XTG_STORED_PASS
             }
         } else if constexpr (GROUP > 1 && GROUP < 32 && Batch64<Acc>::value != 0) {
             typename Batch64<Acc>::T wa;
@@ -5361,8 +5415,8 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
             reduced = !fa.exact();
             if (reduced) {
                 fa.to(acc);
-            } else if (fa.nan()) {
-                if constexpr (IsSel<Acc>::value) {
+            } else if (G > 1 && fa.nan()) {
+                if constexpr (G > 1 && IsSel<Acc>::value) {
                     LastNan<Acc> last{-1};
                     XTG_UNIT_PASS(last)
                     AccSelFrom<Acc> rest;
@@ -5371,7 +5425,22 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
                     acc = rest.s;
                 }
             } else {
-                XTG_UNIT_PASS(acc)
+                XTG_UNIT_PASS(acc)  // (a lane alone: in order)
+            }
+        } else if constexpr (IsSel<Acc>::nans && G > 1) {
+            AccSelNote<Acc> note{acc, false};
+            XTG_UNIT_PASS(note)
+            acc = note.s;
+            if (__any_sync(group_mask<G>(), note.nan)) {
+                const ET* const er = reinterpret_cast<const ET*>(p.eout) + row * p.eks[0];
+                LastNan<Acc> last{-1};
+                for (int r = gl; r < end; r += G)
+                    for (int e = r * VEC; e < r * VEC + VEC; ++e) last.add(er[e * p.ers[0]], e);
+                AccSelFrom<Acc> rest;
+                rest.begin(group_reduce<G>(last, (LastNan<Acc>*)nullptr).p);
+                for (int r = gl; r < end; r += G)
+                    for (int e = r * VEC; e < r * VEC + VEC; ++e) rest.add(er[e * p.ers[0]], e);
+                acc = rest.s;
             }
         } else if constexpr (G > 1 && G < 32 && Batch64<Acc>::value != 0) {
             typename Batch64<Acc>::T wa;
