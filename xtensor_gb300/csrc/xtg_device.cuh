@@ -5236,6 +5236,7 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
     constexpr int UR = 32 / G;  // rows per unit
+    constexpr int BW = PK > 1 ? 1 << (PK - 2) : 64;
     constexpr int kPolls = 1 << 22;
     extern __shared__ __align__(128) unsigned char dsmem[];
     __shared__ u64 bars[4 * NS];
@@ -5365,9 +5366,9 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
         } else if constexpr (ES != 0) {                                                \
             ET ev[VEC];                                                                \
             values(ev, V, e);                                                          \
-            AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, ArrVal>(A, ev, (i64)e, c); \
+            AddVec<HasAdd2<decltype(A)>::value != 0, BW>::template run<VEC, ArrVal>(A, ev, (i64)e, c); \
         } else {                                                                       \
-            AddVec<HasAdd2<decltype(A)>::value != 0>::template run<VEC, Tree>(A, V, (i64)e, c); \
+            AddVec<HasAdd2<decltype(A)>::value != 0, BW>::template run<VEC, Tree>(A, V, (i64)e, c); \
         }                                                                              \
     }
 // The pass over the row's vectors gl, gl + G, gl + 2 G, ..., folding into A:

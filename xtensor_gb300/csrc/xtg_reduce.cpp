@@ -393,8 +393,10 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     const int part_off = (part && !(scratch && scratch->fixed)) ? (int)offsetof(xtg::RedParams, partial) : -1;
 
     // the widest vectors that divide a full reduction's length and fit its
-    // address: the blocks of its sums (AddVec)
-    int bw = vec;
+    // address: the blocks of its sums (AddVec); none for many rows under 32
+    // elements, whose sums are exact to 2^-46 (variances of 16 float32 by
+    // blocks: 2e-7 off)
+    int bw = row && RR == 1 && n_out >= 1024 && n_red < 32 ? 1 : vec;
     if (one_run)
         while (bw > 1 && (n_red % bw || (k13 && !aligned(t.leaves[0].data, (int64_t)bw * dt(t.leaves[0].dtype).size)))) bw >>= 1;
     Kernel* k;
@@ -413,6 +415,9 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
         st = get_kernel(name, 288, &k, smem);  // 8 consumer warps + the producer warp
         if (st == XTG_OK) st = launch(k, grid_cap(k, nsplit), 288, &p, stream, smem, part_off);
     } else if (row) {
+        const std::string pk = !opt("reduce.packed", 1) ? std::string(es ? "" : ", 0, float") + ", 0" :
+                               bw < vec && dfloat ? std::string(es ? "" : ", 0, float") + (bw == 1 ? ", 2" : bw == 2 ? ", 3" : ", 4") :
+                               std::string();
         int group = (chunk >= opt("reduce.cta_chunk", 2048)) ? 256 : 32;
         // Lanes per row of whole rows: about 256 bytes of the row per lane
         // (the unit of a warp is then about 8 KiB), so that short rows share a
@@ -468,8 +473,7 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
                                      std::to_string(post) + ", " + std::to_string(vec) + ", " + std::to_string(group) +
                                      ", " + std::to_string(mask) + ", 2, 4" +
                                      (es ? ", " + std::to_string(es) + ", " + dt(eout->dtype).cname : std::string()) +
-                                     (opt("reduce.packed", 1) ? std::string() : std::string(es ? "" : ", 0, float") + ", 0") +
-                                     ">";
+                                     pk + ">";
             XTG_TRY(get_kernel(name, 128, &k, smem));
             const int64_t units = (n_out * group + 31) / 32;
             return launch(k, grid_cap(k, (units + 3) / 4), 128, &p, stream, smem);
@@ -481,9 +485,7 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
                            std::to_string(RR) + ", " + std::to_string(group) + ", " + (big ? "true" : "false") + ", " +
                            std::to_string(opt("reduce.row_unroll", 4)) +
                            (es ? ", " + std::to_string(es) + ", " + dt(eout->dtype).cname : std::string()) +
-                           (!opt("reduce.packed", 1) ? std::string(es ? "" : ", 0, float") + ", 0" :
-                            bw < vec ? std::string(es ? "" : ", 0, float") + (bw == 1 ? ", 2" : bw == 2 ? ", 3" : ", 4") :
-                            std::string()) + ">";
+                           pk + ">";
         st = get_kernel(name, 256, &k);
         if (st == XTG_OK) {
             int64_t items = n_out * nsplit;
