@@ -1039,7 +1039,8 @@ template <class A, int MAXOP> struct AccSelFast {
         if (!keep) v = o.v;
     }
     XTG_DI bool nan() const { return odd; }
-    XTG_DI bool exact() const { return odd || (IsFloat<A>::value && v == A(0)); }
+    XTG_DI bool exact() const { return odd || zero(); }
+    XTG_DI bool zero() const { return IsFloat<A>::value && v == A(0); }
     XTG_DI void to(AccSel<A, MAXOP>& s) const {
         s.v = v;
         s.pos = -1;
@@ -1060,21 +1061,21 @@ template <int MAXOP> struct AccSelFast<float, MAXOP> {
     template <class X> XTG_DI void add(X x, i64) { v = fsel_nan(v, cvt<float>(x), MAXOP); }
     XTG_DI void merge(const AccSelFast& o) { v = fsel_nan(v, o.v, MAXOP); }
     XTG_DI bool nan() const { return !(v == v); }
-    XTG_DI bool exact() const { return !(v == v) || v == 0.f; }
+    XTG_DI bool exact() const { return nan() || zero(); }
+    XTG_DI bool zero() const { return v == 0.f; }
     XTG_DI void to(AccSel<float, MAXOP>& s) const {
         s.v = v;
         s.pos = -1;
     }
 };
 // double: the key order is the IEEE order except for NaNs and for -0 / +0,
-// so the pass keeps the largest high word magnitude, one more where the low
-// word is not zero: above an infinity's there is a NaN, which asks for the
-// exact pass, as does a best key that is a zero's (0: +0, -1: -0), where the
-// fold's last-visited rule decides.
-XTG_DI unsigned f64_mag_up(i64 b) { return ((unsigned)(b >> 32) & 0x7fffffffu) + ((unsigned)b != 0u ? 1u : 0u); }
+// so the pass keeps the largest high word magnitude (an infinity or a NaN
+// anywhere asks whether there is a NaN) and asks for the exact pass when the
+// best key is a zero's (0: +0, -1: -0), where the fold's last-visited rule
+// decides.
 template <int MAXOP> struct AccSelFast<double, MAXOP> {
     i64 kv;
-    unsigned mh;  // largest f64_mag_up seen
+    unsigned mh;  // largest (high word & 0x7fffffff) seen
     bool odd;
     template <class P> XTG_DI void init(const P& p) {
         AccSel<double, MAXOP> s;
@@ -1085,7 +1086,7 @@ template <int MAXOP> struct AccSelFast<double, MAXOP> {
     }
     template <class X> XTG_DI void add(X x, i64) {
         const i64 b = __double_as_longlong(cvt<double>(x));
-        const unsigned h = f64_mag_up(b);
+        const unsigned h = (unsigned)(b >> 32) & 0x7fffffffu;
         mh = mh > h ? mh : h;
         const i64 ka = key64(b);
         if (MAXOP ? (ka >= kv) : (ka <= kv)) kv = ka;
@@ -1095,8 +1096,9 @@ template <int MAXOP> struct AccSelFast<double, MAXOP> {
         odd |= o.odd;
         if (MAXOP ? (o.kv >= kv) : (o.kv <= kv)) kv = o.kv;
     }
-    XTG_DI bool nan() const { return mh > 0x7ff00000u; }
-    XTG_DI bool exact() const { return odd || nan() || kv == 0 || kv == -1; }
+    XTG_DI bool nan() const { return mh >= 0x7ff00000u; }  // (or an infinity)
+    XTG_DI bool exact() const { return nan() || zero(); }
+    XTG_DI bool zero() const { return odd || kv == 0 || kv == -1; }
     XTG_DI void to(AccSel<double, MAXOP>& s) const {
         s.kv = kv;
         s.pos = -1;
@@ -1104,7 +1106,8 @@ template <int MAXOP> struct AccSelFast<double, MAXOP> {
 };
 template <class A> struct FastSel { enum { value = 0 }; typedef A F; };
 template <class A, int M> struct FastSel<AccSel<A, M>> { enum { value = 1 }; typedef AccSelFast<A, M> F; };
-// The passes over a work item that has a NaN.  The fold drops what lies before
+// The passes over a work item that has a NaN (or, in float64, an infinity: the
+// first pass tells, and the fast pass's result stands where there is none).  The fold drops what lies before
 // a NaN (what follows replaces it), so the result is the fold of the elements
 // from the last NaN on, in which the positions stand for the order again: one
 // pass finds that NaN, one folds from there on, from the type's end (float32
@@ -1734,7 +1737,6 @@ template <class A, int MAXOP> struct AccArgFast {
         }
     }
     XTG_DI bool any_nan() const { return odd; }
-    XTG_DI bool nan() const { return false; }  // no pass here depends on the order
     XTG_DI bool exact() const { return IsFloat<A>::value && odd && !first && v == ends(); }
     XTG_DI void to(AccArg<A, MAXOP>& s) const {
         s.v = v;
@@ -1745,6 +1747,9 @@ template <class A, int MAXOP> struct AccArgFast {
         }
     }
 };
+// a float64's high word magnitude, one more where the low word is not zero:
+// above 0x7ff00000 it is a NaN
+XTG_DI unsigned f64_mag_up(i64 b) { return ((unsigned)(b >> 32) & 0x7fffffffu) + ((unsigned)b != 0u ? 1u : 0u); }
 template <int MAXOP> struct AccArgFast<double, MAXOP> {
     i64 kv;
     u32 off;
@@ -1776,7 +1781,6 @@ template <int MAXOP> struct AccArgFast<double, MAXOP> {
         }
     }
     XTG_DI bool any_nan() const { return mh > 0x7ff00000u; }
-    XTG_DI bool nan() const { return false; }
     XTG_DI bool exact() const {
         return !first && ((any_nan() && kv == (MAXOP ? XTG_KEY_MIN : XTG_KEY_MAX)) || kv == 0 || kv == -1);
     }
@@ -2307,23 +2311,27 @@ __global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 
                     fa.first = is_nan(Tree::ev(rg1, 0, c));
                 }
             }
-            bool ex, nan = false;
-            if (GROUP <= 32) {
+            bool ex;
+            i64 from = -1;  // the last NaN
+            if constexpr (GROUP <= 32) {
                 fa = group_reduce<GROUP>(fa, (F*)nullptr);  // the same in every lane
                 ex = fa.exact();
-                nan = fa.nan();
+                if constexpr (IsSel<Acc>::nans && GROUP > 1) {  // (a lane alone folds in order)
+                    if (fa.nan()) {
+                        LastNan<Acc> last{-1};
+                        XTG_ROW_PASS(last)
+                        from = group_reduce<GROUP>(last, (LastNan<Acc>*)nullptr).p;
+                        if (from < 0) ex = fa.zero();
+                    }
+                }
             } else {
                 ex = __syncthreads_or(fa.exact()) != 0;
             }
             reduced = GROUP <= 32 && !ex;
-            if (nan) {
-                if constexpr (GROUP == 1) {
-                    XTG_ROW_PASS(acc)  // in order
-                } else if constexpr (GROUP <= 32 && IsSel<Acc>::value) {
-                    LastNan<Acc> last{-1};
-                    XTG_ROW_PASS(last)
+            if (from >= 0) {
+                if constexpr (IsSel<Acc>::nans && GROUP > 1 && GROUP <= 32) {
                     AccSelFrom<Acc> rest;
-                    rest.begin(group_reduce<GROUP>(last, (LastNan<Acc>*)nullptr).p);
+                    rest.begin(from);
                     XTG_ROW_PASS(rest)
                     acc = rest.s;
                 }
@@ -5413,20 +5421,28 @@ __global__ void __launch_bounds__(128, MINB) k_reduce_unit(const RedParams p) {
                 }
             }
             fa = group_reduce<G>(fa, (F*)nullptr);  // the same in every lane
-            reduced = !fa.exact();
-            if (reduced) {
-                fa.to(acc);
-            } else if (G > 1 && fa.nan()) {
-                if constexpr (G > 1 && IsSel<Acc>::value) {
+            bool ex = fa.exact();
+            i64 from = -1;  // the last NaN
+            if constexpr (IsSel<Acc>::nans && G > 1) {  // (a lane alone folds in order)
+                if (fa.nan()) {
                     LastNan<Acc> last{-1};
                     XTG_UNIT_PASS(last)
+                    from = group_reduce<G>(last, (LastNan<Acc>*)nullptr).p;
+                    if (from < 0) ex = fa.zero();
+                }
+            }
+            reduced = !ex;
+            if (from >= 0) {
+                if constexpr (IsSel<Acc>::nans && G > 1) {
                     AccSelFrom<Acc> rest;
-                    rest.begin(group_reduce<G>(last, (LastNan<Acc>*)nullptr).p);
+                    rest.begin(from);
                     XTG_UNIT_PASS(rest)
                     acc = rest.s;
                 }
+            } else if (ex) {
+                XTG_UNIT_PASS(acc)
             } else {
-                XTG_UNIT_PASS(acc)  // (a lane alone: in order)
+                fa.to(acc);
             }
         } else if constexpr (IsSel<Acc>::nans && G > 1) {
             AccSelNote<Acc> note{acc, false};
