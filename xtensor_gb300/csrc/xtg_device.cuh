@@ -2127,12 +2127,25 @@ template <class Acc, class Out, int POST, int G> struct LaneFinish {
     }
 };
 // PK: 0 no packed states, 1 packed, 2 + k packed with blocks of 2^k elements.
-// Four blocks per SM for small states over two reduced dims (float64 sums over
-// axes 0 and 2 of 20 x 100000 x 7: 51 us with the compiler's choice of 70
-// registers, 42 with 64).
+// Blocks per SM that the registers have to leave room for, where the compiler
+// would stop at 70 to 76 (three blocks): states of up to 16 bytes over two
+// reduced dims (float64 sums over axes 0 and 2 of 20 x 100000 x 7 51 -> 42 us,
+// maxima of 30 x 40000 x 64 115 -> 106) and in blocks of float64 vectors (sums of
+// 2^26 in rows of 4096 227 -> 202, all of them 167 -> 150); three where vectors
+// of 8 would leave two (variances of bfloat16, 60 x 100000 x 16: 64 -> 59).
+// Single elements need fewer and run best unbound (maxima of float32 rows of
+// 5001: 82, 92 bound).
+template <int RR, int GROUP, int VEC, int ES, int SIZE> struct RowBlocks {
+    enum {
+        two = RR == 2 && GROUP <= 32,
+        value = (two && (SIZE <= 8 || (ES == 0 && VEC > 1 && VEC <= 4 && SIZE <= 16))) ||
+                        (GROUP > 32 && ES == 0 && VEC == 2 && SIZE <= 16) ? 4 :
+                two && ES == 0 && VEC == 8 ? 3 : 0
+    };
+};
 template <class Tree, class LS, class Acc, class Out, int POST, int VEC, int RO, int RR, int GROUP, bool BIG, int UR = 4,
           int ES = 0, class ET = float, int PK = 1>
-__global__ void __launch_bounds__(256, RR == 2 && GROUP <= 32 && sizeof(Acc) <= 8 ? 4 : 0) k_reduce_row(const RedParams p) {
+__global__ void __launch_bounds__(256, (RowBlocks<RR, GROUP, VEC, ES, (int)sizeof(Acc)>::value)) k_reduce_row(const RedParams p) {
     pdl_wait();
     typedef typename LS::template R<VEC>::type RG;
     __shared__ Acc smem[32];
