@@ -2634,9 +2634,10 @@ __global__ void __launch_bounds__(256) k_reduce_col(const RedParams p) {
             }
             // the rest by halves (maxima of 2^26 float64 in 5 rows 281 us one by
             // one, 173; predicated together, their registers cost a third of the
-            // blocks), but for plain sums, whose main loop the compiler then
-            // keeps fewer loads in flight in (float32, 32 rows: 52 us, 61)
-            if constexpr (RestByOne<Acc>::value == 0) {
+            // blocks), but for plain sums of lane-strided outputs, whose main loop
+            // the compiler then keeps fewer loads in flight in (float32, 32 rows:
+            // 52 us, 61)
+            if constexpr (!LSTR || RestByOne<Acc>::value == 0) {
                 if (U > 4 && r + 4 <= re) XTG_COL_BATCH(4)
                 if (U > 2 && r + 2 <= re) XTG_COL_BATCH(2)
             }
