@@ -299,12 +299,11 @@ xtg_status assign_tree(const Tree& t, const xtg_array* out, cudaStream_t stream)
     // Single elements of 4 bytes or less: a thread takes 4 rows of one column,
     // so it decodes one position for four elements (255 x 511 x 1001 float32
     // {1,0,2} 288 us with a decode per element, 167; 8-byte elements gain
-    // nothing: 3000 x 300 x 37 float64 86 us against 104; nor do rows of two or
-    // three 4-byte elements: 2^26 float32 in rows of 2 140, 159, a masked write
-    // of int32 rows of 3 171, 205)
+    // nothing: 3000 x 300 x 37 float64 86 us against 104; nor do pairs of 4
+    // bytes: 2^26 float32 in rows of 2 140, 159)
     int64_t all = 1;
     for (int d = 0; d < RR; ++d) all *= d == in ? D.shape[d] / vec : D.shape[d];
-    const bool rows = vec == 1 && maxsz <= 4 && RR >= 2 && D.shape[in] >= (maxsz == 4 ? 4 : 2) && D.shape[in - 1] >= 16 &&
+    const bool rows = vec == 1 && maxsz <= 4 && RR >= 2 && D.shape[in] >= (maxsz == 4 ? 3 : 2) && D.shape[in - 1] >= 16 &&
                       all <= 0xFFFFFFF0ll;
     const int U = rows ? 4 : (int)opt("assign.unroll", vec * maxsz >= 16 ? 4 : 8);
     p.rows = rows ? D.shape[in - 1] : 0;
