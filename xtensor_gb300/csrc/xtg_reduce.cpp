@@ -253,7 +253,7 @@ static xtg_status run_reduction(const Tree& t, const std::string& accname, int p
     int vec = 16 / maxsz;
     // a full reduction of one run takes the elements behind its whole vectors
     // one by one, so its length does not narrow them (2^28 - 1 bfloat16, all
-    // moments: 391 us by single elements, 125 by vectors)
+    // moments: 1253 us by single elements, 332 by vectors)
     const bool one_run = row && n_out == 1 && RR == 1;
     // (2^28 int8: sums 182 us in vectors of 16, 97 of 8; maxima of 2^27 bfloat16
     // 81 us in vectors of 8, 70 of 4)
